@@ -313,16 +313,14 @@ def run_b200(args):
     src = 'measured' if peaks else 'fallback'
     if top == 'mp_ms':
         ach = mp_bytes / (mean_st['mp_ms'] / 1e3) / 1e9
-        # the rounds kernel this handle runs (block-skipping from 600 templates)
-        kname, prof = (('k_mp_blocks (matching pursuit, block-skipping)', f'k_mp_blocks_384ch_{T}t.md')
-                       if s.round_kernel() else ('k_mp (matching pursuit)', f'k_mp_384ch_{T}t.md'))
+        kname, prof = 'k_mp_lazy (matching pursuit, deferred updates)', f'k_mp_lazy_384ch_{T}t.md'
         roof = {'kernel': kname, 'bound': 'hbm', 'achieved': ach, 'peak': hbm, 'unit': 'GB/s',
                 'frac': ach / hbm, 'traffic': profile_traffic(prof),
                 'traffic_source': 'ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload '
                                   f'(profiles/{prof})',
                 'algorithmic_bytes': mp_bytes, 'peak_source': src,
-                'note': 'achieved counts the algorithmic bytes of every row update; the block-skipping kernel '
-                        'proves most of them no-ops and moves only `traffic`'}
+                'note': 'achieved counts the algorithmic bytes of every row update; the deferred rounds make only '
+                        'the updates that can matter to a decision and move only `traffic`'}
     else:
         ach = gemm_flops / (mean_st['score_ms'] / 1e3) / 1e12
         roof = {'kernel': 'k_score_tc (tcgen05 3xTF32 score GEMM)' if args.precision == 'fp32'
@@ -360,14 +358,14 @@ def run_b200(args):
                                 'ms_per_step': t32 / K, 'stage_ms': st32,
                                 'api': 'lss_set_drift + lss_sort_batch_async, device-resident rows, same batches'}
         # the two rounds kernels on the same batches (identical results): every
-        # row updated, or provably unchanged template-row blocks skipped
+        # row updated in its round, or blocks of rows only once they can matter
         kernels = {}
         default_skip = s32.round_kernel()
         for skip in (False, True):
             s32.set_round_kernel(skip)
             tk, stk = device_resident_rate(s32, rows_d, drifts, ids, nb, K, W, stream, dist, local)
             st_k = s32.stats()
-            kernels['skip_blocks' if skip else 'full'] = {
+            kernels['deferred' if skip else 'full'] = {
                 'rec_s_per_s': world * K * rec_s / (tk / 1e3), 'mp_ms': stk['mp_ms'], 'phases_ms': stk['mp_phases_ms'],
                 'update_items': st_k['mp_items'], 'update_items_changed': st_k['mp_items_updated']}
         s32.set_round_kernel(default_skip)

@@ -167,15 +167,15 @@ int  lss_match_scores(lss_handle* h, const float* B_dev, int64_t N, int64_t* st_
                       float* amps_dev, int64_t capacity, int64_t* n_spikes, void* stream);
 
 /* Which kernel runs the matching-pursuit rounds of this handle (identical
- * spikes, amplitudes and score field either way; a performance choice, no
- * counterpart in the reference): 0 = every template row of every spike window
- * is updated; 1 = template rows are grouped in blocks along the probe and a
- * block whose update provably leaves every score unchanged (terms below a
- * quarter ulp of the block's smallest score) is skipped. The default is 1 from
- * 600 templates up (measured on a B200, 384 channels: 7.40 vs 7.75 ms of rounds
- * per 2-s batch at 800 templates, 2.43 vs 2.15 ms at 400), else 0. */
+ * spikes and amplitudes either way; a performance choice, no counterpart in the
+ * reference): 0 = every template row of every spike window is updated in its
+ * round; 1 = template rows are grouped in blocks along the probe and a block of
+ * the score field is updated only once it can take part in a decision (a bound
+ * of its scores reaches the threshold). A handle that was not told runs the
+ * deferred updates (measured on a B200, 384 channels, 2-s batches: 2.7 vs 7.7 ms
+ * of rounds at 800 templates, 0.90 vs 2.06 ms at 400). */
 int  lss_set_round_kernel(lss_handle* h, int32_t skip_blocks);
-/* The handle's rounds kernel (1: block-skipping, 0: every row). */
+/* The value last set; before that, 1 from 600 templates up, else 0. */
 int  lss_get_round_kernel(const lss_handle* h, int32_t* skip_blocks);
 
 /* The same matching-pursuit rounds for callers that cannot allocate device
@@ -240,9 +240,9 @@ typedef struct lss_stats {
     int64_t recheck_flips;
     int64_t launches;      /* kernels this handle has launched since creation */
     int64_t recheck_rescored;
-    /* matching-pursuit update work items (spike segment x template-row block x
-     * 32 columns) of the last synchronous batch, and how many of them changed
-     * any score: the others were skipped as exact no-ops */
+    /* deferred rounds: (spike, template-row block, 32 columns) items that the
+     * spikes' windows of the last synchronous batch covered, and how many of
+     * them were applied to the score field: the others could not matter */
     int64_t mp_items;
     int64_t mp_items_updated;
     /* the rounds' time split, per CTA of the rounds kernel (mean over CTAs,

@@ -116,7 +116,7 @@ int lss::rebuild_uw(lss_handle* h) {
     const bool bf16 = h->cfg.precision == LSS_PREC_BF16_RECHECK;
     // one product, stored as the tf32 split (FP32 path, BF16 re-check) and, on
     // the BF16 path, as the bf16 split too
-    CK(launch_build_uw(h->U.p, h->Mw.p, h->T, h->K, C, h->CKpad, bf16 ? h->Uw16.p : nullptr,
+    CK(launch_build_uw(h->Uq.p, h->Mw.p, h->T, h->K, C, h->CKpad, bf16 ? h->Uw16.p : nullptr,
                        bf16 ? h->Uw16lo.p : nullptr, h->Uw_hi.p, h->Uw_lo.p, 0));
     h->stats.launches += 1;
     if (bf16) {
@@ -137,17 +137,14 @@ int lss::rebuild_uw(lss_handle* h) {
     return LSS_OK;
 }
 
-// Template rows of the block-skipping rounds, ordered along the probe: by the
-// centre of mass, over the channel index, of each template's energy
-// sum_k U[t, k, c]^2 (channels follow the probe's geometry in the channel map,
-// so templates adjacent in this order sit close together and their
+// Probe order: templates by the centre of mass, over the channel index, of
+// their energy sum_k U[t, k, c]^2 (channels follow the probe's geometry in the
+// channel map, so templates adjacent in this order sit close together and their
 // cross-correlations with distant spikes vanish together). Any order gives the
-// same spikes; this one lets whole blocks be skipped. Then the |ctc| maxima per
-// (spike template, row).
-int lss::rebuild_mp_blocks(lss_handle* h) {
+// same spikes; this one lets whole blocks of rows wait. The score GEMM's
+// template rows and the deferred rounds' ctc are laid out in it.
+int lss::rebuild_probe_order(lss_handle* h, const float* u) {
     const int T = h->T, K = h->K, C = h->C, nb = h->mp_nb;
-    std::vector<float> u((size_t)T * K * C);
-    CK(cudaMemcpy(u.data(), h->U.p, u.size() * sizeof(float), cudaMemcpyDeviceToHost));
     std::vector<double> com(T, 0.0);
     for (int t = 0; t < T; ++t) {
         double w = 0.0, wc = 0.0;
@@ -162,15 +159,16 @@ int lss::rebuild_mp_blocks(lss_handle* h) {
     std::vector<int32_t> perm((size_t)nb * MPB_ROWS, -1);
     for (int t = 0; t < T; ++t) perm[t] = t;
     std::stable_sort(perm.begin(), perm.begin() + T, [&](int32_t i, int32_t j) { return com[i] < com[j]; });
-    std::vector<int32_t> rowof(T);
-    for (int r = 0; r < T; ++r) rowof[perm[r]] = r;
     CK(cudaMemcpy(h->mp_perm.p, perm.data(), perm.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->mp_rowof.p, rowof.data(), T * sizeof(int32_t), cudaMemcpyHostToDevice));
-    // the rounds read each spike template's ctc rows in the score rows' order
-    CK(launch_permute_ctc(h->ctcP.p, h->mp_perm.p, T, 2 * h->nt + 1, h->mp_ctcq.p, 0));
-    CK(launch_ctc_row_max(h->mp_ctcq.p, T, 2 * h->nt + 1, h->mp_cmaxr.p, 0));
+    const bool bf16 = h->cfg.precision == LSS_PREC_BF16_RECHECK;
+    CK(launch_gather_rows(h->U.p, (int64_t)K * C, h->mp_perm.p, T, (int64_t)K * C, h->Uq.p, (int64_t)K * C, 0));
+    CK(launch_gather_rows(h->nm.p, 1, h->mp_perm.p, T, 1, h->nmq.p, 1, 0));
+    CK(launch_template_operand(h->Uq.p, T, K, C, h->CKpad, h->Up_hi.p, h->Up_lo.p, bf16 ? h->Up16.p : nullptr,
+                               bf16 ? h->Up16lo.p : nullptr, 0));
+    h->un_p_stale = true;
+    CK(launch_tile_ctc(h->ctcP.p, h->mp_perm.p, h->nm.p, T, 2 * h->nt + 1, h->mp_ctct.p, h->mp_hg.p, 0));
     CK(cudaDeviceSynchronize());
-    h->stats.launches += 1;
+    h->stats.launches += 4;
     return LSS_OK;
 }
 
@@ -282,7 +280,7 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
     h->C = cfg->n_chan; h->Cbin = cfg->n_chan_bin; h->T = cfg->n_templates; h->K = cfg->n_pcs;
     h->nt = cfg->nt; h->nC = cfg->n_nearest; h->NT = cfg->batch_size;
     h->N = h->NT + 2 * h->nt;
-    h->ld = round_up(h->N, 4);
+    h->ld = round_up(h->N, 32);  // rows begin on 128-byte lines (32-column tiles of the rounds)
     const int C = h->C, T = h->T, K = h->K, nt = h->nt, nC = h->nC;
     const int64_t ld = h->ld, L2 = 2 * nt + 1;
 
@@ -319,13 +317,8 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
         for (int64_t e = 0; e < (int64_t)nC * C; ++e)
             if (t->iCC[e] < 0 || t->iCC[e] >= C) { g_create_err = "iCC entry out of range"; return LSS_ERR_ARG; }
     }
-    // U_p[t, c*K + k] = U[t, k, c]; ctcP[j, i, l] = ctc[i, j, l];
-    // wave[t, c, m] = sum_k U[t, k, c] * wPCA[k, m] (run_online_spikes.py:539)
-    std::vector<float> up((size_t)T * C * K);
-    for (int i = 0; i < T; ++i)
-        for (int k = 0; k < K; ++k)
-            for (int c = 0; c < C; ++c)
-                up[((size_t)i * C + c) * K + k] = t->wall3[((size_t)i * K + k) * C + c];
+    // ctcP[j, i, l] = ctc[i, j, l]; wave[t, c, m] = sum_k U[t, k, c] * wPCA[k, m]
+    // (run_online_spikes.py:539)
     std::vector<float> wave((size_t)T * C * nt);
     for (int i = 0; i < T; ++i)
         for (int c = 0; c < C; ++c)
@@ -346,8 +339,7 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
 
     // one CTA per >= 32 columns (a serving loop lowers it further so that
     // its probes' rounds kernels fit on the device together)
-    h->mp_grid = std::min<int>(std::min(mp_blocks_max_grid(cfg->device), mp_max_grid(cfg->device)),
-                               (int)std::max<int64_t>(1, (h->N + 31) / 32));
+    h->mp_grid = std::min<int>(mp_max_grid(cfg->device), (int)std::max<int64_t>(1, (h->N + 31) / 32));
     cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, cfg->device);
     h->CKpad = (C * K + 63) / 64 * 64;
     const int64_t cap = cfg->max_spikes;
@@ -427,7 +419,7 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
         ALLOC(hpTw, 4096);
     }
     ALLOC(R, (size_t)K * K * (2 * nt - 1));
-    ALLOC(B, (size_t)T * ld);
+    ALLOC(B, (size_t)((T + MPB_ROWS - 1) / MPB_ROWS * MPB_ROWS) * ld);  // rows [T, ld], or tiles of whole row blocks
     ALLOC(nm, T);
     ALLOC(ctcP, (size_t)T * T * L2);
     ALLOC(wave, (size_t)T * C * nt);
@@ -441,24 +433,25 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
     ALLOC(imax, ld);
     ALLOC(colkey, 2 * ld);
     h->mp_nb = (T + MPB_ROWS - 1) / MPB_ROWS;
-    // the block-skipping rounds pay off from a few hundred templates on (more
-    // rows per block far from a spike); below, updating every row is faster
-    h->mp_skip = T >= 600;
+    // The deferred rounds are the faster ones at every size measured (B200, rounds of one batch, against
+    // updating every row): 2.72 vs 7.68 ms at 384 channels, 800 templates, 60000 samples, 0.90 vs 2.06 at 400
+    // templates, 0.122 vs 0.160 at 64 channels and 32 templates, 0.038 vs 0.047 there on 300 samples. Slices
+    // too wide for their shared memory (batches of millions of samples) update every row.
+    h->mp_lazy = mp_lazy_fits(h->N, h->mp_grid, T, nt);
+    h->mp_switch = T >= 600;
     ALLOC(mp_perm, (size_t)h->mp_nb * MPB_ROWS);
-    ALLOC(mp_cmaxr, (size_t)T * T);
-    ALLOC(mp_rowof, T);
+    ALLOC(mp_hg, (size_t)T * h->mp_nb * mp_lag_groups((int)L2));
+    ALLOC(Uq, (size_t)T * K * C);
+    ALLOC(nmq, T);
     {
         const int64_t passes = ((T + 15) / 16 * 16 + 255) / 256;  // the score GEMM's template passes
         ALLOC(sc_part_keys, (size_t)(passes * ld));
         ALLOC(sc_part, (size_t)(4 * passes * ld));
     }
-    ALLOC(mp_ctcq, (size_t)T * T * L2);
+    ALLOC(mp_ctct, (size_t)T * h->mp_nb * MPB_ROWS * L2);
     ALLOC(mp_bkey, (size_t)h->mp_nb * ld);
     ALLOC(mp_phase, 6);
-    // 4 int4 per list entry
-    ALLOC(mp_ent, (size_t)mp_blocks_list_entries(ld, nt, T, h->mp_grid) * 4);
-    ALLOC(mp_ent_cnt, (size_t)h->mp_grid);
-    ALLOC(mp_bmin, (size_t)h->mp_nb * ld);
+    ALLOC(mp_xch, (size_t)mp_lazy_words(ld));
     ALLOC(blk_cnt, 4096);
     ALLOC(blk_x, ld);
     ALLOC(blk_y, ld);
@@ -494,48 +487,19 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
     CK(cudaMemcpy(h->chan_map.p, cmap.data(), C * sizeof(int32_t), cudaMemcpyHostToDevice));
     if (!taps.empty()) CK(cudaMemcpy(h->taps.p, taps.data(), taps.size() * sizeof(float), cudaMemcpyHostToDevice));
     if (bf16) {
-        // U_p as the bf16 split hi = bf16(x), lo = bf16(x - hi), [Tpad, CKpad] with zero padding
-        std::vector<__nv_bfloat16> u16((size_t)plan.Tpad * h->CKpad, __float2bfloat16(0.f)), u16lo(u16);
-        for (int i = 0; i < T; ++i)
-            for (int e = 0; e < C * K; ++e) {
-                const float x = up[(size_t)i * C * K + e];
-                const __nv_bfloat16 hb = __float2bfloat16(x);
-                u16[(size_t)i * h->CKpad + e] = hb;
-                u16lo[(size_t)i * h->CKpad + e] = __float2bfloat16(x - __bfloat162float(hb));
-            }
-        CK(cudaMemcpy(h->Up16.p, u16.data(), u16.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->Up16lo.p, u16lo.data(), u16lo.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice));
+        CK(cudaMemset(h->Up16.p, 0, (size_t)plan.Tpad * h->CKpad * sizeof(__nv_bfloat16)));
+        CK(cudaMemset(h->Up16lo.p, 0, (size_t)plan.Tpad * h->CKpad * sizeof(__nv_bfloat16)));
         CK(cudaMemset(h->B0T.p, 0, (size_t)h->N * h->CKpad * sizeof(__nv_bfloat16)));
         CK(cudaMemset(h->B0T16lo.p, 0, (size_t)h->N * h->CKpad * sizeof(__nv_bfloat16)));
         const size_t rc_bytes = (size_t)(h->N + 127) / 128 * 128 * h->CKpad * sizeof(float);
         CK(cudaMemset(h->Pc_hi.p, 0, rc_bytes));
         CK(cudaMemset(h->Pc_lo.p, 0, rc_bytes));
     }
-    {
-        // U_p split into tf32 parts, each rounded half away like cvt.rna.tf32.f32:
-        // hi = rna(x), lo = rna(x - hi)
-        auto rna = [](float x) {
-            uint32_t u;
-            std::memcpy(&u, &x, 4);
-            if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0x1000u) & 0xffffe000u;
-            float r;
-            std::memcpy(&r, &u, 4);
-            return r;
-        };
-        std::vector<float> hi((size_t)Tpad32 * h->CKpad, 0.f), lo(hi.size(), 0.f);
-        for (int i = 0; i < T; ++i)
-            for (int e = 0; e < C * K; ++e) {
-                const float x = up[(size_t)i * C * K + e];
-                const float xh = rna(x);
-                hi[(size_t)i * h->CKpad + e] = xh;
-                lo[(size_t)i * h->CKpad + e] = rna(x - xh);
-            }
-        CK(cudaMemcpy(h->Up_hi.p, hi.data(), hi.size() * sizeof(float), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->Up_lo.p, lo.data(), lo.size() * sizeof(float), cudaMemcpyHostToDevice));
-        if (!bf16) {
-            CK(cudaMemset(h->B0T_hi.p, 0, (size_t)h->N * h->CKpad * sizeof(float)));
-            CK(cudaMemset(h->B0T_lo.p, 0, (size_t)h->N * h->CKpad * sizeof(float)));
-        }
+    CK(cudaMemset(h->Up_hi.p, 0, (size_t)Tpad32 * h->CKpad * sizeof(float)));
+    CK(cudaMemset(h->Up_lo.p, 0, (size_t)Tpad32 * h->CKpad * sizeof(float)));
+    if (!bf16) {
+        CK(cudaMemset(h->B0T_hi.p, 0, (size_t)h->N * h->CKpad * sizeof(float)));
+        CK(cudaMemset(h->B0T_lo.p, 0, (size_t)h->N * h->CKpad * sizeof(float)));
     }
     CK(cudaMemcpy(h->nm.p, nmv.data(), T * sizeof(float), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->wave.p, wave.data(), wave.size() * sizeof(float), cudaMemcpyHostToDevice));
@@ -592,9 +556,8 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
     CK(cudaMemset(h->status_acc.p, 0, sizeof(int32_t)));
     CK(cudaEventCreateWithFlags(&h->batch_ev, cudaEventDisableTiming));
     CK(cudaMemcpy(h->Wrot.p, t->whitening, (size_t)C * C * sizeof(float), cudaMemcpyHostToDevice));
-    rc = set_mixing(h, t->drift);
-    if (rc) { g_create_err = h->err; return rc; }
-    rc = rebuild_mp_blocks(h);
+    rc = rebuild_probe_order(h, t->wall3);
+    if (!rc) rc = set_mixing(h, t->drift);
     if (rc) { g_create_err = h->err; return rc; }
     // the set-up work is on the legacy stream; waiting for it alone leaves
     // other handles' non-blocking streams (a serving loop's probes) running
@@ -633,13 +596,14 @@ int lss_get_stats(const lss_handle* h, lss_stats* out) {
 int lss_set_round_kernel(lss_handle* h, int32_t skip_blocks) {
     if (!h || (skip_blocks != 0 && skip_blocks != 1)) return LSS_ERR_ARG;
     if (h->streaming) return h->fail(LSS_ERR_STATE, "handle is owned by a serving loop");
-    h->mp_skip = skip_blocks != 0;
+    h->mp_switch = skip_blocks != 0;
+    h->mp_lazy = h->mp_switch && mp_lazy_fits(h->N, h->mp_grid, h->T, h->nt);
     return LSS_OK;
 }
 
 int lss_get_round_kernel(const lss_handle* h, int32_t* skip_blocks) {
     if (!h || !skip_blocks) return LSS_ERR_ARG;
-    *skip_blocks = h->mp_skip ? 1 : 0;
+    *skip_blocks = h->mp_switch ? 1 : 0;
     return LSS_OK;
 }
 
@@ -725,8 +689,8 @@ int lss::run_ingest(lss_handle* h, const int16_t* src, const IngestMap& map, flo
 }
 
 int lss::run_scores(lss_handle* h, const float* X, int64_t ldx, int64_t N, float* B, cudaStream_t s,
-                   bool* maxima_ready, bool folded, bool rows_for_mp) {
-    const int32_t* rowof = (rows_for_mp && h->mp_skip) ? h->mp_rowof.p : nullptr;
+                   bool* maxima_ready, bool folded, bool tiled) {
+    const int tiles = tiled ? h->mp_nb : 0;
     if (h->cfg.precision == LSS_PREC_BF16_RECHECK) {
         CK(launch_pca_proj_t(X, ldx, h->C, N, h->wpca.p, h->K, h->nt, h->B0T.p, h->B0T16lo.p, h->CKpad, s, h->pn2.p));
         h->mark(5, s);
@@ -740,12 +704,13 @@ int lss::run_scores(lss_handle* h, const float* X, int64_t ldx, int64_t N, float
         ex.eps = (float)(3.0 * std::ldexp(1.0, -18) * 1.01 + 2.0 * h->CKpad * std::ldexp(1.0, -24));
         ex.cf_lo = h->cf_lo.p;
         ex.cf_hi = h->cf_hi.p;
-        ex.rowof = rowof;
+        ex.perm = h->mp_perm.p;
+        ex.tile_blocks = tiles;
         ex.part_keys = h->sc_part_keys.p;
         ex.part = h->sc_part.p;
         ex.part_cap = (int64_t)h->sc_part_keys.n;
         CK(launch_score_tc_bf16x3(h->B0T.p, h->B0T16lo.p, h->CKpad, (int)N, folded ? h->Uw16.p : h->Up16.p,
-                                  folded ? h->Uw16lo.p : h->Up16lo.p, h->T, h->CKpad, h->nm.p, B, h->ld, h->cfmax.p,
+                                  folded ? h->Uw16lo.p : h->Up16lo.p, h->T, h->CKpad, h->nmq.p, B, h->ld, h->cfmax.p,
                                   h->imax.p, h->nt, h->status.p, h->sm_count, s, ex));
         // FP32 re-check of the columns whose first-round decisions the BF16
         // error bound leaves open; the column list and its length stay on the
@@ -760,11 +725,12 @@ int lss::run_scores(lss_handle* h, const float* X, int64_t ldx, int64_t N, float
         ex2.map_rows = 1;
         ex2.count_dev = h->rc_count.p;
         ex2.ncols = (int)N;
-        ex2.rowof = rowof;
+        ex2.perm = h->mp_perm.p;
+        ex2.tile_blocks = tiles;
         ex2.keys = h->colkey.p;  // templates split over CTAs; free until the rounds start (they clear it)
         const int max_rows = (int)((N + 127) / 128 * 128);
         CK(launch_score_tc_tf32x3(h->Pc_hi.p, h->Pc_lo.p, h->CKpad, max_rows, folded ? h->Uw_hi.p : h->Up_hi.p,
-                                  folded ? h->Uw_lo.p : h->Up_lo.p, h->T, h->CKpad, h->nm.p, B, h->ld, h->cfmax.p,
+                                  folded ? h->Uw_lo.p : h->Up_lo.p, h->T, h->CKpad, h->nmq.p, B, h->ld, h->cfmax.p,
                                   h->imax.p, h->nt, h->status.p, h->sm_count, s, ex2));
         CK(launch_recheck_flips(h->cfmax.p, h->imax.p, h->rc_cols.p, h->pre_cf.p, h->pre_im.p, h->rc_count.p, (int)N,
                                 th2, s));
@@ -783,9 +749,10 @@ int lss::run_scores(lss_handle* h, const float* X, int64_t ldx, int64_t N, float
     h->mark(5, s);
     TcExtra ex;
     ex.keys = h->colkey.p;  // free until the rounds start (they clear it)
-    ex.rowof = rowof;
+    ex.perm = h->mp_perm.p;
+    ex.tile_blocks = tiles;
     CK(launch_score_tc_tf32x3(h->B0T_hi.p, h->B0T_lo.p, h->CKpad, (int)N, folded ? h->Uw_hi.p : h->Up_hi.p,
-                              folded ? h->Uw_lo.p : h->Up_lo.p, h->T, h->CKpad, h->nm.p, B, h->ld, h->cfmax.p,
+                              folded ? h->Uw_lo.p : h->Up_lo.p, h->T, h->CKpad, h->nmq.p, B, h->ld, h->cfmax.p,
                               h->imax.p, h->nt, h->status.p, h->sm_count, s, ex));
     h->stats.launches += 2 + (h->T > 256 ? 1 : 0);  // + the key maxima of a multi-pass GEMM
     h->mark(6, s);
@@ -828,18 +795,14 @@ int lss::enqueue_mp(lss_handle* h, int64_t N, cudaStream_t s, bool maxima_ready)
     CK(cudaMemsetAsync(h->counters.p, 0, 4 * sizeof(int32_t), s));
     CK(cudaMemsetAsync(h->mp_phase.p, 0, 6 * sizeof(unsigned long long), s));
     a.phase = h->mp_phase.p;
-    if (h->mp_skip) {
+    if (h->mp_lazy) {
         a.perm = h->mp_perm.p;
         a.nb = h->mp_nb;
-        a.cmaxr = h->mp_cmaxr.p;
+        a.hg = h->mp_hg.p;
         a.bkey = h->mp_bkey.p;
-        a.bmin = h->mp_bmin.p;
-        a.ctcP = h->mp_ctcq.p;
-        a.ment = h->mp_ent.p;
-        a.ment_cnt = h->mp_ent_cnt.p;
-        a.ment_cap = (int32_t)std::min<int64_t>(h->mp_ent.n / 4 / G, INT32_MAX);
-        a.init_cols = 1;  // the rounds take their block maxima from the field itself
-        CK(launch_mp_blocks(a, G, s));
+        a.ctcP = h->mp_ctct.p;
+        a.xch = h->mp_xch.p;
+        CK(launch_mp_lazy(a, G, s));
     } else {
         a.init_cols = maxima_ready ? 0 : 1;
         CK(cudaMemsetAsync(h->colkey.p, 0, 2 * h->ld * sizeof(unsigned long long), s));
@@ -1022,10 +985,11 @@ int lss_scores(lss_handle* h, const float* X_dev, int64_t N, float* B_dev, void*
     CK(cudaMemcpy2DAsync(h->X.p, h->ld * sizeof(float), X_dev, N * sizeof(float), N * sizeof(float), h->C,
                          cudaMemcpyDeviceToDevice, s));
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));
-    int rc = run_scores(h, h->X.p, h->ld, N, h->B.p, s, nullptr, false, /*rows_for_mp=*/false);
+    // tiles, which the GEMM writes 64 bytes per thread at a time; one pass brings them into the caller's rows
+    int rc = run_scores(h, h->X.p, h->ld, N, h->B.p, s, nullptr, false, /*tiled=*/true);
     if (rc) return rc;
-    CK(cudaMemcpy2DAsync(B_dev, N * sizeof(float), h->B.p, h->ld * sizeof(float), N * sizeof(float), h->T,
-                         cudaMemcpyDeviceToDevice, s));
+    CK(launch_untile_scores(h->B.p, h->mp_perm.p, h->T, N, B_dev, N, s));
+    h->stats.launches += 1;
     int32_t st = 0;
     CK(cudaMemcpyAsync(&st, h->status.p, sizeof(st), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1070,7 +1034,7 @@ int lss_match(lss_handle* h, const float* X_dev, int64_t N, int64_t* st_dev, flo
                          cudaMemcpyDeviceToDevice, s));
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));
     bool ready = false;
-    int rc = run_scores(h, h->X.p, h->ld, N, h->B.p, s, &ready);
+    int rc = run_scores(h, h->X.p, h->ld, N, h->B.p, s, &ready, false, h->mp_lazy);
     if (rc) return rc;
     return match_common(h, N, h->X.p, st_dev, amps_dev, xres_dev, capacity, n_spikes, s, ready);
 }
@@ -1083,8 +1047,8 @@ int lss_match_scores(lss_handle* h, const float* B_dev, int64_t N, int64_t* st_d
     CK(cudaSetDevice(h->cfg.device));
     cudaStream_t s = (cudaStream_t)stream;
     CK(wait_mixing(h, s));
-    if (h->mp_skip) {  // the block-skipping rounds read the rows in probe order
-        CK(launch_gather_rows(B_dev, N, h->mp_perm.p, h->T, N, h->B.p, h->ld, s));
+    if (h->mp_lazy) {  // the deferred rounds read the field as tiles
+        CK(launch_tile_scores(B_dev, N, h->mp_perm.p, h->T, N, h->B.p, s));
         h->stats.launches += 1;
     } else {
         CK(cudaMemcpy2DAsync(h->B.p, h->ld * sizeof(float), B_dev, N * sizeof(float), N * sizeof(float), h->T,
@@ -1185,7 +1149,7 @@ static int sort_batch_impl(lss_handle* h, const int16_t* raw, int64_t n_rows, in
     if (up_slot >= 0) CK(cudaEventRecord(h->raw_free[up_slot], s));
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));
     bool ready = false;
-    rc = run_scores(h, Xh, h->ld, h->N, h->B.p, s, &ready, /*folded=*/true);
+    rc = run_scores(h, Xh, h->ld, h->N, h->B.p, s, &ready, /*folded=*/true, h->mp_lazy);
     if (rc) return rc;
     // rounds, features and records all read the spike count on the device:
     // the batch has one host synchronisation, at its end

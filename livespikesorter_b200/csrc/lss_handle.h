@@ -64,21 +64,20 @@ struct lss_handle {
     DevBuf<int32_t> imax, blk_cnt, blk_x, blk_y, sp_x, sp_y, sp_round, round_start, counters, status;
     DevBuf<float> sp_amp, blk_amp;
     DevBuf<unsigned long long> colkey;
-    // block-skipping rounds (mp_blocks.cu): template rows in blocks of
-    // MPB_ROWS ordered along the probe, |ctc| maxima, per-block column state
+    // deferred rounds (mp_lazy.cu): template rows in blocks of MPB_ROWS
+    // ordered along the probe, bounds of their ctc rows, the CTAs' exchange words
     bool un_p_stale = true;                      // plain-template norms (BF16 bound) need recomputing
-    bool mp_skip = false;                        // rounds kernel: block-skipping (mp_blocks.cu) or full (mp.cu)
+    bool mp_lazy = false;                        // rounds kernel: deferred (mp_lazy.cu) or every row (mp.cu)
+    bool mp_switch = false;                      // lss_get_round_kernel's answer
     int mp_nb = 0;
     DevBuf<int32_t> mp_perm;
-    DevBuf<float> mp_cmaxr, mp_bmin;
-    DevBuf<unsigned long long> mp_bkey;
+    DevBuf<float2> mp_hg;
+    DevBuf<unsigned long long> mp_bkey, mp_xch;
     DevBuf<unsigned long long> mp_phase;         // [6] phase clock of the rounds kernel
-    DevBuf<int4> mp_ent;                         // block-skipping rounds: per-CTA lists of blocks to process
-    DevBuf<int32_t> mp_ent_cnt;                  // [grid] entries per list
-    DevBuf<int32_t> mp_rowof;                    // [T] score row of each template in probe order
     DevBuf<unsigned long long> sc_part_keys;     // [passes, ld] score GEMM: per-pass best keys (error-bound split)
     DevBuf<float> sc_part;                       // [passes, 4, ld] per-pass bound partials
-    DevBuf<float> mp_ctcq;                       // [T, T, 2nt+1] ctc rows in probe order
+    DevBuf<float> mp_ctct;                       // [T, nb, 2nt+1, MPB_ROWS] ctc by (spike template, block, lag), a block's rows adjacent
+    DevBuf<float> Uq, nmq;                       // templates and energies in probe order
     // BF16 path (BF16x3 GEMM): projection and templates as bf16 hi / lo splits
     DevBuf<__nv_bfloat16> B0T, B0T16lo, Up16, Up16lo;
     DevBuf<float> B0T_hi, B0T_lo, Up_hi, Up_lo;  // FP32 path (3xTF32): tf32 hi/lo splits
@@ -167,7 +166,7 @@ struct lss_handle {
         tF.release(); iCC.release(); iU.release(); cfmax.release(); imax.release(); blk_cnt.release();
         blk_x.release(); blk_y.release(); sp_x.release(); sp_y.release(); sp_round.release();
         round_start.release(); counters.release(); status.release(); sp_amp.release(); blk_amp.release(); colkey.release();
-        mp_perm.release(); mp_cmaxr.release(); mp_phase.release(); mp_ent.release(); mp_ent_cnt.release(); mp_rowof.release(); mp_ctcq.release(); sc_part_keys.release(); sc_part.release(); mp_bmin.release(); mp_bkey.release();
+        mp_perm.release(); mp_hg.release(); mp_phase.release(); mp_xch.release(); mp_ctct.release(); Uq.release(); nmq.release(); sc_part_keys.release(); sc_part.release(); mp_bkey.release();
         bar.release(); rec_time.release(); rec_count.release(); rec_tmpl.release(); rec_slot.release(); rec_amp.release();
         rec_pc.release(); B0T.release(); B0T16lo.release(); Up16.release(); Up16lo.release();
         B0T_hi.release(); B0T_lo.release(); Up_hi.release(); Up_lo.release();
@@ -202,19 +201,20 @@ namespace lss {
 int run_ingest(lss_handle* h, const int16_t* src, const IngestMap& map, float* Xout, cudaStream_t s,
                const float** pre_out);
 // Projection and score GEMM of X [C, ldx] into B; *maxima_ready when the
-// column maxima were fused into the GEMM. rows_for_mp: B rows in the order
-// the selected rounds kernel reads (probe order for the block-skipping one).
+// column maxima were fused into the GEMM. tiled: B as the deferred
+// rounds' tiles, else as rows [T, ld].
 int run_scores(lss_handle* h, const float* X, int64_t ldx, int64_t N, float* B, cudaStream_t s,
-               bool* maxima_ready = nullptr, bool folded = false, bool rows_for_mp = true);
+               bool* maxima_ready = nullptr, bool folded = false, bool tiled = false);
 // Whitening-folded template operands from U and Mw (after a template or drift change).
 int rebuild_uw(lss_handle* h);
 // Orders stream s after the last template / drift rebuild (no host wait).
 inline cudaError_t wait_mixing(lss_handle* h, cudaStream_t s) {
     return h->mix_ev ? cudaStreamWaitEvent(s, h->mix_ev, 0) : cudaSuccess;
 }
-// Template order and |ctc| maxima of the block-skipping rounds (after the
-// templates or ctc change; synchronous).
-int rebuild_mp_blocks(lss_handle* h);
+// Probe order of the templates (u: U [T, K, C] on the host), and what is laid
+// out in it: the score GEMM's plain operands and energies, the deferred rounds'
+// ctc tiles and bounds (after the templates or ctc change; synchronous).
+int rebuild_probe_order(lss_handle* h, const float* u);
 // Mw = Mdrift @ Wrot with Mdrift already on the device, then rebuild_uw.
 int mix_device_drift(lss_handle* h);
 // Matching-pursuit rounds on h->B, enqueued only (counts stay on the device).

@@ -90,9 +90,12 @@ struct TcExtra {
     unsigned long long* part_keys = nullptr;
     float* part = nullptr;  // 4 x part_cap
     int64_t part_cap = 0;
-    // score rows in another order: template t's row of B is rowof[t] (the
-    // block-skipping rounds keep rows in probe order); null: row t
-    const int32_t* rowof = nullptr;
+    // the operand's template rows (and nm, un) are in probe order: row r is
+    // template perm[r] (null: r). B gets template t's scores as row t, or with
+    // tile_blocks = nb > 0 as the deferred rounds' tiles of R = MPB_ROWS rows:
+    // element (row r, column s) at ((s / 32 * nb + r / R) * 32 + s % 32) * R + r % R
+    const int32_t* perm = nullptr;
+    int tile_blocks = 0;
 };
 // B[t, s] (row stride ldb) = sum_kk B0T[s, kk] * Up[t, kk] with B0T [N, ldk] and Up [Tpad, CKpad]
 // bf16, CKpad a multiple of 64; also writes the column maxima cfmax/imax of Cf.
@@ -136,6 +139,11 @@ cudaError_t launch_recheck_flips(const float* cfmax, const int32_t* imax, const 
 // un[t] = ||hi[t, :] + lo[t, :]|| over rows of length ld
 cudaError_t launch_row_norms(const float* hi, const float* lo, int32_t T, int64_t ld, float* un, cudaStream_t s);
 
+// the score GEMM's plain template operand U_p[t, c*K + k] = U[t, k, c] as the tf32 split and (b16 given)
+// the bf16 split (setup.cu)
+cudaError_t launch_template_operand(const float* U, int32_t T, int32_t K, int32_t C, int64_t ldk, float* hi, float* lo,
+                                    __nv_bfloat16* b16, __nv_bfloat16* b16lo, cudaStream_t s);
+
 // ---- matching pursuit (mp.cu) ----
 struct MPArgs {
     float* B;                 // [T, ldb] score field, updated in place
@@ -165,34 +173,38 @@ struct MPArgs {
     int32_t cols_per_blk;     // W
     int32_t init_cols;        // 1: compute column maxima of B before round 0
     unsigned long long* phase = nullptr;    // [6] phase clock of the rounds (PhaseClock), zero at launch; may be null
-    // block-skipping rounds (mp_blocks.cu) only: the score rows of B are in
-    // probe order (row r holds template perm[r]) and grouped in blocks of
-    // MPB_ROWS; ctcP then points at ctcQ [T(spike template), T(row), 2nt+1]
+    // deferred rounds (mp_lazy.cu) only: B is laid out as tiles (TcExtra), rows
+    // in probe order (row r holds template perm[r]) in blocks of MPB_ROWS; ctcP
+    // then points at ctct [T(spike template), nb, 2nt+1, MPB_ROWS]
     const int32_t* perm = nullptr;          // [nb * MPB_ROWS] template of each row, -1 past T
     int32_t nb = 0;                         // row blocks
-    const float* cmaxr = nullptr;           // [T(spike template), T(row)] max |ctc| over lags
-    unsigned long long* bkey = nullptr;     // [nb, ldk] per block and column: max (Cf bits << 32 | ~t)
-    float* bmin = nullptr;                  // [nb, ldk] per block and column: min |B|
-    int4* ment = nullptr;                   // [G * ment_cap * 4] per-CTA lists of blocks to process (64-byte
-                                            // entries); null: blocks are processed where they are decided
-    int32_t* ment_cnt = nullptr;            // [G] entries per list
-    int32_t ment_cap = 0;                   // entries per list
+    const float2* hg = nullptr;             // [T(spike template), groups of MPB_LAGS lags, nb] bounds of a block's ctc rows
+    unsigned long long* bkey = nullptr;     // [nb, ldk] the tiles' keys where shared memory does not hold them
+    unsigned long long* xch = nullptr;      // [mp_lazy_words(N)] words the CTAs exchange
+    int32_t log_cap = 0, new_cap = 0;       // spikes of a CTA's log, of one round (set by the launcher)
 };
 enum : int32_t { STATUS_TIMEOUT = 1, STATUS_CAPACITY = 2, STATUS_LIST = 4 };
 cudaError_t launch_mp(MPArgs a, int grid, cudaStream_t s);
-// the same rounds, skipping (spike, row block) updates that provably leave
-// every score of the block unchanged; needs perm, nb, cmaxr, bkey, bmin
-constexpr int MPB_ROWS = 32;
-cudaError_t launch_mp_blocks(MPArgs a, int grid, cudaStream_t s);
-int mp_blocks_max_grid(int device);
-// entries the lists of a grid of `grid` CTAs hold in all (ment_cap = that / grid
-// keeps every round of at most (N + nt) / (nt + 1) peaks in list mode)
-int64_t mp_blocks_list_entries(int64_t N, int nt, int T, int grid);
-// cmaxr[y, t] = max over lags of |ctcP[y, t, :]| (infinite where a lag is NaN)
-cudaError_t launch_ctc_row_max(const float* ctcP, int32_t T, int32_t L2, float* cmaxr, cudaStream_t s);
-// ctcQ[y, r, :] = ctcP[y, perm[r], :] (the block-skipping rounds' copy, rows in probe order)
-cudaError_t launch_permute_ctc(const float* ctcP, const int32_t* perm, int32_t T, int32_t L2, float* ctcQ,
+// the same rounds, updating a tile of the field only when it can take part in
+// a decision; needs perm, nb, hg, bkey, xch and rows of B aligned to 32 columns
+constexpr int MPB_ROWS = 16;  // template rows of a tile
+constexpr int MPB_LAGS = 8;   // lags of a group of the bounds
+inline int mp_lag_groups(int L2) { return (L2 + MPB_LAGS - 1) / MPB_LAGS; }
+cudaError_t launch_mp_lazy(MPArgs a, int max_grid, cudaStream_t s);
+// whether the deferred rounds can run a batch of N columns on at most grid CTAs
+bool mp_lazy_fits(int64_t N, int grid, int T, int nt);
+// 64-bit words of MPArgs::xch for batches of at most N columns
+int64_t mp_lazy_words(int64_t N);
+// ctct[y, b, l, u] = ctcP[y, perm[MPB_ROWS b + u], l] (zero past T), and hg
+// [T, lag groups, nb]: bounds of each block's rows per spike template and lag group
+cudaError_t launch_tile_ctc(const float* ctcP, const int32_t* perm, const float* nm, int32_t T, int32_t L2, float* ctct,
+                            float2* hg, cudaStream_t s);
+// score rows [T, N] (row stride lds) as the deferred rounds' tiles
+cudaError_t launch_tile_scores(const float* src, int64_t lds, const int32_t* perm, int32_t T, int64_t N, float* dst,
                                cudaStream_t s);
+// ... and back: tiles of N columns to rows [T, N] in template order
+cudaError_t launch_untile_scores(const float* src, const int32_t* perm, int32_t T, int64_t N, float* dst, int64_t ldd,
+                                 cudaStream_t s);
 // dst row r = src row perm[r], N columns
 cudaError_t launch_gather_rows(const float* src, int64_t lds, const int32_t* perm, int32_t rows, int64_t N,
                                float* dst, int64_t ldd, cudaStream_t s);

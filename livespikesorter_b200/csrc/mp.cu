@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(MP_THREADS, 1) k_mp(MPArgs a) {
         }
     }
     if (!grid_sync(a.bar, a.status)) return;
-    __shared__ unsigned long long s_clk[5];
+    __shared__ unsigned long long s_clk[PhaseClock::WORDS];
     PhaseClock clk{s_clk};
     if (tid == 0) clk.start();
     int base = 0;

@@ -1,6 +1,6 @@
 // Device helpers shared by the two matching-pursuit kernels (mp.cu: the
-// rounds over the whole score field; mp_blocks.cu: the rounds that skip
-// template-row blocks whose update leaves every score unchanged).
+// rounds that update every row; mp_lazy.cu: the rounds that update a tile of
+// the score field only when it can take part in a decision).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -74,61 +74,41 @@ __device__ __forceinline__ float ld_stream(const float* a, uint64_t pol) {
     return v;
 }
 
-
-// Predicated store (no branch around it), so that the rows of a batch stay
-// in one basic block and their chains interleave.
-__device__ __forceinline__ void st_keep_if(float* a, float v, bool p, uint64_t pol) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
-        "@q st.global.cg.L2::cache_hint.f32 [%0], %1, %3;\n\t}" ::"l"(a),
-        "f"(v), "r"((int)p), "l"(pol)
-        : "memory");
-}
-// Asynchronous 4-byte copy global -> shared (skipped where p is false), and
-// its group commit / wait. The copies go through L1 (cp.async of 4 bytes has
-// only the .ca form); rows that other CTAs updated in an earlier round are
-// visible because every round ends at a grid barrier whose gpu-scope fences
-// order those writes before this CTA's later reads.
-__device__ __forceinline__ void cp_async4_if(uint32_t dst, const float* src, bool p, uint64_t pol) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
-        "@q cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 4, %3;\n\t}" ::"r"(dst),
-        "l"(src), "r"((int)p), "l"(pol)
-        : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 // Phase clock of the rounds (thread 0 of each CTA): time in the peak phase,
-// waiting at the grid barrier after it, in the update phase and waiting after
-// it, summed over the rounds; added to phase[0..3] (sums over CTAs) with the
-// slowest CTA's peak and update totals in phase[4], phase[5].
-// The clock lives in shared memory (s: time of the last lap, then the four
-// sums), so that no register is held for it across the rounds.
+// waiting after it, in the update phase and waiting after it, summed over the
+// rounds; added to phase[0..3] in ns (sums over CTAs) with the slowest CTA's
+// peak and update totals in phase[4], phase[5]. Laps read the SM's cycle
+// counter (the global timer takes about half a microsecond per read); the
+// totals are scaled by the global timer's span over the cycles' span.
+// The clock lives in shared memory, so that no register is held for it.
 struct PhaseClock {
-    unsigned long long* s;  // [5] shared
+    static constexpr int WORDS = 7;
+    unsigned long long* s;  // [WORDS] shared: last lap, four sums, first cycle, first time
     __device__ __forceinline__ static unsigned long long now() {
         unsigned long long v;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v));
         return v;
     }
     __device__ __forceinline__ void start() {
-        s[0] = now();
+        s[6] = now();
+        s[0] = s[5] = (unsigned long long)clock64();
         for (int i = 1; i < 5; ++i) s[i] = 0;
     }
     __device__ __forceinline__ void lap(int i) {
-        const unsigned long long u = now();
+        const unsigned long long u = (unsigned long long)clock64();
         s[1 + i] += u - s[0];
         s[0] = u;
     }
     __device__ __forceinline__ void flush(unsigned long long* phase) const {
         if (!phase) return;
-        for (int i = 0; i < 4; ++i) atomicAdd(phase + i, s[1 + i]);
-        atomicMax(phase + 4, s[1]);
-        atomicMax(phase + 5, s[3]);
+        const double ns = (double)(now() - s[6]) / (double)max(1ull, (unsigned long long)clock64() - s[5]);
+        unsigned long long t[4];
+        for (int i = 0; i < 4; ++i) {
+            t[i] = (unsigned long long)((double)s[1 + i] * ns);
+            atomicAdd(phase + i, t[i]);
+        }
+        atomicMax(phase + 4, t[0]);
+        atomicMax(phase + 5, t[2]);
     }
 };
 

@@ -210,7 +210,7 @@ int enqueue_stream_batch(Probe* p) {
     if (rc) return p->fail(rc, h->err);
     PCK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));
     bool ready = false;
-    rc = run_scores(h, Xh, h->ld, h->N, h->B.p, s, &ready, /*folded=*/true);
+    rc = run_scores(h, Xh, h->ld, h->N, h->B.p, s, &ready, /*folded=*/true, h->mp_lazy);
     if (rc) return p->fail(rc, h->err);
     rc = enqueue_mp(h, h->N, s, ready);
     if (rc) return p->fail(rc, h->err);
@@ -517,11 +517,7 @@ int lss_server_admit(lss_server* s, const lss_config* cfg, const lss_tensors* t,
     // every admitted probe's rounds kernel (a cooperative grid, one CTA per
     // SM) must fit beside the others': at most SMs / max_probes CTAs each
     h->mp_grid = std::max(1, std::min(h->mp_grid, h->sm_count / (int)s->probes.size()));
-    // short stream batches: the block-skipping rounds' extra grid barrier per
-    // round costs more latency than the rows it skips (measured on a B200, 800
-    // templates, 300-sample blocks: p99 2.66 ms against about 2 ms), so every
-    // row is updated
-    h->mp_skip = false;
+    h->mp_lazy = mp_lazy_fits(h->N, h->mp_grid, h->T, h->nt);
     h->streaming = true;
     rc = capture(p.get());
     if (!rc) rc = calibrate_clock(p.get());

@@ -90,6 +90,13 @@ __global__ void k_up(const float* __restrict__ U, int T, int K, int C, int64_t l
     }
 }
 
+cudaError_t launch_template_operand(const float* U, int32_t T, int32_t K, int32_t C, int64_t ldk, float* hi, float* lo,
+                                    __nv_bfloat16* b16, __nv_bfloat16* b16lo, cudaStream_t s) {
+    const int64_t n = (int64_t)T * C * K;
+    k_up<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(U, T, K, C, ldk, hi, lo, b16, b16lo);
+    return cudaGetLastError();
+}
+
 // wave[t, c, m] = sum_k U[t, k, c] wPCA[k, m] (double, k order)
 __global__ void k_wave(const float* __restrict__ U, const float* __restrict__ W, int T, int K, int C, int nt,
                        float* __restrict__ wave) {
@@ -272,11 +279,6 @@ int lss_set_templates(lss_handle* h, const float* U, const float* wPCA) {
     k_basis<<<(nb + 255) / 256, 256, 0, s>>>(h->wpca.p, K, nt, h->R.p, wtw.p);
     k_nm_iu<<<(T + 127) / 128, 128, 0, s>>>(h->U.p, T, K, C, h->nm.p, nC > 0 ? h->iU.p : nullptr);
     if (nC > 0) k_ucc<<<(nC * T * K + 255) / 256, 256, 0, s>>>(h->U.p, h->iCC.p, h->iU.p, nC, T, K, C, h->Ucc.p);
-    const int64_t nup = (int64_t)T * C * K;
-    const bool bf16 = h->cfg.precision == LSS_PREC_BF16_RECHECK;
-    k_up<<<(unsigned)((nup + 255) / 256), 256, 0, s>>>(h->U.p, T, K, C, h->CKpad, h->Up_hi.p, h->Up_lo.p,
-                                                       bf16 ? h->Up16.p : nullptr, bf16 ? h->Up16lo.p : nullptr);
-    h->un_p_stale = true;  // the plain templates changed
     const int64_t nw = (int64_t)T * C * nt;
     k_wave<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(h->U.p, h->wpca.p, T, K, C, nt, h->wave.p);
     const int M = T * K;
@@ -285,7 +287,7 @@ int lss_set_templates(lss_handle* h, const float* U, const float* wPCA) {
     if (smem > 48 * 1024) SCK(cudaFuncSetAttribute(k_ctc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_ctc<<<dim3((T + CJ - 1) / CJ, T), 128, smem, s>>>(utu.p, wtw.p, T, K, nt, h->ctcP.p);
     SCK(cudaGetLastError());
-    h->stats.launches += 7 + (nC > 0);
+    h->stats.launches += 6 + (nC > 0);
     SCK(cudaStreamSynchronize(s));
     // energies must stay positive for the rounds' division
     std::vector<float> nmv(T);
@@ -293,9 +295,9 @@ int lss_set_templates(lss_handle* h, const float* U, const float* wPCA) {
     for (int i = 0; i < T; ++i)
         if (!(nmv[i] > 0.f) || !std::isfinite(nmv[i]))
             return h->fail(LSS_ERR_ARG, "template " + std::to_string(i) + " has zero or non-finite energy");
-    // the rounds' template order and |ctc| maxima, and the whitening-folded
-    // operands, follow the new templates
-    const int rc = rebuild_mp_blocks(h);
+    // the templates' probe order and what is laid out in it, and the
+    // whitening-folded operands, follow the new templates
+    const int rc = rebuild_probe_order(h, U);
     if (rc) return rc;
     return rebuild_uw(h);
 }

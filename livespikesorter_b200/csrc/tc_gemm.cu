@@ -72,7 +72,8 @@ struct Args {
     const int32_t* rowmap;    // GEMM row r scores sample rowmap[r / map_rows] * map_rows + r % map_rows (null: r)
     int map_rows;
     const int32_t* count_dev; // rows = min(N, count_dev[0] * map_rows) (null: N)
-    const int32_t* rowof;     // template t's score row is Bout row rowof[t] (null: t)
+    const int32_t* perm;      // template of each operand row (null: the row's number)
+    int tile_blocks;          // > 0: Bout as the deferred rounds' tiles, that many row blocks
     int ncols;                // samples in the batch (edge columns are the first/last nt)
     float* cf2;               // runner-up Cf of each column (null: not tracked)
     int pass_w;               // templates per pass (<= MAX_NP)
@@ -215,6 +216,13 @@ __device__ __forceinline__ void st_keep(float* a, float v, uint64_t pol) {
     asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(a), "f"(v), "l"(pol) : "memory");
 }
 
+// 8 consecutive floats (32-byte aligned), kept in L2 like st_keep
+__device__ __forceinline__ void st_keep8(float* a, const uint32_t* v) {
+    asm volatile("st.global.L2::evict_last.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "l"(a)
+                 : "memory");
+}
+
 // Running column maximum of Cf with the rounds kernel's exact rule, plus the
 // runner-up (to within the 3-ulp reciprocal approximation) when asked for.
 struct ColMax {
@@ -223,7 +231,7 @@ struct ColMax {
     float second = -1.f;
     int bi = 0;
     template <bool SECOND>
-    __device__ __forceinline__ void consider(float b, float nmv, float inv, int t) {
+    __device__ __forceinline__ void consider(float b, float nmv, float inv, int t, const int32_t* perm) {
         const float r = fmaxf(b, 0.f);
         const float sq = __fmul_rn(r, r);
         const float approx = __fmul_rn(sq, inv);
@@ -232,7 +240,8 @@ struct ColMax {
             return;
         }
         const float cf = __fdiv_rn(sq, nmv);
-        if (cf > best) {
+        // the smaller template on ties (rows in any order)
+        if (cf > best || (cf == best && perm && __ldg(perm + t) < __ldg(perm + bi))) {
             if (SECOND) second = fmaxf(second, best);
             best = cf;
             bi = t;
@@ -435,18 +444,25 @@ __global__ void __launch_bounds__(THREADS, 1)
                 for (int c = 0; c < np; c += 16) {
                     uint32_t r[16];
                     tmem_ld16(tbase + (uint32_t)c, r);
-                    const int t0 = p * PW + c;
+                    const int t0 = p * PW + c;  // operand row (probe order)
                     if (valid) {
+                        if (a.tile_blocks) {
+                            // this thread's column of one tile: 64 bytes
+                            static_assert(MPB_ROWS == 16, "one tile per 16 operand rows");
+                            float* bt = a.Bout + (((int64_t)(n >> 5) * a.tile_blocks + (t0 >> 4)) * 32 + (n & 31)) * MPB_ROWS;
+                            st_keep8(bt, r);
+                            st_keep8(bt + 8, r + 8);
+                        }
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
                             const int t = t0 + j;
                             if (t < a.T) {
                                 const float v = __uint_as_float(r[j]);
-                                const int orow = a.rowof ? __ldg(a.rowof + t) : t;
-                                st_keep(a.Bout + (int64_t)orow * a.ldb + n, v, pol);
+                                if (!a.tile_blocks)
+                                    st_keep(a.Bout + (int64_t)(a.perm ? __ldg(a.perm + t) : t) * a.ldb + n, v, pol);
                                 if (!edge) {
-                                    if (second) m.consider<true>(v, s_nm[t], s_inv[t], t);
-                                    else m.consider<false>(v, s_nm[t], s_inv[t], t);
+                                    if (second) m.consider<true>(v, s_nm[t], s_inv[t], t, a.perm);
+                                    else m.consider<false>(v, s_nm[t], s_inv[t], t, a.perm);
                                     if (bounds) {
                                         // Cf of the FP32 path lies in [lo, hi]: B within +-dB,
                                         // directed rounding, then a margin for the
@@ -477,6 +493,10 @@ __global__ void __launch_bounds__(THREADS, 1)
                 acc = (acc + 1) % a.nacc;
             }
             if (ok && valid) {
+                if (a.perm) {  // operand rows to templates
+                    m.bi = __ldg(a.perm + m.bi);
+                    if (thi1 >= 0) thi1 = __ldg(a.perm + thi1);
+                }
                 if (split && bounds) {
                     const int64_t nc = a.ncols;
                     const float cf = edge ? 0.f : fmaxf(m.best, 0.f);
@@ -693,7 +713,8 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     a.rowmap = ex.rowmap;
     a.map_rows = ex.map_rows;
     a.count_dev = ex.count_dev;
-    a.rowof = ex.rowof;
+    a.perm = ex.perm;
+    a.tile_blocks = ex.tile_blocks;
     a.ncols = ex.rowmap ? ex.ncols : N;
     a.cf2 = ex.cf2;
     a.pass_w = p.pass_w;

@@ -337,13 +337,13 @@ class Sorter:
         self._check(self._lib.lss_reset_postprocess(self._h))
 
     def set_round_kernel(self, skip_blocks: bool):
-        """Rounds kernel: skip provably unchanged template-row blocks (True) or
-        update every row (False); the results are identical. The default is
-        True from 600 templates up."""
+        """Rounds kernel: update a block of template rows only once it can take
+        part in a decision (True) or every row in its round (False); the
+        results are identical. A sorter that was not told defers."""
         self._check(self._lib.lss_set_round_kernel(self._h, int(bool(skip_blocks))))
 
     def round_kernel(self) -> bool:
-        """True when the rounds skip provably unchanged template-row blocks."""
+        """The value last set; before that, True from 600 templates up."""
         import ctypes
         v = ctypes.c_int32(0)
         self._check(self._lib.lss_get_round_kernel(self._h, ctypes.byref(v)))
