@@ -14,25 +14,32 @@
 //   dL/dU[t]    = sum_{i: y_i = t} a_i P_i
 //   dL/dwPCA    = sum_i a_i sum_c U[y_i, :, c] G[c, x_i + (.) - nt/2]
 //   dL/da_i     = sum_{k, c} U[y_i, k, c] P_i[k, c]
-// Both passes are deterministic: the forward gathers per output column over
-// the spikes in time order, the backward runs one CTA per template over that
-// template's spikes in a fixed order and reduces dL/dwPCA over templates in
-// template order. F = float or double (the finite-difference checks run the
-// same kernels in FP64).
+// Both passes are deterministic (fixed orders, no atomics). F = float or double
+// (the finite-difference checks run the same kernels in FP64).
+//
+// The backward pass needs each spike's window of G only twice, an element at a
+// time: with S_t[c, m] = sum_{i: y_i = t} a_i G[c, x_i + m - nt/2],
+//   dL/dU[t]  = wPCA S_t^T,   dL/dwPCA = sum_t U[t] S_t,
+//   dL/da_i   = sum_{c, m} (sum_k U[y_i, k, c] wPCA[k, m]) G[c, x_i + m - nt/2],
+// so the K-fold contractions are taken once per template instead of per spike.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "lss.h"
 #include "lss_kernels.cuh"
 
 namespace lss {
 
-constexpr int RF_COLS = 128;   // output columns per CTA
-constexpr int RF_CH = 32;      // channels per CTA
-constexpr int RF_SP = 8;       // spikes staged per step
-constexpr int RB_CH = 32;      // channels per backward chunk
+constexpr int RF_COLS = 64;    // output columns per CTA (two warps of 32)
+constexpr int RF_CH = 128;     // channels per CTA (four groups of 32, one per warp)
+constexpr int RF_THREADS = 256;
 constexpr int RB_THREADS = 256;
+constexpr int RB_SP = 64;      // spikes whose dL/da shares are kept before they are summed over the cluster
+constexpr int RB_MAXZ = 8;     // CTAs of a cluster (portable limit)
 
 __device__ __forceinline__ int lower_bound_i(const int32_t* a, int n, int v) {
     int lo = 0, hi = n;
@@ -43,168 +50,294 @@ __device__ __forceinline__ int lower_bound_i(const int32_t* a, int n, int v) {
     return lo;
 }
 
-// xs/ys/as: spikes sorted by x.
-template <typename F>
-__global__ void __launch_bounds__(RF_COLS) k_recon_fwd(const F* __restrict__ U, const F* __restrict__ W, int K, int C,
-                                                       int nt, const int32_t* __restrict__ xs,
-                                                       const int32_t* __restrict__ ys, const F* __restrict__ as,
-                                                       int n, F* __restrict__ R, int64_t N) {
-    extern __shared__ unsigned char rf_smem[];
-    F* Ws = reinterpret_cast<F*>(rf_smem);       // [K][nt]
-    F* Us = Ws + K * nt;                          // [RF_SP][K][RF_CH]
-    __shared__ int s_x[RF_SP];
-    __shared__ F s_a[RF_SP];
-    const int h = nt / 2;
+// xs/ys/as: spikes sorted by x. A warp owns 32 columns (lane = column) of 32
+// channels (in registers) and takes the tile's spikes in time order, skipping
+// the ones whose window misses its columns: acc[c] += U[y, k, c] * (a W[k, m]).
+// U rows of SP spikes at a time are staged in shared memory (broadcast reads, 16
+// bytes each), W is staged once with 32 zeros on either side.
+// Bound by the FP32 pipe and shared-memory reads about equally: 9000 spikes at
+// 384 channels x 60000 samples are 2.5 GFLOP that must be done and 3.9 GFLOP done
+// (a window covers 61 of the 92 columns it is taken over), over 92 MB written.
+template <typename F, int SP>
+__global__ void __launch_bounds__(RF_THREADS) k_recon_fwd(const F* __restrict__ U, const F* __restrict__ W, int K,
+                                                          int C, int nt, const int32_t* __restrict__ xs,
+                                                          const int32_t* __restrict__ ys, const F* __restrict__ as,
+                                                          int n, F* __restrict__ R, int64_t N) {
+    extern __shared__ __align__(16) unsigned char rf_smem[];
+    F* Us = reinterpret_cast<F*>(rf_smem);        // [SP][K][RF_CH]
+    F* Ws = Us + SP * K * RF_CH;                   // [K][nt + 64]
+    __shared__ int s_x[SP];
+    __shared__ F s_a[SP];
+    const int h = nt / 2, wp = nt + 64;
     const int64_t t0 = (int64_t)blockIdx.x * RF_COLS;
     const int c0 = blockIdx.y * RF_CH;
-    const int nc = min(RF_CH, C - c0);
-    const int64_t col = t0 + threadIdx.x;
-    for (int e = threadIdx.x; e < K * nt; e += blockDim.x) Ws[e] = W[e];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wc = (warp >> 1) * 32;                       // the warp's channels, from c0
+    const int64_t w0 = t0 + (warp & 1) * 32;               // its first column
+    const int64_t col = w0 + lane;
+    const bool on = c0 + wc < C && w0 < N;
+    for (int e = threadIdx.x; e < K * wp; e += RF_THREADS) {
+        const int k = e / wp, m = e % wp - 32;
+        Ws[e] = (m >= 0 && m < nt) ? W[k * nt + m] : F(0);
+    }
     // spikes whose window [x - h, x - h + nt) meets [t0, t0 + RF_COLS)
     const int lo = lower_bound_i(xs, n, (int)(t0 - (nt - 1 - h)));
     const int hi = lower_bound_i(xs, n, (int)(t0 + RF_COLS + h));
-    F acc[RF_CH];
+    F acc[32];
 #pragma unroll
-    for (int c = 0; c < RF_CH; ++c) acc[c] = F(0);
-    for (int i0 = lo; i0 < hi; i0 += RF_SP) {
-        const int ns = min(RF_SP, hi - i0);
+    for (int c = 0; c < 32; ++c) acc[c] = F(0);
+    for (int i0 = lo; i0 < hi; i0 += SP) {
+        const int ns = min(SP, hi - i0);
         __syncthreads();
-        for (int e = threadIdx.x; e < ns * K * RF_CH; e += blockDim.x) {
-            const int q = e / (K * RF_CH), r = e % (K * RF_CH);
+        for (int e = threadIdx.x; e < ns * K * RF_CH; e += RF_THREADS) {
+            const int q = e / (K * RF_CH), r = e - q * (K * RF_CH);
             const int k = r / RF_CH, c = r % RF_CH;
-            Us[e] = (c < nc) ? U[((int64_t)ys[i0 + q] * K + k) * C + c0 + c] : F(0);
+            Us[e] = (c0 + c < C) ? U[((int64_t)ys[i0 + q] * K + k) * C + c0 + c] : F(0);
         }
         if (threadIdx.x < ns) {
             s_x[threadIdx.x] = xs[i0 + threadIdx.x];
             s_a[threadIdx.x] = as[i0 + threadIdx.x];
         }
         __syncthreads();
+        if (!on) continue;
         for (int q = 0; q < ns; ++q) {
-            const int m = (int)(col - s_x[q] + h);
-            if (m < 0 || m >= nt) continue;
+            const int64_t d = w0 - s_x[q] + h;             // lag of the warp's first column
+            if (d <= -32 || d >= nt) continue;
             const F a = s_a[q];
-            const F* uq = Us + q * K * RF_CH;
+            const F* wq = Ws + (int)d + lane + 32;
+            const F* uq = Us + q * K * RF_CH + wc;
+            for (int k = 0; k < K; ++k) {
+                const F b = a * wq[k * wp];
 #pragma unroll
-            for (int c = 0; c < RF_CH; ++c) {
-                F w = F(0);
-                for (int k = 0; k < K; ++k) w += uq[k * RF_CH + c] * Ws[k * nt + m];
-                acc[c] += a * w;
+                for (int c = 0; c < 32; ++c) acc[c] += uq[k * RF_CH + c] * b;
             }
         }
     }
-    if (col < N)
-        for (int c = 0; c < nc; ++c) R[(int64_t)(c0 + c) * N + col] = acc[c];
+    if (on && col < N) {
+        F* out = R + (int64_t)(c0 + wc) * N + col;
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+            if (c0 + wc + c < C) out[(int64_t)c * N] = acc[c];
+    }
 }
 
-// One CTA per template t; order[tstart[t] .. tstart[t+1]) are its spikes.
-template <typename F>
+// A cluster of Z CTAs per template t; order[tstart[t] .. tstart[t+1]) are its
+// spikes. CTA z takes channel chunks z, z + Z, ...: a warp's channels w + 8j (j <
+// CJ), lags lane + 32u (u < NM) of a window in registers, S and the template's
+// waveform beside them, so a spike costs one coalesced read and two FMAs per
+// element. The clusters' shared memories are then summed in rank order.
+// Bound by L2 reads of the windows (9000 spikes x 384 channels x 61 samples =
+// 843 MB; the 92 MB gradient stays in L2).
+template <typename F, int NM>
 __global__ void __launch_bounds__(RB_THREADS) k_recon_bwd(const F* __restrict__ U, const F* __restrict__ W, int K,
                                                           int C, int nt, const int32_t* __restrict__ x,
                                                           const F* __restrict__ amp, const int32_t* __restrict__ order,
                                                           const int32_t* __restrict__ tstart, const F* __restrict__ G,
                                                           int64_t N, F* __restrict__ dU, F* __restrict__ Qt,
                                                           F* __restrict__ damp) {
-    extern __shared__ unsigned char rb_smem[];
+    constexpr int CJ = 16 / NM, CH = 8 * CJ;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char rb_smem[];
+    const int ntp = nt | 1;
     F* Ws = reinterpret_cast<F*>(rb_smem);        // [K][nt]
-    F* Ut = Ws + K * nt;                           // [K][C]  U[t]
-    F* dUt = Ut + K * C;                           // [K][C]  accumulated dU[t]
-    F* Qa = dUt + K * C;                           // [K][nt] accumulated a_i * Q_i
-    F* win = Qa + K * nt;                          // [RB_CH][nt + 1]
-    F* red = win + RB_CH * (nt + 1);               // [RB_THREADS]
-    const int t = blockIdx.x;
+    F* Us = Ws + K * nt;                           // [K][CH]  U[t] of the chunk
+    F* S = Us + K * CH;                            // [CH][ntp]
+    F* Qp = S + CH * ntp;                          // [K][nt] this CTA's share of U[t] S_t
+    F* red = Qp + K * nt;                          // [RB_SP][8] shares of dL/da_i by warp
+    __shared__ int s_i[RB_SP], s_x[RB_SP];
+    __shared__ F s_a[RB_SP];
+    const int Z = (int)cl.num_blocks(), z = (int)cl.block_rank();
+    const int t = blockIdx.x / Z;
     const int h = nt / 2;
-    const int ntp = nt + 1;
-    for (int e = threadIdx.x; e < K * nt; e += blockDim.x) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int e = threadIdx.x; e < K * nt; e += RB_THREADS) {
         Ws[e] = W[e];
-        Qa[e] = F(0);
-    }
-    for (int e = threadIdx.x; e < K * C; e += blockDim.x) {
-        Ut[e] = U[(int64_t)t * K * C + e];
-        dUt[e] = F(0);
+        Qp[e] = F(0);
     }
     const int j0 = tstart[t], j1 = tstart[t + 1];
-    for (int j = j0; j < j1; ++j) {
-        const int i = order[j];
-        const int xi = x[i];
-        const F ai = amp[i];
-        F dsum = F(0);  // this thread's share of dL/da_i
-        for (int c0 = 0; c0 < C; c0 += RB_CH) {
-            const int nc = min(RB_CH, C - c0);
-            __syncthreads();
-            for (int e = threadIdx.x; e < nc * nt; e += blockDim.x) {
-                const int c = e / nt, m = e % nt;
-                const int64_t s = (int64_t)xi + m - h;
-                win[c * ntp + m] = (s >= 0 && s < N) ? G[(int64_t)(c0 + c) * N + s] : F(0);
-            }
-            __syncthreads();
-            // P_i[k, c] for the chunk: dU and dL/da_i
-            for (int e = threadIdx.x; e < nc * K; e += blockDim.x) {
-                const int c = e / K, k = e % K;
-                F p = F(0);
-                for (int m = 0; m < nt; ++m) p += Ws[k * nt + m] * win[c * ntp + m];
-                dUt[k * C + c0 + c] += ai * p;
-                dsum += Ut[k * C + c0 + c] * p;
-            }
-            // Q_i[k, m] over the chunk's channels (each (k, m) owned by one thread)
-            for (int e = threadIdx.x; e < K * nt; e += blockDim.x) {
-                const int k = e / nt, m = e % nt;
-                F q = F(0);
-                for (int c = 0; c < nc; ++c) q += Ut[k * C + c0 + c] * win[c * ntp + m];
-                Qa[e] += ai * q;
-            }
-        }
-        // dL/da_i: fixed-order tree reduction of the threads' shares
-        red[threadIdx.x] = dsum;
+    const int nchunk = (C + CH - 1) / CH;
+    for (int it = 0; it * Z < nchunk; ++it) {
+        const int c0 = (it * Z + z) * CH;  // past C: the CTA only takes part in the sums
         __syncthreads();
-        for (int w = RB_THREADS / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-            __syncthreads();
+        for (int e = threadIdx.x; e < K * CH; e += RB_THREADS) {
+            const int k = e / CH, c = e % CH;
+            Us[e] = (c0 + c < C) ? U[((int64_t)t * K + k) * C + c0 + c] : F(0);
         }
-        if (threadIdx.x == 0 && damp) damp[i] = red[0];
+        __syncthreads();
+        F s[CJ][NM], wv[CJ][NM];
+#pragma unroll
+        for (int j = 0; j < CJ; ++j)
+#pragma unroll
+            for (int u = 0; u < NM; ++u) {
+                const int m = lane + 32 * u;
+                F v = F(0);
+                if (m < nt)
+                    for (int k = 0; k < K; ++k) v += Us[k * CH + warp + 8 * j] * Ws[k * nt + m];
+                wv[j][u] = v;
+                s[j][u] = F(0);
+            }
+        for (int b0 = j0; b0 < j1; b0 += RB_SP) {
+            const int nb = min(RB_SP, j1 - b0);
+            __syncthreads();
+            if (threadIdx.x < nb) {
+                const int i = order[b0 + threadIdx.x];
+                s_i[threadIdx.x] = i;
+                s_x[threadIdx.x] = x[i];
+                s_a[threadIdx.x] = amp[i];
+            }
+            __syncthreads();
+            for (int q = 0; q < nb; ++q) {
+                const int64_t x0 = (int64_t)s_x[q] - h;
+                const F a = s_a[q];
+                const bool whole = x0 >= 0 && x0 + nt <= N;
+                F v[CJ][NM];
+                const F* g = G + (int64_t)(c0 + warp) * N + x0 + lane;
+#pragma unroll
+                for (int j = 0; j < CJ; ++j)
+#pragma unroll
+                    for (int u = 0; u < NM; ++u) {
+                        const int64_t p = x0 + lane + 32 * u;
+                        const bool in = lane + 32 * u < nt && c0 + warp + 8 * j < C && (whole || (p >= 0 && p < N));
+                        v[j][u] = in ? __ldg(g + (int64_t)(8 * j) * N + 32 * u) : F(0);
+                    }
+                F d = F(0);
+#pragma unroll
+                for (int j = 0; j < CJ; ++j)
+#pragma unroll
+                    for (int u = 0; u < NM; ++u) {
+                        s[j][u] += a * v[j][u];
+                        d += wv[j][u] * v[j][u];
+                    }
+                if (damp) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+                    if (lane == 0) red[q * 8 + warp] = d;
+                }
+            }
+            if (damp) {
+                // dL/da_i: over ranks and warps in order; later chunks add on
+                cl.sync();
+                if (z == 0 && threadIdx.x < nb) {
+                    F d = it ? damp[s_i[threadIdx.x]] : F(0);
+                    for (int r = 0; r < Z; ++r) {
+                        const F* rr = cl.map_shared_rank(red, r) + threadIdx.x * 8;
+                        for (int w = 0; w < 8; ++w) d += rr[w];
+                    }
+                    damp[s_i[threadIdx.x]] = d;
+                }
+                cl.sync();
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < CJ; ++j)
+#pragma unroll
+            for (int u = 0; u < NM; ++u)
+                if (lane + 32 * u < nt) S[(warp + 8 * j) * ntp + lane + 32 * u] = s[j][u];
+        __syncthreads();
+        for (int e = threadIdx.x; e < K * CH; e += RB_THREADS) {
+            const int k = e / CH, c = e % CH;
+            if (c0 + c >= C) continue;
+            F v = F(0);
+            for (int m = 0; m < nt; ++m) v += Ws[k * nt + m] * S[c * ntp + m];
+            dU[((int64_t)t * K + k) * C + c0 + c] = v;
+        }
+        for (int e = threadIdx.x; e < K * nt; e += RB_THREADS) {
+            const int k = e / nt, m = e % nt;
+            F v = F(0);
+            for (int c = 0; c < CH; ++c) v += Us[k * CH + c] * S[c * ntp + m];
+            Qp[e] += v;
+        }
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < K * C; e += blockDim.x) dU[(int64_t)t * K * C + e] = dUt[e];
-    for (int e = threadIdx.x; e < K * nt; e += blockDim.x) Qt[(int64_t)t * K * nt + e] = Qa[e];
+    cl.sync();
+    if (z == 0)
+        for (int e = threadIdx.x; e < K * nt; e += RB_THREADS) {
+            F v = F(0);
+            for (int r = 0; r < Z; ++r) v += cl.map_shared_rank(Qp, r)[e];
+            Qt[(int64_t)t * K * nt + e] = v;
+        }
+    cl.sync();  // the other ranks' shared memory is read until here
 }
 
+// dW[e] = sum_t Qt[t, e]: 32 columns per CTA, the templates strided over 8 rows
+// of threads, whose sums are combined in order
 template <typename F>
-__global__ void k_reduce_templates(const F* __restrict__ Qt, int T, int KN, F* __restrict__ dW) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= KN) return;
+__global__ void __launch_bounds__(256) k_reduce_templates(const F* __restrict__ Qt, int T, int KN, F* __restrict__ dW) {
+    __shared__ F part[8][32];
+    const int e = blockIdx.x * 32 + threadIdx.x;
     F s = F(0);
-    for (int t = 0; t < T; ++t) s += Qt[(int64_t)t * KN + e];
-    dW[e] = s;
+    if (e < KN)
+        for (int t = threadIdx.y; t < T; t += 8) s += Qt[(int64_t)t * KN + e];
+    part[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && e < KN) {
+        for (int r = 1; r < 8; ++r) s += part[r][threadIdx.x];
+        dW[e] = s;
+    }
 }
 
 template <typename F>
 static cudaError_t recon_fwd(const void* U, const void* W, int K, int C, int nt, const int32_t* xs, const int32_t* ys,
                              const void* as, int n, void* R, int64_t N, cudaStream_t s) {
-    const size_t smem = sizeof(F) * ((size_t)K * nt + (size_t)RF_SP * K * RF_CH);
+    constexpr int SP = sizeof(F) == 4 ? 8 : 4;
+    const size_t smem = sizeof(F) * ((size_t)SP * K * RF_CH + (size_t)K * (nt + 64));
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_recon_fwd<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(k_recon_fwd<F, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
     dim3 grid((unsigned)((N + RF_COLS - 1) / RF_COLS), (unsigned)((C + RF_CH - 1) / RF_CH));
-    k_recon_fwd<F><<<grid, RF_COLS, smem, s>>>(static_cast<const F*>(U), static_cast<const F*>(W), K, C, nt, xs, ys,
-                                               static_cast<const F*>(as), n, static_cast<F*>(R), N);
+    k_recon_fwd<F, SP><<<grid, RF_THREADS, smem, s>>>(static_cast<const F*>(U), static_cast<const F*>(W), K, C, nt, xs,
+                                                      ys, static_cast<const F*>(as), n, static_cast<F*>(R), N);
     return cudaGetLastError();
+}
+
+// NM: lags per lane (ceil(nt / 32) rounded up to a power of two)
+template <typename F, int NM>
+static cudaError_t recon_bwd_nm(const F* U, const F* W, int T, int K, int C, int nt, const int32_t* x, const F* amp,
+                                const int32_t* order, const int32_t* tstart, const F* G, int64_t N, F* dU, F* work,
+                                F* damp, cudaStream_t s) {
+    constexpr int CH = 8 * (16 / NM);
+    const size_t smem = sizeof(F) * (2 * (size_t)K * nt + (size_t)K * CH + (size_t)CH * (nt | 1) + RB_SP * 8);
+    auto kern = k_recon_bwd<F, NM>;
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    const int Z = std::min(RB_MAXZ, (C + CH - 1) / CH);
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)T * (unsigned)Z);
+    lc.blockDim = dim3(RB_THREADS);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)Z;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, kern, U, W, K, C, nt, x, amp, order, tstart, G, N, dU, work, damp);
 }
 
 template <typename F>
 static cudaError_t recon_bwd(const void* U, const void* W, int T, int K, int C, int nt, const int32_t* x,
                              const void* amp, const int32_t* order, const int32_t* tstart, const void* G, int64_t N,
                              void* dU, void* dW, void* damp, void* work, cudaStream_t s) {
-    const size_t smem = sizeof(F) * (2 * (size_t)K * nt + 2 * (size_t)K * C + (size_t)RB_CH * (nt + 1) + RB_THREADS);
-    if (smem > 227 * 1024) return cudaErrorInvalidValue;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_recon_bwd<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    k_recon_bwd<F><<<T, RB_THREADS, smem, s>>>(static_cast<const F*>(U), static_cast<const F*>(W), K, C, nt, x,
-                                               static_cast<const F*>(amp), order, tstart, static_cast<const F*>(G),
-                                               N, static_cast<F*>(dU), static_cast<F*>(work), static_cast<F*>(damp));
+    // channels and components are bounded as the shared memory of one CTA per template would bound them
+    if (sizeof(F) * (2 * (size_t)K * nt + 2 * (size_t)K * C + (size_t)32 * (nt + 1) + 256) > 227 * 1024)
+        return cudaErrorInvalidValue;
+    auto run = [&](auto kind) {
+        return recon_bwd_nm<F, decltype(kind)::value>(
+            static_cast<const F*>(U), static_cast<const F*>(W), T, K, C, nt, x, static_cast<const F*>(amp), order, tstart,
+            static_cast<const F*>(G), N, static_cast<F*>(dU), static_cast<F*>(work), static_cast<F*>(damp), s);
+    };
+    const cudaError_t e = nt <= 32    ? run(std::integral_constant<int, 1>())
+                          : nt <= 64  ? run(std::integral_constant<int, 2>())
+                          : nt <= 128 ? run(std::integral_constant<int, 4>())
+                                      : run(std::integral_constant<int, 8>());
+    if (e != cudaSuccess) return e;
     const int KN = K * nt;
-    k_reduce_templates<F><<<(KN + 255) / 256, 256, 0, s>>>(static_cast<const F*>(work), T, KN, static_cast<F*>(dW));
+    k_reduce_templates<F><<<(KN + 31) / 32, dim3(32, 8), 0, s>>>(static_cast<const F*>(work), T, KN, static_cast<F*>(dW));
     return cudaGetLastError();
 }
 
