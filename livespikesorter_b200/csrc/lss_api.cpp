@@ -754,7 +754,7 @@ int lss::run_scores(lss_handle* h, const float* X, int64_t ldx, int64_t N, float
     CK(launch_score_tc_tf32x3(h->B0T_hi.p, h->B0T_lo.p, h->CKpad, (int)N, folded ? h->Uw_hi.p : h->Up_hi.p,
                               folded ? h->Uw_lo.p : h->Up_lo.p, h->T, h->CKpad, h->nmq.p, B, h->ld, h->cfmax.p,
                               h->imax.p, h->nt, h->status.p, h->sm_count, s, ex));
-    h->stats.launches += 2 + (h->T > 256 ? 1 : 0);  // + the key maxima of a multi-pass GEMM
+    h->stats.launches += 2 + (h->T > 256 && !tiles ? 1 : 0);  // + the key maxima of a multi-pass GEMM over rows
     h->mark(6, s);
     if (maxima_ready) *maxima_ready = true;
     return LSS_OK;

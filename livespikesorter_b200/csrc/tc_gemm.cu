@@ -13,10 +13,10 @@
 //
 // Warp roles (192 threads): warp 0 issues TMA, warp 1 owns TMEM and issues the
 // MMAs (one elected lane), warps 2-5 drain the accumulator: each thread owns
-// one sample (TMEM lane), so the stores of B[t, s] for a fixed template are
-// 128-byte coalesced across a warp, and the same thread forms the column
-// maximum of Cf = relu(B)^2 / nm over all templates (the matching pursuit's
-// first Cfmax / imax), exactly as the rounds' kernel does.
+// one sample (TMEM lane) and stores its 16 scores of a tile of the deferred rounds
+// as 64 adjacent bytes (or, as rows, a template's scores 128 bytes at a time across
+// a warp). Where they are wanted, the same thread forms the column maximum of
+// Cf = relu(B)^2 / nm over all templates, exactly as the rounds do.
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag,
 // drains what it issued and frees its tensor memory before returning.
@@ -75,8 +75,10 @@ struct Args {
     const int32_t* perm;      // template of each operand row (null: the row's number)
     int tile_blocks;          // > 0: Bout as the deferred rounds' tiles, that many row blocks
     int ncols;                // samples in the batch (edge columns are the first/last nt)
-    float* cf2;               // runner-up Cf of each column (null: not tracked)
+    float* cf2;               // (error bounds) largest upper bound of any other template
     int pass_w;               // templates per pass (<= MAX_NP)
+    bool split;               // one work item per (sample tile, pass) instead of per tile
+    bool maxima;              // column maxima are wanted (the deferred rounds take theirs from the tiles)
     unsigned long long* keys; // split mode: one work item per (sample tile, pass); column maxima are
                               // combined as atomicMax of (Cf bits << 32 | ~t) (null: a CTA owns whole rows)
     // error bounds (BF16 path): |B - B_fp32| <= eps * un[t] * sqrt(pn2[s]) per score; per column
@@ -223,32 +225,38 @@ __device__ __forceinline__ void st_keep8(float* a, const uint32_t* v) {
                  : "memory");
 }
 
-// Running column maximum of Cf with the rounds kernel's exact rule, plus the
-// runner-up (to within the 3-ulp reciprocal approximation) when asked for.
+// Running column maximum of Cf = fl(fl(r*r) / nm) over a thread's scores, and
+// the largest and second largest upper bounds of Cf. One warp per scheduler runs
+// the epilogue, so nothing here branches: the quick quotient q = fl(fl(r*r) *
+// fl(1/nm)) errs by 3.01 * 2^-24, the running state is the largest q, its row and
+// score and the second largest q, and the exact quotient is formed once at the
+// end; only where the two are within 8 * 2^-24 are the rows looked at again. (A
+// branching form, with an exact quotient at every new maximum, bounded the BF16x3
+// GEMM at about 650 cycles per score: with rows in probe order the scores rise
+// step by step towards each unit. BF16x3 scores and re-check of 384 channels x 800
+// templates x 60122 columns: 1.57 -> 0.84 ms.)
 struct ColMax {
-    float best = -1.f;
-    float thr = -1.f;
-    float second = -1.f;
-    int bi = 0;
-    template <bool SECOND>
-    __device__ __forceinline__ void consider(float b, float nmv, float inv, int t, const int32_t* perm) {
-        const float r = fmaxf(b, 0.f);
-        const float sq = __fmul_rn(r, r);
-        const float approx = __fmul_rn(sq, inv);
-        if (approx < thr) {
-            if (SECOND) second = fmaxf(second, approx);
-            return;
-        }
-        const float cf = __fdiv_rn(sq, nmv);
-        // the smaller template on ties (rows in any order)
-        if (cf > best || (cf == best && perm && __ldg(perm + t) < __ldg(perm + bi))) {
-            if (SECOND) second = fmaxf(second, best);
-            best = cf;
-            bi = t;
-            thr = (cf >= 1e-30f) ? __fmul_rd(cf, 0.99999952316f) : -1.f;
-        } else if (SECOND) {
-            second = fmaxf(second, cf);
-        }
+    float q1 = -1.f, q2 = -1.f, vb = 0.f;
+    int tb = 0;
+    float hi1 = 0.f, hi2 = 0.f;
+    int thi1 = -1;
+    __device__ __forceinline__ void consider(float v, float inv, int t) {
+        const float r = fmaxf(v, 0.f);
+        const float q = __fmul_rn(__fmul_rn(r, r), inv);
+        q2 = fmaxf(q2, fminf(q1, q));
+        const bool up = q > q1;
+        q1 = fmaxf(q1, q);
+        vb = up ? v : vb;
+        tb = up ? t : tb;
+    }
+    // upper bound of the FP32 path's Cf for B within +-dB: directed rounding,
+    // then a margin for the reciprocal and the rounded squares
+    __device__ __forceinline__ void bound(float v, float dB, float inv, int t) {
+        const float bh = fmaxf(__fadd_ru(v, dB), 0.f);
+        const float hi = __fmul_ru(__fmul_ru(__fmul_ru(bh, bh), inv), 1.000001f);
+        hi2 = fmaxf(hi2, fminf(hi1, hi));
+        thi1 = hi > hi1 ? t : thi1;
+        hi1 = fmaxf(hi1, hi);
     }
 };
 
@@ -313,7 +321,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int ntiles = (rows + BM - 1) / BM;
     const int PW = a.pass_w;
     const int npass = (a.Tpad + PW - 1) / PW;
-    const bool split = a.keys != nullptr || a.part_keys != nullptr;
+    const bool split = a.split;
     const int items = split ? ntiles * npass : ntiles;
 
     if (warp == 0) {
@@ -430,12 +438,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             const bool valid = gr < rows && n < a.ncols;
             const bool edge = (n < a.nt) || (n >= a.ncols - a.nt);
             const bool bounds = a.un != nullptr;
-            const bool second = a.cf2 != nullptr && !bounds;
             ColMax m;
             // bound of this column's score errors per unit template norm
             const float epsp = (bounds && valid) ? __fmul_ru(a.eps, __fsqrt_ru(a.pn2[n])) : 0.f;
-            float lo_best = 0.f, hi1 = 0.f, hi2 = 0.f;
-            int thi1 = -1;
+            float* tile0 = a.Bout + ((int64_t)(n >> 5) * a.tile_blocks * 32 + (n & 31)) * MPB_ROWS;  // (tiles) this column's first rows
             for (int p = pb; p < pe; ++p) {
                 const int np = min(PW, a.Tpad - p * PW);
                 if (!mbar_wait(accf_bar(acc), acc_ph[acc], abort_flag, a.status)) { ok = false; break; }
@@ -449,39 +455,35 @@ __global__ void __launch_bounds__(THREADS, 1)
                         if (a.tile_blocks) {
                             // this thread's column of one tile: 64 bytes
                             static_assert(MPB_ROWS == 16, "one tile per 16 operand rows");
-                            float* bt = a.Bout + (((int64_t)(n >> 5) * a.tile_blocks + (t0 >> 4)) * 32 + (n & 31)) * MPB_ROWS;
-                            st_keep8(bt, r);
-                            st_keep8(bt + 8, r + 8);
-                        }
+                            st_keep8(tile0 + (int64_t)(t0 >> 4) * 32 * MPB_ROWS, r);
+                            st_keep8(tile0 + (int64_t)(t0 >> 4) * 32 * MPB_ROWS + 8, r + 8);
+                        } else {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int t = t0 + j;
-                            if (t < a.T) {
-                                const float v = __uint_as_float(r[j]);
-                                if (!a.tile_blocks)
-                                    st_keep(a.Bout + (int64_t)(a.perm ? __ldg(a.perm + t) : t) * a.ldb + n, v, pol);
-                                if (!edge) {
-                                    if (second) m.consider<true>(v, s_nm[t], s_inv[t], t, a.perm);
-                                    else m.consider<false>(v, s_nm[t], s_inv[t], t, a.perm);
-                                    if (bounds) {
-                                        // Cf of the FP32 path lies in [lo, hi]: B within +-dB,
-                                        // directed rounding, then a margin for the
-                                        // reciprocal and the rounded squares
-                                        const float dB = __fmul_ru(epsp, s_un[t]);
-                                        const float bh = fmaxf(__fadd_ru(v, dB), 0.f);
-                                        const float bl = fmaxf(__fsub_rd(v, dB), 0.f);
-                                        const float hi = __fmul_ru(__fmul_ru(__fmul_ru(bh, bh), s_inv[t]), 1.000001f);
-                                        const float lo = __fmul_rd(__fmul_rd(__fmul_rd(bl, bl), s_inv[t]), 0.999999f);
-                                        if (m.bi == t) lo_best = lo;  // t just became the best
-                                        if (hi > hi1) {
-                                            hi2 = hi1;
-                                            hi1 = hi;
-                                            thi1 = t;
-                                        } else {
-                                            hi2 = fmaxf(hi2, hi);
-                                        }
-                                    }
-                                }
+                            for (int j = 0; j < 16; ++j)
+                                if (t0 + j < a.T)
+                                    st_keep(a.Bout + (int64_t)(a.perm ? __ldg(a.perm + t0 + j) : t0 + j) * a.ldb + n,
+                                            __uint_as_float(r[j]), pol);
+                        }
+                    }
+                    // (rows past T are zero in the operand, their nm 1 and norm 0: never a maximum)
+                    if (a.maxima) {
+                        if (bounds) {
+#pragma unroll
+                            for (int j = 0; j < 16; j += 2) {
+                                const float2 inv = *reinterpret_cast<const float2*>(s_inv + t0 + j);
+                                const float2 un = *reinterpret_cast<const float2*>(s_un + t0 + j);
+                                const float v0 = __uint_as_float(r[j]), v1 = __uint_as_float(r[j + 1]);
+                                m.consider(v0, inv.x, t0 + j);
+                                m.bound(v0, __fmul_ru(epsp, un.x), inv.x, t0 + j);
+                                m.consider(v1, inv.y, t0 + j + 1);
+                                m.bound(v1, __fmul_ru(epsp, un.y), inv.y, t0 + j + 1);
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; j += 2) {
+                                const float2 inv = *reinterpret_cast<const float2*>(s_inv + t0 + j);
+                                m.consider(__uint_as_float(r[j]), inv.x, t0 + j);
+                                m.consider(__uint_as_float(r[j + 1]), inv.y, t0 + j + 1);
                             }
                         }
                     }
@@ -492,32 +494,59 @@ __global__ void __launch_bounds__(THREADS, 1)
                 acc_ph[acc] ^= 1u;
                 acc = (acc + 1) % a.nacc;
             }
-            if (ok && valid) {
-                if (a.perm) {  // operand rows to templates
-                    m.bi = __ldg(a.perm + m.bi);
-                    if (thi1 >= 0) thi1 = __ldg(a.perm + thi1);
+            if (ok && valid && a.maxima) {
+                // the best Cf and its first template
+                float best = 0.f, lo_best = 0.f;
+                int bi = 0;
+                if (!edge) {
+                    auto cf_of = [&](float v, int t) {
+                        const float rl = fmaxf(v, 0.f);
+                        return __fdiv_rn(__fmul_rn(rl, rl), s_nm[t]);
+                    };
+                    auto id_of = [&](int t) { return a.perm ? __ldg(a.perm + t) : t; };
+                    best = cf_of(m.vb, m.tb);
+                    bi = id_of(m.tb);
+                    if (!(m.q1 >= 1e-30f && m.q2 < __fmul_rd(m.q1, 0.99999952316f))) {
+                        // several rows may be the best: each in turn, read back as this thread wrote it
+                        const int t_end = min(a.T, pe * PW);
+                        best = -1.f;
+                        for (int t = pb * PW; t < t_end; ++t) {
+                            const int id = id_of(t);
+                            const float v = a.tile_blocks ? __ldcg(tile0 + (int64_t)(t >> 4) * 32 * MPB_ROWS + (t & 15))
+                                                          : __ldcg(a.Bout + (int64_t)id * a.ldb + n);
+                            const float cf = cf_of(v, t);
+                            if (cf > best || (cf == best && id < bi)) {
+                                best = cf;
+                                bi = id;
+                                m.tb = t;
+                                m.vb = v;
+                            }
+                        }
+                    }
+                    if (bounds) {
+                        // lower bound of the best template's Cf in the FP32 path
+                        const float bl = fmaxf(__fsub_rd(m.vb, __fmul_ru(epsp, s_un[m.tb])), 0.f);
+                        lo_best = __fmul_rd(__fmul_rd(__fmul_rd(bl, bl), s_inv[m.tb]), 0.999999f);
+                        if (m.thi1 >= 0) m.thi1 = id_of(m.thi1);
+                    }
                 }
                 if (split && bounds) {
                     const int64_t nc = a.ncols;
-                    const float cf = edge ? 0.f : fmaxf(m.best, 0.f);
-                    const uint32_t t = edge ? 0u : (uint32_t)m.bi;
-                    a.part_keys[pb * nc + n] = ((unsigned long long)__float_as_uint(cf) << 32) | (unsigned long long)(~t);
-                    a.part[(pb * 4 + 0) * nc + n] = edge ? 0.f : lo_best;
-                    a.part[(pb * 4 + 1) * nc + n] = edge ? 0.f : hi1;
-                    a.part[(pb * 4 + 2) * nc + n] = __int_as_float(edge ? -1 : thi1);
-                    a.part[(pb * 4 + 3) * nc + n] = edge ? 0.f : hi2;
+                    a.part_keys[pb * nc + n] =
+                        ((unsigned long long)__float_as_uint(best) << 32) | (unsigned long long)(~(uint32_t)bi);
+                    a.part[(pb * 4 + 0) * nc + n] = lo_best;
+                    a.part[(pb * 4 + 1) * nc + n] = edge ? 0.f : m.hi1;
+                    a.part[(pb * 4 + 2) * nc + n] = __int_as_float(edge ? -1 : m.thi1);
+                    a.part[(pb * 4 + 3) * nc + n] = edge ? 0.f : m.hi2;
                 } else if (split) {
-                    const float cf = edge ? 0.f : fmaxf(m.best, 0.f);
-                    const uint32_t t = edge ? 0u : (uint32_t)m.bi;
-                    atomicMax(a.keys + n, ((unsigned long long)__float_as_uint(cf) << 32) | (unsigned long long)(~t));
+                    atomicMax(a.keys + n, ((unsigned long long)__float_as_uint(best) << 32) | (unsigned long long)(~(uint32_t)bi));
                 } else {
-                    a.cfmax[n] = edge ? 0.f : m.best;
-                    a.imax[n] = edge ? 0 : m.bi;
-                    if (second) a.cf2[n] = edge ? 0.f : m.second;
+                    a.cfmax[n] = best;
+                    a.imax[n] = bi;
                     if (bounds) {
-                        a.cf2[n] = edge ? 0.f : ((thi1 == m.bi) ? hi2 : hi1);
-                        a.cf_lo[n] = edge ? 0.f : lo_best;
-                        a.cf_hi[n] = edge ? 0.f : hi1;
+                        a.cf2[n] = edge ? 0.f : ((m.thi1 == bi) ? m.hi2 : m.hi1);
+                        a.cf_lo[n] = lo_best;
+                        a.cf_hi[n] = edge ? 0.f : m.hi1;
                     }
                 }
             }
@@ -669,8 +698,10 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     const int tpad = (T + 15) / 16 * 16;
     const int npass = (tpad + 255) / 256;
     const int even_w = ((tpad + npass - 1) / npass + 15) / 16 * 16;
-    const bool split_map = ex.keys && ex.rowmap && ex.count_dev && !ex.cf2 && !ex.un && T > tc::MAPPED_SPLIT_W;
-    const bool split_short = ex.keys && !ex.cf2 && !ex.un && !ex.rowmap && 2 * ntiles < grid && T > tc::SPLIT_W;
+    // (the deferred rounds take the column maxima from the tiles' keys: none are formed here)
+    const bool maxima = !(ex.tile_blocks && !ex.un && !ex.rowmap);
+    const bool split_map = ex.keys && ex.rowmap && ex.count_dev && !ex.un && T > tc::MAPPED_SPLIT_W;
+    const bool split_short = (ex.keys || !maxima) && !ex.un && !ex.rowmap && 2 * ntiles < grid && T > tc::SPLIT_W;
     // Several passes over a full batch: one work item per (tile, pass), so that
     // a tile's passes run on consecutive CTAs at the same time and its sample
     // operand is read from DRAM once (tile by tile the passes would stream it
@@ -678,7 +709,7 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     // through keys, or per-pass partials for the error bounds.
     const bool bounds_part = ex.un && ex.part_keys && ex.part && (int64_t)npass * N <= ex.part_cap;
     const bool split_pass = !split_map && !split_short && !ex.rowmap && npass > 1 &&
-                            ((ex.keys && !ex.cf2 && !ex.un) || bounds_part);
+                            (((ex.keys || !maxima) && !ex.un) || bounds_part);
     const bool split = split_map || split_short || split_pass;
     const bool part_mode = split_pass && bounds_part;
     const TcPlan p = tc_plan(T, OP, split_map ? tc::MAPPED_SPLIT_W : (split_short ? tc::SPLIT_W : even_w));
@@ -718,6 +749,8 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     a.ncols = ex.rowmap ? ex.ncols : N;
     a.cf2 = ex.cf2;
     a.pass_w = p.pass_w;
+    a.split = split;
+    a.maxima = maxima;
     a.keys = (split && !part_mode) ? ex.keys : nullptr;
     a.part_keys = part_mode ? ex.part_keys : nullptr;
     a.part = part_mode ? ex.part : nullptr;
@@ -730,7 +763,7 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     cudaError_t e = cudaFuncSetAttribute(tc::k_score_tc<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
     if (e != cudaSuccess) return e;
     const int items = split ? ntiles * ((p.Tpad + p.pass_w - 1) / p.pass_w) : ntiles;
-    if (split && !part_mode) {
+    if (split && !part_mode && maxima) {
         e = cudaMemsetAsync(ex.keys, 0, (size_t)(split_map ? ex.ncols : N) * sizeof(unsigned long long), s);
         if (e != cudaSuccess) return e;
     }
@@ -741,7 +774,7 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     else if (split_map)
         tc::k_keys_to_maxima_mapped<<<(N + 255) / 256, 256, 0, s>>>(ex.keys, ex.rowmap, ex.count_dev, ex.map_rows, N,
                                                                     cfmax, imax);
-    else if (split)
+    else if (split && maxima)
         tc::k_keys_to_maxima<<<(N + 255) / 256, 256, 0, s>>>(ex.keys, N, cfmax, imax);
     return cudaGetLastError();
 }
