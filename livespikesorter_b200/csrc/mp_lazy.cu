@@ -138,7 +138,7 @@ __device__ __forceinline__ bool reaches(float ub, float th2) {
 template <bool KSMEM>
 __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_total, s_pref, s_nnew, s_qn, s_qnext;
+    __shared__ int s_total, s_pref, s_nnew, s_qn, s_qold, s_qnext;
     __shared__ int s_rcnt[MPL_REGIONS];
     __shared__ unsigned long long s_clk[PhaseClock::WORDS];
 
@@ -207,10 +207,26 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
     }
     for (int q = tid; q < ntile; q += MPL_THREADS) s_app[q] = -1;
     for (int c = tid; c < cpc; c += MPL_THREADS) s_touch[c] = 1;
-    if (tid == 0) s_qn = s_qnext = 0;
+    if (tid == 0) s_qn = s_qold = s_qnext = 0;
     __syncthreads();
     int n_app = 0, n_items = 0;  // (spike, tile) updates applied (per warp) and met (per lane)
 
+    // bounds {h, g} of a spike's ctc rows of block blk over the lags at which it
+    // meets the chunk that begins at c_lo
+    auto lag_bounds = [&](const int4& ev, int c_lo, int blk) {
+        const int g0 = max(c_lo - ev.x + nt, 0) / MPB_LAGS, g1 = (min(c_lo + 31, ev.y) - ev.x + nt) / MPB_LAGS;
+        const float2* hp = a.hg + ((int64_t)ev.z * ng + g0) * nb + blk;
+        float2 m = make_float2(0.f, 0.f), t[5];  // 32 lags lie in at most 5 groups of 8
+#pragma unroll
+        for (int u = 0; u < 5; ++u) t[u] = g0 + u <= g1 ? __ldg(hp + u * nb) : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 5; ++u) m = make_float2(fmaxf(m.x, t[u].x), fmaxf(m.y, t[u].y));
+        return m;
+    };
+    // smallest |score| of a tile from the lanes' minima
+    auto tile_min = [&](float mn, bool act) {
+        return __uint_as_float(__reduce_min_sync(FULL, act ? __float_as_uint(mn) : 0x7f800000u));
+    };
     // Brings tile q = c * nb + blk up to date with the log's first nlog
     // entries: its rows in registers (lane = column), the pending spikes'
     // terms one spike at a time, then its keys, bound and tmin.
@@ -228,68 +244,46 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
             for (int u = 0; u < MPB_ROWS; ++u)
                 if (u >= nr) v[u] = -INFINITY;
         }
-        int cur = s_app[q];
-        const bool changed = cur >= 0;
+        const int first = s_app[q];
+        const bool changed = first >= 0;
         float mn = INFINITY;
-        int wbase = max(cur, 0) & ~31;  // 32 log entries at a time: which of them reach the chunk
-        unsigned wmask = 0u;
-        auto scan = [&]() {
-            const int i = wbase + lane;
-            bool p = false;
-            if (i < nlog) {
-                const int4 e = s_log[i];
-                p = e.x - nt <= c_hi && e.y >= c_lo;
+        // 32 log entries at a time, lane = entry: hm = the largest |term| that
+        // the spike can have in the tile (-1: it does not reach the chunk), so
+        // that after each spike the next one that matters is a ballot away
+        for (int w0 = first; changed && w0 < nlog; w0 += 32) {
+            float hm = -1.f;
+            int4 ev = make_int4(0, 0, 0, 0);
+            if (w0 + lane < nlog) {
+                ev = s_log[w0 + lane];
+                if (ev.x - nt <= c_hi && ev.y >= c_lo) hm = fabsf(__fmul_rn(__int_as_float(ev.w), lag_bounds(ev, c_lo, blk).x));
             }
-            wmask = __ballot_sync(FULL, p);
-        };
-        auto next = [&](int after) -> int {  // first entry past `after` that reaches the chunk, -1: none
-            if (after + 1 - wbase < 32) {
-                const unsigned m = wmask & (FULL << (after + 1 - wbase));
-                if (m) return wbase + __ffs(m) - 1;
-            }
-            for (wbase += 32; wbase < nlog; wbase += 32) {
-                scan();
-                if (wmask) return wbase + __ffs(wmask) - 1;
-            }
-            return -1;
-        };
-        if (changed) scan();
-        while (cur >= 0) {
             // the first pending spike is known to change the tile; later ones
             // are tested against the scores that the ones before them left
-            const int4 e = s_log[cur];
-            const bool cov = act && s >= e.x - nt && s <= e.y;
-            const float amp = cov ? __int_as_float(e.w) : 0.f;
-            const float* cp = a.ctcP + (((int64_t)e.z * nb + blk) * L2 + (s - e.x + nt)) * MPB_ROWS;
+            float thr = quarter_ulp(tile_min(mn, act));
+            unsigned left = __ballot_sync(FULL, w0 == first ? lane == 0 : hm != -1.f && !(hm < thr));
+            while (left) {
+                const int l = __ffs(left) - 1;
+                const int x = __shfl_sync(FULL, ev.x, l), xe = __shfl_sync(FULL, ev.y, l);
+                const int y = __shfl_sync(FULL, ev.z, l), aw = __shfl_sync(FULL, ev.w, l);
+                const bool cov = act && s >= x - nt && s <= xe;
+                const float amp = cov ? __int_as_float(aw) : 0.f;
+                const float* cp = a.ctcP + (((int64_t)y * nb + blk) * L2 + (s - x + nt)) * MPB_ROWS;
 #pragma unroll
-            for (int u = 0; u < MPB_ROWS; u += 8) {
+                for (int u = 0; u < MPB_ROWS; u += 8) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) w[u + i] = 0.f;
-                if (cov) ld_ctc8(cp + u, w + u);
-            }
-            float hn = -1.f;  // largest |term| of the next spike in this column, -1: none
-            auto ld_h = [&](int i) {
-                const int4 en = s_log[i];
-                hn = -1.f;
-                if (act && s >= en.x - nt && s <= en.y)
-                    hn = fabsf(__fmul_rn(__int_as_float(en.w),
-                                         __ldg(a.hg + ((int64_t)en.z * ng + (s - en.x + nt) / MPB_LAGS) * nb + blk).x));
-            };
-            int nx = next(cur);
-            if (nx >= 0) ld_h(nx);
-            mn = INFINITY;
+                    for (int i = 0; i < 8; ++i) w[u + i] = 0.f;
+                    if (cov) ld_ctc8(cp + u, w + u);
+                }
+                mn = INFINITY;
 #pragma unroll
-            for (int u = 0; u < MPB_ROWS; ++u) {
-                v[u] = __fsub_rn(v[u], __fmul_rn(amp, w[u]));
-                mn = fminf(mn, fabsf(v[u]));
+                for (int u = 0; u < MPB_ROWS; ++u) {
+                    v[u] = __fsub_rn(v[u], __fmul_rn(amp, w[u]));
+                    mn = fminf(mn, fabsf(v[u]));
+                }
+                ++n_app;
+                thr = quarter_ulp(tile_min(mn, act));
+                left = __ballot_sync(FULL, hm != -1.f && !(hm < thr)) & ~(FULL >> (31 - l));
             }
-            ++n_app;
-            const float thr = quarter_ulp(mn);
-            while (nx >= 0 && !__any_sync(FULL, hn != -1.f && !(hn < thr))) {
-                nx = next(nx);
-                if (nx >= 0) ld_h(nx);
-            }
-            cur = nx;
         }
         if (!changed) {
 #pragma unroll
@@ -331,10 +325,10 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
             }
         }
         if (act) st_key(blk, c, k);
-        const unsigned tm = __reduce_min_sync(FULL, act ? __float_as_uint(mn) : 0x7f800000u);
+        const float tm = tile_min(mn, act);
         const unsigned cm = __reduce_max_sync(FULL, act ? (unsigned)(k >> 32) : 0u);
         if (lane == 0) {
-            s_tmin[q] = __uint_as_float(tm);
+            s_tmin[q] = tm;
             s_ub[q] = bound_of(__uint_as_float(cm));
             s_app[q] = -1;
         }
@@ -344,13 +338,13 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
     int todo_all = 1;  // every tile is due: 1 at the start (keys of the initial field), 2 when the log is full
     for (;; ++r) {
         // ---- the tiles that are due, one warp each
-        const int qn = todo_all ? qend : s_qn;
+        const int n_old = s_qold, qn = todo_all ? qend : s_qn + n_old;
         for (;;) {
             int i = 0;
             if (lane == 0) i = atomicAdd(&s_qnext, 1);
             i = __shfl_sync(FULL, i, 0);
             if (i >= qn) break;
-            const int q = todo_all ? i : s_queue[i];
+            const int q = todo_all ? i : s_queue[i < n_old ? i : ntile - 1 - (i - n_old)];
             if (todo_all != 2 || s_app[q] >= 0) resolve(q, nlog);
         }
         if (todo_all == 2) nlog = 0;  // nothing is pending: the log starts again
@@ -432,7 +426,7 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
                 s_amp[c * 32 + lane] = __fdiv_rn(__ldcg(tile_at(row / MPB_ROWS, c) + row % MPB_ROWS), s_nm[row]);
             }
         }
-        if (tid == 0) s_qn = s_qnext = 0;
+        if (tid == 0) s_qn = s_qold = s_qnext = 0;
         __syncthreads();
         // ---- publish: this CTA's peaks in time order, their count
         int own = 0;
@@ -578,27 +572,17 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
             for (int e = 0; e < n_new; ++e) {
                 const int4 ev = s_new[e];
                 if (ev.x - nt > c_hi || ev.y < c_lo) continue;
-                const int g0 = max(c_lo - ev.x + nt, 0) / MPB_LAGS, g1 = (min(c_hi, ev.y) - ev.x + nt) / MPB_LAGS;
-                float h = 0.f, g = 0.f;
                 if (blk < nb) {
-                    const float2* hp = a.hg + ((int64_t)ev.z * ng + g0) * nb + blk;
-                    float2 hv[6];  // 32 lags lie in at most 5 groups of 8; 6 keeps the loads in one batch
-#pragma unroll
-                    for (int u = 0; u < 6; ++u) hv[u] = g0 + u <= g1 ? __ldg(hp + u * nb) : make_float2(0.f, 0.f);
-#pragma unroll
-                    for (int u = 0; u < 6; ++u) {
-                        h = fmaxf(h, hv[u].x);
-                        g = fmaxf(g, hv[u].y);
-                    }
+                    const float2 hg = lag_bounds(ev, c_lo, blk);
                     if (!met) {
                         app = s_app[q];
                         ub = s_ub[q];
                         thr = quarter_ulp(s_tmin[q]);
                     }
                     const float amp = __int_as_float(ev.w);
-                    if (app >= 0 || !(fabsf(__fmul_rn(amp, h)) < thr)) {
+                    if (app >= 0 || !(fabsf(__fmul_rn(amp, hg.x)) < thr)) {
                         if (app < 0) app = nlog + e;
-                        ub = amp > 0.f ? __fmul_ru(__fadd_ru(ub, __fmul_ru(amp, g)), 1.000001f) : INFINITY;
+                        ub = amp > 0.f ? __fmul_ru(__fadd_ru(ub, __fmul_ru(amp, hg.y)), 1.000001f) : INFINITY;
                     }
                     ++n_items;
                 }
@@ -607,11 +591,19 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
             if (lane == 0 && blk < 32) s_touch[c] = met;
             if (met) {
                 const bool due = blk < nb && app >= 0 && reaches(ub, a.th2);
-                const unsigned bal = __ballot_sync(FULL, due);
-                int at = 0;
-                if (lane == 0 && bal) at = atomicAdd(&s_qn, __popc(bal));
-                at = __shfl_sync(FULL, at, 0) + __popc(bal & ((1u << lane) - 1u));
-                if (due) s_queue[at] = q;
+                // tiles with spikes from earlier rounds take longer: they go to the
+                // front of the queue, the others to its back
+                const bool old = due && app < nlog;
+                const unsigned b_old = __ballot_sync(FULL, old), b_new = __ballot_sync(FULL, due && !old);
+                int at_old = 0, at_new = 0;
+                if (lane == 0) {
+                    if (b_old) at_old = atomicAdd(&s_qold, __popc(b_old));
+                    if (b_new) at_new = atomicAdd(&s_qn, __popc(b_new));
+                }
+                const unsigned below = (1u << lane) - 1u;
+                at_old = __shfl_sync(FULL, at_old, 0) + __popc(b_old & below);
+                at_new = __shfl_sync(FULL, at_new, 0) + __popc(b_new & below);
+                if (due) s_queue[old ? at_old : ntile - 1 - at_new] = q;
                 if (blk < nb) {
                     s_app[q] = app;
                     s_ub[q] = ub;
