@@ -12,6 +12,7 @@
 #include "lss_kernels.cuh"
 
 #include <algorithm>
+#include <climits>
 
 namespace lss {
 
@@ -409,131 +410,326 @@ __device__ __forceinline__ void pc_features_one(
     }
 }
 
-// Warp per spike (projection-row path, nC = NCC and K = KPC known at compile
-// time): lane l sums channels l, l + 32, ... of every (j, k) feature, the 32
-// partial sums are combined by a butterfly, then each lane owns one or two
-// features for the neighbour corrections (list order) and the amp * Ucc term.
-constexpr int FW_LIST = 256;  // neighbours per spike (all rounds, within +-nt)
-template <int KPC, int NCC, typename PT>
-__global__ void __launch_bounds__(256, 2) k_pc_features_warp(
-    int32_t C, int32_t nt, int32_t T, const float* __restrict__ Mw, const float* __restrict__ U,
-    const float* __restrict__ R, const int64_t* __restrict__ iCC, const int64_t* __restrict__ iU,
-    const float* __restrict__ Ucc, const int32_t* __restrict__ sp_x, const int32_t* __restrict__ sp_y,
-    const float* __restrict__ sp_amp, const int32_t* __restrict__ round_start, int32_t rounds, int32_t n,
-    const int32_t* __restrict__ counters, float* __restrict__ tF, int32_t* status, const PT* __restrict__ Phi,
-    const PT* __restrict__ Plo, int64_t ldp) {
-    constexpr int F = NCC * KPC;
-    __shared__ int s_lx[8][FW_LIST], s_ly[8][FW_LIST];
-    __shared__ float s_la[8][FW_LIST];
-    if (counters) {
-        n = counters[0];
-        rounds = counters[1];
+// Projection-row path for ten nearest channels, K = KPC components known at
+// compile time. A CTA (one per SM) takes the spikes of `cols` columns: it first lists, in
+// matching order, every spike within nt of them (one pass over the spikes' columns
+// instead of a search of every round per spike); then a warp takes a spike at a
+// time. Lanes own quads of channels (whole lines of P and of the Mw rows per
+// load; a lane per feature reads ten lines per load and was bound by the L1) and
+// sum all ten channels' features over them; the partial sums are combined and
+// dealt out together, a lane keeping half the features at every step (the same
+// additions as a butterfly per feature: 62 shuffles instead of 300 for 60
+// features). Each lane then finishes its FP features: the neighbours' projected
+// waveforms, FS_NB loaded together and subtracted in list order, and amp * Ucc. A
+// neighbour whose template is exactly zero on all of the spike's channels (urange:
+// a template's first and last channel that is not) subtracts nothing and is not
+// loaded; templates are local, on a 384-channel probe three of four are skipped.
+// 384 channels, 19.3k spikes of 800 templates: 0.16 ms (0.40 with a search of
+// every round per spike, five butterfly steps per feature and a neighbour at a time).
+constexpr int FS_LIST = 1024;   // spikes listed per CTA (more: the warps read the spikes themselves)
+constexpr int FS_WARPS = 16;    // most warps of a CTA
+constexpr int FS_MIN_COLS = 16; // least columns of a CTA
+// neighbours per spike (all rounds, within +-nt), more are refused
+constexpr int fw_list(int K) { return K == 6 ? 256 : FT_LIST; }
+constexpr int FS_NC = 10;
+constexpr int FS_NB = 4;        // neighbours whose templates are loaded together
+
+// four projection values (hi or lo parts)
+__device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 ld4(const __nv_bfloat16* p) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+    const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.x));
+    const float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// One halving step: lanes with bit OFF of their number clear keep v[0 .. N),
+// the others v[N .. 2N), each plus its partner's.
+template <int N, int OFF>
+__device__ __forceinline__ void halve(float* v, int lane) {
+    const bool up = lane & OFF;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const float keep = up ? v[N + i] : v[i], give = up ? v[i] : v[N + i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, OFF);
     }
+}
+
+template <int KPC, typename PT>
+__global__ void __launch_bounds__(32 * FS_WARPS, 1) k_pc_features(
+    int32_t C, int32_t nt, int32_t T, const float* __restrict__ Mw, const float* __restrict__ Ut,
+    const int2* __restrict__ urange, const float* __restrict__ R, const int64_t* __restrict__ iCC,
+    const int64_t* __restrict__ iU, const float* __restrict__ Ucc, const int32_t* __restrict__ sp_x,
+    const int32_t* __restrict__ sp_y, const float* __restrict__ sp_amp, int32_t n, const int32_t* __restrict__ counters, float* __restrict__ tF,
+    int32_t* status, const PT* __restrict__ Phi, const PT* __restrict__ Plo, int64_t ldp, int32_t cols) {
+    constexpr int NC = FS_NC, F = NC * KPC, FP = (F + 31) / 32;
+    constexpr bool ONE_J = KPC % FP == 0;  // a lane's features belong to one channel
+    constexpr int NB = ONE_J ? FS_NB : FS_NB / 2;  // (registers)
+    extern __shared__ __align__(16) float fs_sm[];
+    constexpr int NW = FS_WARPS;
+    float* Rs = fs_sm;  // [lag][k'][k]: R[k, k', lag]
+    __shared__ int l_x[FS_LIST], l_y[FS_LIST], l_i[FS_LIST], l_own[FS_LIST];
+    __shared__ float l_a[FS_LIST];
+    __shared__ int s_cnt[FS_WARPS], s_ocnt[FS_WARPS], s_next;
+    __shared__ int s_ch[FS_WARPS][NC];  // the spike's channels
+    if (counters) n = counters[0];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const int nd = 2 * nt - 1;
-    for (int i = blockIdx.x * 8 + wl; i < n; i += gridDim.x * 8) {
-        const int x = sp_x[i], y = sp_y[i];
+    const int s0 = blockIdx.x * cols;
+    // ---- the spikes near the CTA's columns, in matching order: every warp
+    // counts its share of the spikes, then writes it
+    const int per = (((n + NW - 1) / NW) + 3) & ~3;  // whole groups of 4
+    const int i_lo = min(n, wl * per), i_hi = min(n, i_lo + per);
+    int n_list = 0, n_own = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        int c_all = 0, c_own = 0;
+        if (pass)
+            for (int w = 0; w < NW; ++w) {
+                if (w < wl) {
+                    c_all += s_cnt[w];
+                    c_own += s_ocnt[w];
+                }
+                n_list += s_cnt[w];
+                n_own += s_ocnt[w];
+            }
+        if (pass && n_list > FS_LIST) break;
+        for (int ib = i_lo; ib < i_hi; ib += 512) {
+            int xs[4][4];  // four groups of 128 spikes in flight
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const int i = ib + 128 * v + 4 * lane;
+                if (i + 4 <= i_hi) {
+                    const int4 q = __ldg(reinterpret_cast<const int4*>(sp_x + i));
+                    xs[v][0] = q.x;
+                    xs[v][1] = q.y;
+                    xs[v][2] = q.z;
+                    xs[v][3] = q.w;
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) xs[v][u] = i + u < i_hi ? __ldg(sp_x + i + u) : INT_MIN;
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+            const int i = ib + 128 * v + 4 * lane;
+            const int(&xv)[4] = xs[v];
+            int m = 0, own = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (xv[u] > s0 - nt && xv[u] < s0 + cols - 1 + nt) m |= 1 << u;
+                if (xv[u] >= s0 && xv[u] < s0 + cols) own |= 1 << u;
+            }
+            if (!__any_sync(0xffffffffu, m)) continue;
+            int inc = __popc(m), oinc = __popc(own);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, inc, o), b = __shfl_up_sync(0xffffffffu, oinc, o);
+                if (lane >= o) {
+                    inc += a;
+                    oinc += b;
+                }
+            }
+            if (pass) {
+                int at = c_all + inc - __popc(m), oat = c_own + oinc - __popc(own);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if ((m >> u) & 1) {
+                        l_x[at] = xv[u];
+                        l_y[at] = __ldg(sp_y + i + u);
+                        l_a[at] = __ldg(sp_amp + i + u);
+                        l_i[at] = i + u;
+                        if ((own >> u) & 1) l_own[oat++] = at;
+                        ++at;
+                    }
+            }
+            c_all += __shfl_sync(0xffffffffu, inc, 31);
+            c_own += __shfl_sync(0xffffffffu, oinc, 31);
+            }
+        }
+        if (!pass) {
+            if (lane == 0) {
+                s_cnt[wl] = c_all;
+                s_ocnt[wl] = c_own;
+            }
+            if (threadIdx.x == 0) s_next = NW;
+            __syncthreads();
+            int any = 0;
+            for (int w = 0; w < NW; ++w) any += s_ocnt[w];
+            if (!any) return;  // no spike in these columns
+            for (int p = wl; p < KPC * KPC; p += NW)  // a warp per pair of components
+#pragma unroll 4
+                for (int d = lane; d < nd; d += 32)
+                    Rs[d * (KPC * KPC) + (p % KPC) * KPC + p / KPC] = __ldg(R + (int64_t)p * nd + d);
+        }
+    }
+    __syncthreads();
+    const bool listed = n_list <= FS_LIST;
+    // spikes to scan for neighbours: the list, or (a list that is too long) all of them
+    const int n_scan = listed ? n_list : n;
+    for (int o = wl;;) {
+        // the o-th spike of the CTA's columns
+        int i = -1, x = 0, y = 0;
+        float amp = 0.f;
+        if (listed) {
+            if (o >= n_own) break;
+            const int e = l_own[o];
+            i = l_i[e];
+            x = l_x[e];
+            y = l_y[e];
+            amp = l_a[e];
+        } else {
+            if (o >= n) break;
+            i = o;
+            x = __ldg(sp_x + o);
+            y = __ldg(sp_y + o);
+            amp = __ldg(sp_amp + o);
+        }
+        int nx = 0;
+        if (lane == 0) nx = atomicAdd(&s_next, 1);
+        o = __shfl_sync(0xffffffffu, nx, 0);
+        if (x < s0 || x >= s0 + cols) continue;
         const int64_t u = iU[y];
-        int chl = 0;  // lane j < NCC holds channel j's index
-        if (lane < NCC) chl = (int)iCC[(int64_t)lane * C + u];
-        int ch[NCC];
+        int chl = 0;  // lane j < NC holds channel j's index
+        if (lane < NC) chl = (int)iCC[(int64_t)lane * C + u];
+        const int ch_min = __reduce_min_sync(0xffffffffu, lane < NC ? chl : INT_MAX);
+        const int ch_max = __reduce_max_sync(0xffffffffu, lane < NC ? chl : -1);
+        __syncwarp();
+        if (lane < NC) s_ch[wl][lane] = chl;
+        __syncwarp();
+        // ---- sums over channels: acc[j * K + k] = sum_c Mw[ch_j, c] * P[x, c*K + k]
+        float acc[32 * FP];
 #pragma unroll
-        for (int j = 0; j < NCC; ++j) ch[j] = __shfl_sync(0xffffffffu, chl, j);
-        // ---- sum over channels: acc[j][k] = sum_c Mw[ch_j, c] * P[x, c*K + k]
-        float acc[NCC][KPC];
+        for (int f = 0; f < 32 * FP; ++f) acc[f] = 0.f;
+        {
+            const PT* ph = Phi + (int64_t)x * ldp;
+            const PT* pl = Plo + (int64_t)x * ldp;
+            if ((C & 3) == 0) {  // (rows of P and Mw are then whole 16-byte pieces)
+                for (int c = 4 * lane; c < C; c += 128) {
+                    float pv[4 * KPC];
 #pragma unroll
-        for (int j = 0; j < NCC; ++j)
+                    for (int e = 0; e < 4 * KPC; e += 4) {
+                        const float4 h = ld4(ph + c * KPC + e), l = ld4(pl + c * KPC + e);
+                        pv[e] = __fadd_rn(h.x, l.x);
+                        pv[e + 1] = __fadd_rn(h.y, l.y);
+                        pv[e + 2] = __fadd_rn(h.z, l.z);
+                        pv[e + 3] = __fadd_rn(h.w, l.w);
+                    }
 #pragma unroll
-            for (int k = 0; k < KPC; ++k) acc[j][k] = 0.f;
-        const int64_t o = (int64_t)x * ldp;
-        for (int c = lane; c < C; c += 32) {
-            float pv[KPC];
+                    for (int j = 0; j < NC; ++j) {
+                        const float4 mv = ld4(Mw + (int64_t)s_ch[wl][j] * C + c);
 #pragma unroll
-            for (int k = 0; k < KPC; ++k) pv[k] = __fadd_rn(pval(Phi + o + c * KPC + k), pval(Plo + o + c * KPC + k));
+                        for (int k = 0; k < KPC; ++k) {
+                            float v = acc[j * KPC + k];
+                            v = fmaf(mv.x, pv[k], v);
+                            v = fmaf(mv.y, pv[KPC + k], v);
+                            v = fmaf(mv.z, pv[2 * KPC + k], v);
+                            acc[j * KPC + k] = fmaf(mv.w, pv[3 * KPC + k], v);
+                        }
+                    }
+                }
+            } else {
+                for (int c = lane; c < C; c += 32) {
+                    float pv[KPC];
 #pragma unroll
-            for (int j = 0; j < NCC; ++j) {
-                const float mv = __ldg(Mw + (int64_t)ch[j] * C + c);
+                    for (int k = 0; k < KPC; ++k) pv[k] = __fadd_rn(pval(ph + c * KPC + k), pval(pl + c * KPC + k));
 #pragma unroll
-                for (int k = 0; k < KPC; ++k) acc[j][k] = fmaf(mv, pv[k], acc[j][k]);
+                    for (int j = 0; j < NC; ++j) {
+                        const float mv = __ldg(Mw + (int64_t)s_ch[wl][j] * C + c);
+#pragma unroll
+                        for (int k = 0; k < KPC; ++k) acc[j * KPC + k] = fmaf(mv, pv[k], acc[j * KPC + k]);
+                    }
+                }
             }
         }
+        halve<16 * FP, 16>(acc, lane);
+        halve<8 * FP, 8>(acc, lane);
+        halve<4 * FP, 4>(acc, lane);
+        halve<2 * FP, 2>(acc, lane);
+        halve<FP, 1>(acc, lane);
+        // ---- this lane's features f = lane * FP + q
+        int jf[FP], kf[FP], cf[FP];
 #pragma unroll
-        for (int j = 0; j < NCC; ++j)
-#pragma unroll
-            for (int k = 0; k < KPC; ++k) {
-                float v = acc[j][k];
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-                acc[j][k] = v;  // every lane holds the total
-            }
-        // ---- neighbours (any round, round order) whose window overlaps x's
+        for (int q = 0; q < FP; ++q) {
+            const int f = min(lane * FP + q, F - 1);
+            jf[q] = f / KPC;
+            kf[q] = f % KPC;
+            cf[q] = s_ch[wl][jf[q]];
+        }
+        // ---- neighbours (any round, matching order) whose window overlaps x's
         int nl = 0;
-        for (int rb = 0; rb < rounds; rb += 32) {
-            const int r = rb + lane;
-            int lo = 0, cnt = 0;
-            if (r < rounds) {
-                const int b = round_start[r + 1];
-                int hi2 = b;
-                lo = round_start[r];
-                while (lo < hi2) {
-                    const int m = (lo + hi2) >> 1;
-                    if (sp_x[m] <= x - nt) lo = m + 1; else hi2 = m;
-                }
-                int e = lo;
-                while (e < b && sp_x[e] < x + nt) ++e;
-                cnt = e - lo;
-            }
-            int inc = cnt;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int v2 = __shfl_up_sync(0xffffffffu, inc, off);
-                if (lane >= off) inc += v2;
-            }
-            const int base = nl + inc - cnt;
-            for (int q = 0; q < cnt; ++q) {
-                const int slot = base + q;
-                if (slot < FW_LIST) {
-                    s_lx[wl][slot] = sp_x[lo + q];
-                    s_ly[wl][slot] = sp_y[lo + q];
-                    s_la[wl][slot] = sp_amp[lo + q];
+        for (int b0 = 0; b0 < n_scan; b0 += 32) {
+            const int e = b0 + lane;
+            int xq = INT_MIN, yq = 0;
+            float aq = 0.f;
+            if (e < n_scan) {
+                xq = listed ? l_x[e] : __ldg(sp_x + e);
+                if (xq > x - nt && xq < x + nt) {
+                    yq = listed ? l_y[e] : __ldg(sp_y + e);
+                    aq = listed ? l_a[e] : __ldg(sp_amp + e);
                 }
             }
-            nl += __shfl_sync(0xffffffffu, inc, 31);
-        }
-        __syncwarp();
-        if (nl > FW_LIST) {
-            if (lane == 0) atomicOr(status, STATUS_LIST);
-            nl = FW_LIST;
-        }
-        // ---- each lane finishes features f = lane and lane + 32
-#pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
-            const int f = lane + 32 * h2;
-            if (f >= F) break;
-            const int j = f / KPC, k = f % KPC;
-            float v = 0.f;
-#pragma unroll
-            for (int jj = 0; jj < NCC; ++jj)
-#pragma unroll
-                for (int kk = 0; kk < KPC; ++kk)
-                    if (jj * KPC + kk == f) v = acc[jj][kk];
-            int chj = 0;
-#pragma unroll
-            for (int jj = 0; jj < NCC; ++jj)
-                if (jj == j) chj = ch[jj];
-            for (int q = 0; q < nl; ++q) {
-                const int d = x - s_lx[wl][q];
-                const float* rk = R + ((int64_t)k * KPC) * nd + (d + nt - 1);
-                const float* uy = U + (int64_t)s_ly[wl][q] * KPC * C + chj;
-                float sub = 0.f;
-#pragma unroll
-                for (int kk = 0; kk < KPC; ++kk) sub = fmaf(__ldg(uy + (int64_t)kk * C), __ldg(rk + (int64_t)kk * nd), sub);
-                v = __fsub_rn(v, __fmul_rn(s_la[wl][q], sub));
+            const bool near = xq > x - nt && xq < x + nt;
+            nl += __popc(__ballot_sync(0xffffffffu, near));
+            bool some = near;  // (an infinite amplitude times zero is not zero)
+            if (near && fabsf(aq) < INFINITY) {
+                const int2 ur = __ldg(urange + yq);
+                some = ur.x <= ch_max && ur.y >= ch_min;
             }
-            v = __fadd_rn(v, __fmul_rn(sp_amp[i], Ucc[((int64_t)j * T + y) * KPC + k]));
-            tF[(int64_t)i * F + f] = v;
+            unsigned m = __ballot_sync(0xffffffffu, some);
+            while (m) {
+                // the next NB neighbours (an = 0 past the last: it subtracts nothing)
+                int d[NB];
+                float an[NB], uv[NB][ONE_J ? 1 : FP][KPC];
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    const int src = m ? __ffs(m) - 1 : 0;
+                    const int yn = __shfl_sync(0xffffffffu, yq, src);
+                    const float ab = __shfl_sync(0xffffffffu, aq, src);
+                    const int xb = __shfl_sync(0xffffffffu, xq, src);
+                    const bool on = m != 0u;
+                    m &= m - 1u;
+                    d[b] = on ? x - xb + nt - 1 : -1;
+                    an[b] = ab;
+                    if (on) {
+#pragma unroll
+                        for (int q = 0; q < (ONE_J ? 1 : FP); ++q) {
+                            const float* uy = Ut + ((int64_t)yn * C + cf[q]) * KPC;
+                            if constexpr (KPC % 2 == 0) {
+#pragma unroll
+                                for (int kk = 0; kk < KPC; kk += 2) {
+                                    const float2 t = __ldg(reinterpret_cast<const float2*>(uy + kk));
+                                    uv[b][q][kk] = t.x;
+                                    uv[b][q][kk + 1] = t.y;
+                                }
+                            } else {
+#pragma unroll
+                                for (int kk = 0; kk < KPC; ++kk) uv[b][q][kk] = __ldg(uy + kk);
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+                    if (d[b] >= 0) {
+#pragma unroll
+                        for (int q = 0; q < FP; ++q) {
+                            const float* rk = Rs + d[b] * (KPC * KPC) + kf[q];
+                            float sub = 0.f;
+#pragma unroll
+                            for (int kk = 0; kk < KPC; ++kk) sub = fmaf(uv[b][ONE_J ? 0 : q][kk], rk[kk * KPC], sub);
+                            acc[q] = __fsub_rn(acc[q], __fmul_rn(an[b], sub));
+                        }
+                    }
+            }
         }
-        __syncwarp();
+        if (nl > fw_list(KPC) && lane == 0) atomicOr(status, STATUS_LIST);
+#pragma unroll
+        for (int q = 0; q < FP; ++q) {
+            const int f = lane * FP + q;
+            if (f < F)
+                tF[(int64_t)i * F + f] =
+                    __fadd_rn(acc[q], __fmul_rn(amp, Ucc[((int64_t)jf[q] * T + y) * KPC + kf[q]]));
+        }
     }
 }
 
@@ -560,21 +756,52 @@ __global__ void __launch_bounds__(256) k_pc_features_folded(
     }
 }
 
+template <int KPC, typename PT>
+static cudaError_t launch_pcs(int32_t C, int32_t N, int32_t nt, int32_t T, const float* Mw, const float* Ut, const int2* urange, const float* R,
+                              const int64_t* iCC, const int64_t* iU, const float* Ucc, const int32_t* sp_x,
+                              const int32_t* sp_y, const float* sp_amp, int32_t n, const int32_t* counters, float* tF,
+                              int32_t* status, const PT* Phi, const PT* Plo, int64_t ldp, size_t smem, cudaStream_t s) {
+    const cudaError_t e = cudaFuncSetAttribute(k_pc_features<KPC, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    // one CTA per SM
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int cols = std::max(FS_MIN_COLS, (N + sms - 1) / std::max(sms, 1));
+    k_pc_features<KPC, PT><<<(N + cols - 1) / cols, 32 * FS_WARPS, smem, s>>>(C, nt, T, Mw, Ut, urange, R, iCC, iU, Ucc, sp_x, sp_y,
+                                                                          sp_amp, n, counters, tF, status, Phi, Plo, ldp,
+                                                                          cols);
+    return cudaGetLastError();
+}
+
 template <typename PT>
 static cudaError_t launch_pcf(const float* Xh, int64_t ldx, int32_t C, int32_t nt, int32_t K, int32_t nC, int32_t T,
-                              const float* wpca, const float* Mw, const float* U, const float* R, const int64_t* iCC,
-                              const int64_t* iU, const float* Ucc, const int32_t* sp_x, const int32_t* sp_y,
-                              const float* sp_amp, const int32_t* round_start, int32_t rounds, int32_t n,
+                              int32_t N, const float* wpca, const float* Mw, const float* U, const float* Ut,
+                              const int2* urange, const float* R, const int64_t* iCC, const int64_t* iU, const float* Ucc,
+                              const int32_t* sp_x, const int32_t* sp_y, const float* sp_amp,
+                              const int32_t* round_start, int32_t rounds, int32_t n,
                               const int32_t* counters, float* tF, int32_t* status, const PT* Phi, const PT* Plo,
                               int64_t ldp, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    if (Phi && K == 6 && nC == 10) {
-        // warp per spike; n: the spike count or (counters) the grid bound in spikes
-        const int grid = (n + 7) / 8;
-        k_pc_features_warp<6, 10, PT><<<grid, 256, 0, s>>>(C, nt, T, Mw, U, R, iCC, iU, Ucc, sp_x, sp_y, sp_amp,
-                                                           round_start, rounds, n, counters, tF, status, Phi, Plo,
-                                                           ldp);
-        return cudaGetLastError();
+    // ten channels: a CTA per SM while the basis correlations fit beside the lists in shared memory; else a CTA per
+    // spike
+    const size_t rs = 4 * (size_t)(2 * nt - 1) * K * K;
+    if (Phi && nC == FS_NC && K >= 1 && K <= 8 && rs <= 180 * 1024) {
+#define LSS_PCS(k)                                                                                                       \
+    case k:                                                                                                              \
+        return launch_pcs<k, PT>(C, N, nt, T, Mw, Ut, urange, R, iCC, iU, Ucc, sp_x, sp_y, sp_amp, n, counters, tF, status, Phi, \
+                                 Plo, ldp, rs, s)
+        switch (K) {
+            LSS_PCS(1);
+            LSS_PCS(2);
+            LSS_PCS(3);
+            LSS_PCS(4);
+            LSS_PCS(5);
+            LSS_PCS(6);
+            LSS_PCS(7);
+            LSS_PCS(8);
+        }
+#undef LSS_PCS
     }
     if (nC * K > 256) return cudaErrorInvalidValue;  // one (j, k) per thread
     const size_t front = std::max<size_t>((size_t)K * nt + (size_t)FT_CH * (nt + 1) + (size_t)FT_CH * K +
@@ -591,18 +818,19 @@ static cudaError_t launch_pcf(const float* Xh, int64_t ldx, int32_t C, int32_t n
 }
 
 cudaError_t launch_pc_features_folded(const float* Xh, int64_t ldx, int32_t C, int32_t nt, int32_t K, int32_t nC,
-                                      int32_t T, const float* wpca, const float* Mw, const float* U, const float* R,
-                                      const int64_t* iCC, const int64_t* iU, const float* Ucc, const int32_t* sp_x,
-                                      const int32_t* sp_y, const float* sp_amp, const int32_t* round_start,
+                                      int32_t T, int32_t N, const float* wpca, const float* Mw, const float* U,
+                                      const float* Ut, const int2* urange, const float* R, const int64_t* iCC, const int64_t* iU,
+                                      const float* Ucc, const int32_t* sp_x, const int32_t* sp_y, const float* sp_amp,
+                                      const int32_t* round_start,
                                       int32_t rounds, int32_t n, const int32_t* counters, float* tF,
                                       int32_t* status, const void* Phi, const void* Plo, int32_t p_bf16, int64_t ldp,
                                       cudaStream_t s) {
     if (p_bf16)
-        return launch_pcf<__nv_bfloat16>(Xh, ldx, C, nt, K, nC, T, wpca, Mw, U, R, iCC, iU, Ucc, sp_x, sp_y, sp_amp,
+        return launch_pcf<__nv_bfloat16>(Xh, ldx, C, nt, K, nC, T, N, wpca, Mw, U, Ut, urange, R, iCC, iU, Ucc, sp_x, sp_y, sp_amp,
                                          round_start, rounds, n, counters, tF, status,
                                          static_cast<const __nv_bfloat16*>(Phi),
                                          static_cast<const __nv_bfloat16*>(Plo), ldp, s);
-    return launch_pcf<float>(Xh, ldx, C, nt, K, nC, T, wpca, Mw, U, R, iCC, iU, Ucc, sp_x, sp_y, sp_amp, round_start,
+    return launch_pcf<float>(Xh, ldx, C, nt, K, nC, T, N, wpca, Mw, U, Ut, urange, R, iCC, iU, Ucc, sp_x, sp_y, sp_amp, round_start,
                              rounds, n, counters, tF, status, static_cast<const float*>(Phi),
                              static_cast<const float*>(Plo), ldp, s);
 }

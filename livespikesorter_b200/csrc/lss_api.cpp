@@ -166,9 +166,10 @@ int lss::rebuild_probe_order(lss_handle* h, const float* u) {
     CK(launch_template_operand(h->Uq.p, T, K, C, h->CKpad, h->Up_hi.p, h->Up_lo.p, bf16 ? h->Up16.p : nullptr,
                                bf16 ? h->Up16lo.p : nullptr, 0));
     h->un_p_stale = true;
+    CK(launch_transpose_u(h->U.p, T, K, C, h->Ut.p, h->urange.p, 0));
     CK(launch_tile_ctc(h->ctcP.p, h->mp_perm.p, h->nm.p, T, 2 * h->nt + 1, h->mp_ctct.p, h->mp_hg.p, 0));
     CK(cudaDeviceSynchronize());
-    h->stats.launches += 4;
+    h->stats.launches += 6;
     return LSS_OK;
 }
 
@@ -442,6 +443,8 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
     ALLOC(mp_perm, (size_t)h->mp_nb * MPB_ROWS);
     ALLOC(mp_hg, (size_t)T * h->mp_nb * mp_lag_groups((int)L2));
     ALLOC(Uq, (size_t)T * K * C);
+    ALLOC(Ut, (size_t)T * K * C);
+    ALLOC(urange, T);
     ALLOC(nmq, T);
     {
         const int64_t passes = ((T + 15) / 16 * 16 + 255) / 256;  // the score GEMM's template passes
@@ -1165,7 +1168,7 @@ static int sort_batch_impl(lss_handle* h, const int16_t* raw, int64_t n_rows, in
     if (need_tf) {
         // the projection rows of the score GEMM: tf32 parts (FP32 path) or bf16 parts (BF16 path)
         const int grid = std::min(n_bound, 16 * h->sm_count);
-        CK(launch_pc_features_folded(Xh, h->ld, h->C, h->nt, h->K, h->nC, h->T, h->wpca.p, h->Mw.p, h->U.p, h->R.p,
+        CK(launch_pc_features_folded(Xh, h->ld, h->C, h->nt, h->K, h->nC, h->T, h->N, h->wpca.p, h->Mw.p, h->U.p, h->Ut.p, h->urange.p, h->R.p,
                                      h->iCC.p, h->iU.p, h->Ucc.p, h->sp_x.p, h->sp_y.p, h->sp_amp.p,
                                      h->round_start.p, 0, grid, h->counters.p, h->tF.p, h->status.p,
                                      bf16 ? (const void*)h->B0T.p : (const void*)h->B0T_hi.p,

@@ -78,6 +78,8 @@ struct lss_handle {
     DevBuf<float> sc_part;                       // [passes, 4, ld] per-pass bound partials
     DevBuf<float> mp_ctct;                       // [T, nb, 2nt+1, MPB_ROWS] ctc by (spike template, block, lag), a block's rows adjacent
     DevBuf<float> Uq, nmq;                       // templates and energies in probe order
+    DevBuf<float> Ut;                            // [T, C, K] templates, components adjacent (PC features)
+    DevBuf<int2> urange;                         // [T] first and last channel of a template that is not zero
     // BF16 path (BF16x3 GEMM): projection and templates as bf16 hi / lo splits
     DevBuf<__nv_bfloat16> B0T, B0T16lo, Up16, Up16lo;
     DevBuf<float> B0T_hi, B0T_lo, Up_hi, Up_lo;  // FP32 path (3xTF32): tf32 hi/lo splits
@@ -166,7 +168,7 @@ struct lss_handle {
         tF.release(); iCC.release(); iU.release(); cfmax.release(); imax.release(); blk_cnt.release();
         blk_x.release(); blk_y.release(); sp_x.release(); sp_y.release(); sp_round.release();
         round_start.release(); counters.release(); status.release(); sp_amp.release(); blk_amp.release(); colkey.release();
-        mp_perm.release(); mp_hg.release(); mp_phase.release(); mp_xch.release(); mp_ctct.release(); Uq.release(); nmq.release(); sc_part_keys.release(); sc_part.release(); mp_bkey.release();
+        mp_perm.release(); mp_hg.release(); mp_phase.release(); mp_xch.release(); mp_ctct.release(); Uq.release(); nmq.release(); Ut.release(); urange.release(); sc_part_keys.release(); sc_part.release(); mp_bkey.release();
         bar.release(); rec_time.release(); rec_count.release(); rec_tmpl.release(); rec_slot.release(); rec_amp.release();
         rec_pc.release(); B0T.release(); B0T16lo.release(); Up16.release(); Up16lo.release();
         B0T_hi.release(); B0T_lo.release(); Up_hi.release(); Up_lo.release();

@@ -144,6 +144,9 @@ cudaError_t launch_row_norms(const float* hi, const float* lo, int32_t T, int64_
 cudaError_t launch_template_operand(const float* U, int32_t T, int32_t K, int32_t C, int64_t ldk, float* hi, float* lo,
                                     __nv_bfloat16* b16, __nv_bfloat16* b16lo, cudaStream_t s);
 
+// Ut[t, c, k] = U[t, k, c], urange[t] = first and last channel whose components are not all exactly zero (setup.cu)
+cudaError_t launch_transpose_u(const float* U, int32_t T, int32_t K, int32_t C, float* Ut, int2* urange, cudaStream_t s);
+
 // ---- matching pursuit (mp.cu) ----
 struct MPArgs {
     float* B;                 // [T, ldb] score field, updated in place
@@ -272,11 +275,15 @@ cudaError_t launch_records(const int32_t* sp_x, const int32_t* sp_y, const float
                            cudaStream_t s);
 // PC features from the highpassed batch (or, when Phi is given, the projection rows
 // P = Phi + Plo [N, ldp] of the score GEMM: fp32 tf32 parts, or bf16 parts when
-// p_bf16) and the folded whitening (no residual array)
+// p_bf16) and the folded whitening (no residual array); N columns, Ut [T, C, K] the
+// templates with their components adjacent, urange [T] their first and last channel
+// that is not exactly zero
 cudaError_t launch_pc_features_folded(const float* Xh, int64_t ldx, int32_t C, int32_t nt, int32_t K, int32_t nC,
-                                      int32_t T, const float* wpca, const float* Mw, const float* U, const float* R,
-                                      const int64_t* iCC, const int64_t* iU, const float* Ucc, const int32_t* sp_x,
-                                      const int32_t* sp_y, const float* sp_amp, const int32_t* round_start,
+                                      int32_t T, int32_t N, const float* wpca, const float* Mw, const float* U,
+                                      const float* Ut, const int2* urange, const float* R, const int64_t* iCC,
+                                      const int64_t* iU,
+                                      const float* Ucc, const int32_t* sp_x, const int32_t* sp_y, const float* sp_amp,
+                                      const int32_t* round_start,
                                       int32_t rounds, int32_t n, const int32_t* counters, float* tF,
                                       int32_t* status, const void* Phi, const void* Plo, int32_t p_bf16, int64_t ldp,
                                       cudaStream_t s);

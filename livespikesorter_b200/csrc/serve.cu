@@ -217,8 +217,8 @@ int enqueue_stream_batch(Probe* p) {
     const bool bf16 = h->cfg.precision == LSS_PREC_BF16_RECHECK;
     if (p->feat > 0) {
         const int grid = (int)std::min<int64_t>(p->cap, 2 * (int64_t)h->sm_count);
-        PCK(launch_pc_features_folded(Xh, h->ld, h->C, h->nt, h->K, h->nC, h->T, h->wpca.p, h->Mw.p, h->U.p,
-                                      h->R.p, h->iCC.p, h->iU.p, h->Ucc.p, h->sp_x.p, h->sp_y.p, h->sp_amp.p,
+        PCK(launch_pc_features_folded(Xh, h->ld, h->C, h->nt, h->K, h->nC, h->T, h->N, h->wpca.p, h->Mw.p, h->U.p,
+                                      h->Ut.p, h->urange.p, h->R.p, h->iCC.p, h->iU.p, h->Ucc.p, h->sp_x.p, h->sp_y.p, h->sp_amp.p,
                                       h->round_start.p, 0, grid, h->counters.p, h->tF.p, h->status.p,
                                       bf16 ? (const void*)h->B0T.p : (const void*)h->B0T_hi.p,
                                       bf16 ? (const void*)h->B0T16lo.p : (const void*)h->B0T_lo.p, bf16 ? 1 : 0,

@@ -21,6 +21,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -94,6 +95,36 @@ cudaError_t launch_template_operand(const float* U, int32_t T, int32_t K, int32_
                                     __nv_bfloat16* b16, __nv_bfloat16* b16lo, cudaStream_t s) {
     const int64_t n = (int64_t)T * C * K;
     k_up<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(U, T, K, C, ldk, hi, lo, b16, b16lo);
+    return cudaGetLastError();
+}
+
+__global__ void k_transpose_u(const float* __restrict__ U, int T, int K, int C, float* __restrict__ Ut) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (int64_t)T * C * K) return;
+    const int64_t t = e / ((int64_t)C * K);
+    const int r = (int)(e - t * C * K), c = r / K, k = r - c * K;
+    Ut[e] = U[(t * K + k) * C + c];
+}
+
+// one warp per template
+__global__ void k_channel_range(const float* __restrict__ U, int T, int K, int C, int2* __restrict__ urange) {
+    const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (t >= T) return;
+    int lo = INT_MAX, hi = -1;
+    for (int e = lane; e < K * C; e += 32)
+        if (!(U[(int64_t)t * K * C + e] == 0.f)) {
+            lo = min(lo, e % C);
+            hi = max(hi, e % C);
+        }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) urange[t] = make_int2(lo, hi);
+}
+
+cudaError_t launch_transpose_u(const float* U, int32_t T, int32_t K, int32_t C, float* Ut, int2* urange, cudaStream_t s) {
+    const int64_t n = (int64_t)T * C * K;
+    k_transpose_u<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(U, T, K, C, Ut);
+    k_channel_range<<<(T + 7) / 8, 256, 0, s>>>(U, T, K, C, urange);
     return cudaGetLastError();
 }
 
