@@ -32,31 +32,45 @@ __device__ __forceinline__ float tf32_rna(float x) {
     return __uint_as_float(r);
 }
 
+// Two FMAs per instruction on a register pair (each rounded on its own, so the
+// bits are fmaf's).
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long dup2(float x) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
+    return v;
+}
+
 // Thread = (channel, 8-sample group) with the channel fastest across a warp,
 // so the K values a thread writes per sample land next to its neighbours'
-// and a warp writes 32*K contiguous outputs per sample row.
+// and a warp writes 32*K contiguous outputs per sample row. The FP32 pipe bounds
+// it (17 GFLOP at 384 channels x 60122 samples, K = 6, nt = 61: 0.24 ms at the FP32
+// peak), so components go in pairs through packed FMAs and one sample load, one
+// duplication and K/4 weight loads serve 8K of them: 0.43 ms with the tf32 split
+// (0.49 with one FMA per instruction; a packed one takes the pipe two cycles, what
+// it saves is issue slots). A walk over several tiles per CTA with the next one's
+// samples copied ahead and rows staged per warp was slower (0.45 ms).
 template <int KPC, int PC, bool TF32, int NTP>
 __global__ void __launch_bounds__(256, KPC <= 6 ? 3 : 2) k_pca_proj_t(const float* __restrict__ X, int64_t ldx, int32_t C, int64_t N,
                                                     const float* __restrict__ wpca, int32_t nt, void* __restrict__ out0,
                                                     void* __restrict__ out_lo, int64_t ldk,
-                                                    const int32_t* __restrict__ tiles, const int32_t* __restrict__ ntiles,
                                                     float* __restrict__ norm2) {
-    extern __shared__ float sm[];
-    // tiles != null: CTA x projects sample tile tiles[x] into output rows x*PT_S.. (the first *ntiles entries)
-    if (tiles && (int)blockIdx.x >= *ntiles) return;
-    const int64_t s0 = tiles ? (int64_t)tiles[blockIdx.x] * PT_S : (int64_t)blockIdx.x * PT_S;
-    const int64_t o0 = (int64_t)blockIdx.x * PT_S;
+    extern __shared__ __align__(16) float sm[];
+    const int64_t s0 = (int64_t)blockIdx.x * PT_S;
     const int ntp = NTP ? NTP : (nt + 7) & ~7;     // taps padded to 8 (zero weights)
     const int xw = PT_S + ntp + 9;                 // staged samples per channel row (odd: no bank conflicts)
-    float* ws = sm;                                // [KPC][ntp]
-    float* xs = ws + KPC * ntp;                    // [PC][xw]
-    float* stage = xs + PC * xw + ((PC * xw) & 3 ? 4 - ((PC * xw) & 3) : 0);  // [PT_S][PC*KPC], 16-byte aligned
+    constexpr int KP = (KPC + 1) / 2;              // pairs of components (the last may be half empty)
+    float* ws = sm;                                // [ntp][2 KP]: a tap's components
+    float* xs = ws + 2 * KP * ntp;                 // [PC][xw]
+    float* stage = sm + ((2 * KP * ntp + PC * xw + 3) & ~3);  // [PT_S][PC*KPC], 16-byte aligned
     const int c0 = blockIdx.y * PC;
     const int nc = min(PC, C - c0);
     const int half = nt / 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    for (int k = warp; k < KPC; k += nwarps)
-        for (int m = lane; m < ntp; m += 32) ws[k * ntp + m] = (m < nt) ? wpca[k * nt + m] : 0.f;
+    for (int k = warp; k < 2 * KP; k += nwarps)
+        for (int m = lane; m < ntp; m += 32) ws[m * 2 * KP + k] = (m < nt && k < KPC) ? wpca[k * nt + m] : 0.f;
     if constexpr (NTP > 0 && PC % 8 == 0) {
         // fixed tap count: a warp's channel rows loaded into registers first, so
         // that all of them are in flight at once, then stored (256 threads)
@@ -94,36 +108,53 @@ __global__ void __launch_bounds__(256, KPC <= 6 ? 3 : 2) k_pca_proj_t(const floa
         const int c = task % PC, sg = task / PC;
         if (c >= nc) continue;
         const float* xr = xs + c * xw + sg * 8;
-        float acc[KPC][8];
+        unsigned long long acc[KP][8];
 #pragma unroll
-        for (int k = 0; k < KPC; ++k)
+        for (int k = 0; k < KP; ++k)
 #pragma unroll
-            for (int r = 0; r < 8; ++r) acc[k][r] = 0.f;
-        float w[16];
+            for (int r = 0; r < 8; ++r) acc[k][r] = 0ull;
+        // the samples that the current tap meets, twice each; sample r of tap m is x[(m + r) % 8]
+        unsigned long long x[8];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) w[r] = xr[r];
-        // every accumulator sums its taps in ascending order (one fmaf each)
+        for (int r = 0; r < 8; ++r) x[r] = dup2(xr[r]);
+        // every accumulator sums its taps in ascending order (one fma each)
 #pragma unroll(NTP ? NTP / 8 : 1)
         for (int mb = 0; mb < ntp; mb += 8) {
 #pragma unroll
-            for (int r = 0; r < 8; ++r) w[8 + r] = xr[mb + 8 + r];
+            for (int u = 0; u < 8; u += 2) {
+                // the weights of two taps (whole 16-byte pieces)
+                unsigned long long wt[2 * KP];
+                const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(ws + (mb + u) * 2 * KP);
 #pragma unroll
-            for (int k = 0; k < KPC; ++k) {
-                const float4 wa = *reinterpret_cast<const float4*>(ws + k * ntp + mb);
-                const float4 wb = *reinterpret_cast<const float4*>(ws + k * ntp + mb + 4);
-                const float tk[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+                for (int k = 0; k < KP; ++k) {
+                    const ulonglong2 p = wp[k];
+                    wt[2 * k] = p.x;
+                    wt[2 * k + 1] = p.y;
+                }
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
+                for (int v = 0; v < 2; ++v) {
 #pragma unroll
-                    for (int r = 0; r < 8; ++r) acc[k][r] = fmaf(tk[u], w[r + u], acc[k][r]);
+                    for (int k = 0; k < KP; ++k)
+#pragma unroll
+                        for (int r = 0; r < 8; ++r) fma2(acc[k][r], wt[v * KP + k], x[(u + v + r) & 7]);
+                    x[(u + v) & 7] = dup2(xr[mb + u + v + 8]);
+                }
             }
-#pragma unroll
-            for (int r = 0; r < 8; ++r) w[r] = w[8 + r];
         }
 #pragma unroll
         for (int r = 0; r < 8; ++r)
 #pragma unroll
-            for (int k = 0; k < KPC; ++k) stage[(sg * 8 + r) * (PC * KPC) + c * KPC + k] = acc[k][r];
+            for (int k = 0; k < KP; ++k) {
+                float lo, hi;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[k][r]));
+                float* d = stage + (sg * 8 + r) * (PC * KPC) + c * KPC + 2 * k;
+                if constexpr (KPC % 2 == 0) {
+                    *reinterpret_cast<float2*>(d) = make_float2(lo, hi);
+                } else {
+                    d[0] = lo;
+                    if (2 * k + 1 < KPC) d[1] = hi;
+                }
+            }
     }
     __syncthreads();
     // rows of nc*KPC outputs, written as 16-byte vectors (ldk and c0*KPC are
@@ -133,7 +164,7 @@ __global__ void __launch_bounds__(256, KPC <= 6 ? 3 : 2) k_pca_proj_t(const floa
     for (int r = warp; r < PT_S; r += nwarps) {
         const int64_t s = s0 + r;
         if (s >= N) continue;
-        const int64_t orow = (o0 + r) * ldk + (int64_t)c0 * KPC;
+        const int64_t orow = (s0 + r) * ldk + (int64_t)c0 * KPC;
         const float* srow = stage + r * (PC * KPC);
         for (int q = lane; q < nv4; q += 32) {
             const float4 v = *reinterpret_cast<const float4*>(srow + 4 * q);
@@ -185,41 +216,39 @@ __global__ void __launch_bounds__(256, KPC <= 6 ? 3 : 2) k_pca_proj_t(const floa
 
 template <int KPC, bool TF32>
 static cudaError_t launch_pjt(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t nt,
-                              void* out0, void* out_lo, int64_t ldk, const int32_t* tiles, const int32_t* ntiles,
-                              float* norm2, cudaStream_t s) {
+                              void* out0, void* out_lo, int64_t ldk, float* norm2, cudaStream_t s) {
     constexpr int PC = 32;
     const int ntp = (nt + 7) & ~7;
-    const size_t smem = sizeof(float) * ((size_t)KPC * ntp + (size_t)PC * (PT_S + ntp + 9) + 4 + (size_t)PT_S * PC * KPC);
+    const size_t smem = sizeof(float) * ((size_t)(KPC + 1) / 2 * 2 * ntp + (size_t)PC * (PT_S + ntp + 9) + 4 + (size_t)PT_S * PC * KPC);
     dim3 grid((unsigned)((N + PT_S - 1) / PT_S), (unsigned)((C + PC - 1) / PC));
     if (ntp == 64) {  // nt = 57..64 (Kilosort's 61): taps fully unrolled
         auto kern = k_pca_proj_t<KPC, PC, TF32, 64>;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2);
+        kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2);
     } else {
         auto kern = k_pca_proj_t<KPC, PC, TF32, 0>;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2);
+        kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2);
     }
     return cudaGetLastError();
 }
 
 template <bool TF32>
 static cudaError_t pjt_dispatch(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t K,
-                                int32_t nt, void* out0, void* out_lo, int64_t ldk, const int32_t* tiles,
-                                const int32_t* ntiles, float* norm2, cudaStream_t s) {
+                                int32_t nt, void* out0, void* out_lo, int64_t ldk, float* norm2, cudaStream_t s) {
     if (norm2) {
         const cudaError_t e = cudaMemsetAsync(norm2, 0, sizeof(float) * N, s);
         if (e != cudaSuccess) return e;
     }
     switch (K) {
-        case 1: return launch_pjt<1, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2, s);
-        case 2: return launch_pjt<2, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2, s);
-        case 3: return launch_pjt<3, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2, s);
-        case 4: return launch_pjt<4, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2, s);
-        case 5: return launch_pjt<5, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2, s);
-        case 6: return launch_pjt<6, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2, s);
-        case 7: return launch_pjt<7, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2, s);
-        case 8: return launch_pjt<8, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, tiles, ntiles, norm2, s);
+        case 1: return launch_pjt<1, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
+        case 2: return launch_pjt<2, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
+        case 3: return launch_pjt<3, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
+        case 4: return launch_pjt<4, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
+        case 5: return launch_pjt<5, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
+        case 6: return launch_pjt<6, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
+        case 7: return launch_pjt<7, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
+        case 8: return launch_pjt<8, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -227,12 +256,12 @@ static cudaError_t pjt_dispatch(const float* X, int64_t ldx, int32_t C, int64_t 
 cudaError_t launch_pca_proj_t(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t K,
                               int32_t nt, __nv_bfloat16* B0T_hi, __nv_bfloat16* B0T_lo, int64_t ldk, cudaStream_t s,
                               float* norm2) {
-    return pjt_dispatch<false>(X, ldx, C, N, wpca, K, nt, B0T_hi, B0T_lo, ldk, nullptr, nullptr, norm2, s);
+    return pjt_dispatch<false>(X, ldx, C, N, wpca, K, nt, B0T_hi, B0T_lo, ldk, norm2, s);
 }
 
 cudaError_t launch_pca_proj_t_tf32(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t K,
                                    int32_t nt, float* hi, float* lo, int64_t ldk, cudaStream_t s) {
-    return pjt_dispatch<true>(X, ldx, C, N, wpca, K, nt, hi, lo, ldk, nullptr, nullptr, nullptr, s);
+    return pjt_dispatch<true>(X, ldx, C, N, wpca, K, nt, hi, lo, ldk, nullptr, s);
 }
 
 
