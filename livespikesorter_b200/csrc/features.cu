@@ -10,6 +10,7 @@
 // * records: time = (x - nt) + ibatch*NT - nt/2 + nt0min, dropping negative
 //   times of batch 0 (template_matching.py:53-68), in run_matching order.
 #include "lss_kernels.cuh"
+#include "mp_common.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -31,7 +32,7 @@ __global__ void __launch_bounds__(XR_COLS) k_xres(const float* __restrict__ X, i
                                                   const int32_t* __restrict__ sp_y,
                                                   const float* __restrict__ sp_amp,
                                                   const int32_t* __restrict__ round_start, int32_t rounds,
-                                                  float* __restrict__ Xres, int32_t* status) {
+                                                  float* __restrict__ Xres, int64_t ldr, int32_t* status) {
     __shared__ int l_x[XR_LIST_MAX], l_y[XR_LIST_MAX];
     __shared__ float l_a[XR_LIST_MAX];
     __shared__ int r_cnt[XR_COLS], r_off[XR_COLS + 1];
@@ -57,13 +58,18 @@ __global__ void __launch_bounds__(XR_COLS) k_xres(const float* __restrict__ X, i
         }
         r_cnt[threadIdx.x] = cnt;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            int o = 0;
-            for (int i = 0; i < XR_COLS; ++i) {
-                r_off[i] = o;
-                o += r_cnt[i];
+        if (threadIdx.x < 32) {
+            constexpr int PL = XR_COLS / 32;
+            int v[PL], o = 0;
+#pragma unroll
+            for (int i = 0; i < PL; ++i) {
+                v[i] = o;
+                o += r_cnt[threadIdx.x * PL + i];
             }
-            r_off[XR_COLS] = o;
+            const int inc = warp_inc_scan(o, threadIdx.x);
+#pragma unroll
+            for (int i = 0; i < PL; ++i) r_off[threadIdx.x * PL + i] = inc - o + v[i];
+            if (threadIdx.x == 31) r_off[XR_COLS] = inc;
         }
         __syncthreads();
         for (int k = 0; k < cnt; ++k) {
@@ -83,8 +89,8 @@ __global__ void __launch_bounds__(XR_COLS) k_xres(const float* __restrict__ X, i
     }
     const int s = s0 + threadIdx.x;
     if (s >= N) return;
-    for (int c0 = 0; c0 < C; c0 += XR_CH) {
-        const int nc = min(XR_CH, C - c0);
+    {
+        const int c0 = blockIdx.y * XR_CH, nc = min(XR_CH, C - c0);
         float v[XR_CH];
 #pragma unroll
         for (int k = 0; k < XR_CH; ++k) v[k] = (k < nc) ? X[(int64_t)(c0 + k) * ldx + s] : 0.f;
@@ -99,18 +105,17 @@ __global__ void __launch_bounds__(XR_COLS) k_xres(const float* __restrict__ X, i
         }
 #pragma unroll
         for (int k = 0; k < XR_CH; ++k)
-            if (k < nc) Xres[(int64_t)(c0 + k) * ldx + s] = v[k];
+            if (k < nc) Xres[(int64_t)(c0 + k) * ldr + s] = v[k];
     }
 }
 
 cudaError_t launch_xres(const float* X, int64_t ldx, int32_t C, int32_t N, int32_t nt, const float* wave,
                         const int32_t* sp_x, const int32_t* sp_y, const float* sp_amp,
-                        const int32_t* round_start, const int32_t* counters, int32_t rounds,
-                        float* Xres, int32_t* status, cudaStream_t s) {
-    (void)counters;
-    const int grid = (N + XR_COLS - 1) / XR_COLS;
+                        const int32_t* round_start, int32_t rounds,
+                        float* Xres, int64_t ldr, int32_t* status, cudaStream_t s) {
+    const dim3 grid((N + XR_COLS - 1) / XR_COLS, (C + XR_CH - 1) / XR_CH);
     k_xres<<<grid, XR_COLS, 0, s>>>(X, ldx, C, N, nt, wave, sp_x, sp_y, sp_amp, round_start, rounds, Xres,
-                                     status);
+                                     ldr, status);
     return cudaGetLastError();
 }
 

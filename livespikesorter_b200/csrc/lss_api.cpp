@@ -621,7 +621,7 @@ int lss_set_drift(lss_handle* h, const float* M) {
 
 // ---------------------------------------------------------------- stages
 // Ingest of one padded batch. Xout (may be null) receives the whitened,
-// drift-corrected batch; *pre_out the highpassed batch before whitening.
+// drift-corrected batch (rows of ldo); *pre_out the highpassed batch before whitening.
 // The rows of a batch that are read (Kilosort's batch layout): the first
 // batch is NT + nt rows with the nt leading ones replicated, the last may be
 // short, the others are NT + 2nt.
@@ -650,7 +650,8 @@ static int batch_map(lss_handle* h, const int16_t* raw, int64_t n_rows, int64_t 
 }
 
 static int run_filter(lss_handle* h, const int16_t* raw, int64_t n_rows, int64_t ibatch, int64_t n_batches,
-                      int32_t raw_on_device, float* Xout, cudaStream_t s, const float** pre_out = nullptr) {
+                      int32_t raw_on_device, float* Xout, int64_t ldo, cudaStream_t s,
+                      const float** pre_out = nullptr) {
     IngestMap map;
     int rc = batch_map(h, raw, n_rows, ibatch, n_batches, map);
     if (rc) return rc;
@@ -661,10 +662,10 @@ static int run_filter(lss_handle* h, const int16_t* raw, int64_t n_rows, int64_t
         src = h->raw.p;
     }
     h->mark(1, s);
-    return run_ingest(h, src, map, Xout, s, pre_out);
+    return run_ingest(h, src, map, Xout, ldo, s, pre_out);
 }
 
-int lss::run_ingest(lss_handle* h, const int16_t* src, const IngestMap& map, float* Xout, cudaStream_t s,
+int lss::run_ingest(lss_handle* h, const int16_t* src, const IngestMap& map, float* Xout, int64_t ldo, cudaStream_t s,
                     const float** pre_out) {
     const int64_t N = h->N;
     const float sign = h->cfg.invert_sign ? -1.f : 1.f;
@@ -683,7 +684,7 @@ int lss::run_ingest(lss_handle* h, const int16_t* src, const IngestMap& map, flo
     }
     h->mark(3, s);
     if (Xout) {
-        CK(launch_sgemm(h->Mw.p, h->C, pre, h->ld, Xout, h->ld, h->C, (int)N, h->C, s));
+        CK(launch_sgemm(h->Mw.p, h->C, pre, h->ld, Xout, ldo, h->C, (int)N, h->C, s));
         h->stats.launches += 1;
     }
     h->mark(4, s);
@@ -842,9 +843,8 @@ static int run_mp(lss_handle* h, int64_t N, int32_t* n_out, int32_t* rounds_out,
 
 static int run_xres(lss_handle* h, const float* X, int64_t ldx, int64_t N, int rounds, float* Xres,
                     int64_t ldr, cudaStream_t s) {
-    (void)ldr;
     CK(launch_xres(X, ldx, h->C, (int)N, h->nt, h->wave.p, h->sp_x.p, h->sp_y.p, h->sp_amp.p,
-                   h->round_start.p, h->counters.p, rounds, Xres, h->status.p, s));
+                   h->round_start.p, rounds, Xres, ldr, h->status.p, s));
     h->stats.launches += 1;
     return LSS_OK;
 }
@@ -962,6 +962,18 @@ int lss_set_postprocess(lss_handle* h, const lss_post_config* pc) {
     return lss_reset_postprocess(h);
 }
 
+// May a kernel on `device` read or write p's floats in place? Else a copy is made, which takes whatever
+// cudaMemcpy takes (another device's memory, odd addresses) and refuses the rest with an error.
+static bool kernel_accessible(const void* p, int device) {
+    return (reinterpret_cast<uintptr_t>(p) & 3) == 0 && lss::device_accessible(p, device);
+}
+
+// The caller's batch [C, N] in the handle's buffer, rows of ld.
+static cudaError_t copy_batch(lss_handle* h, const float* X_dev, int64_t N, cudaStream_t s) {
+    return cudaMemcpy2DAsync(h->X.p, h->ld * sizeof(float), X_dev, N * sizeof(float), N * sizeof(float), h->C,
+                             cudaMemcpyDeviceToDevice, s);
+}
+
 int lss_filter(lss_handle* h, const int16_t* raw, int64_t n_rows, int64_t ibatch, int64_t n_batches,
                int32_t raw_on_device, float* X_dev, void* stream) {
     if (!h || !X_dev) return LSS_ERR_ARG;
@@ -969,11 +981,15 @@ int lss_filter(lss_handle* h, const int16_t* raw, int64_t n_rows, int64_t ibatch
     CK(cudaSetDevice(h->cfg.device));
     cudaStream_t s = (cudaStream_t)stream;
     CK(wait_mixing(h, s));
-    // the GEMM writes rows of stride ld; the caller's buffer has stride N
-    int rc = run_filter(h, raw, n_rows, ibatch, n_batches, raw_on_device, h->X.p, s);
-    if (rc) return rc;
-    CK(cudaMemcpy2DAsync(X_dev, h->N * sizeof(float), h->X.p, h->ld * sizeof(float), h->N * sizeof(float), h->C,
-                         cudaMemcpyDeviceToDevice, s));
+    if (kernel_accessible(X_dev, h->cfg.device)) {
+        int rc = run_filter(h, raw, n_rows, ibatch, n_batches, raw_on_device, X_dev, h->N, s);
+        if (rc) return rc;
+    } else {
+        int rc = run_filter(h, raw, n_rows, ibatch, n_batches, raw_on_device, h->X.p, h->ld, s);
+        if (rc) return rc;
+        CK(cudaMemcpy2DAsync(X_dev, h->N * sizeof(float), h->X.p, h->ld * sizeof(float), h->N * sizeof(float), h->C,
+                             cudaMemcpyDeviceToDevice, s));
+    }
     CK(cudaStreamSynchronize(s));
     return LSS_OK;
 }
@@ -985,14 +1001,25 @@ int lss_scores(lss_handle* h, const float* X_dev, int64_t N, float* B_dev, void*
     CK(cudaSetDevice(h->cfg.device));
     cudaStream_t s = (cudaStream_t)stream;
     CK(wait_mixing(h, s));
-    CK(cudaMemcpy2DAsync(h->X.p, h->ld * sizeof(float), X_dev, N * sizeof(float), N * sizeof(float), h->C,
-                         cudaMemcpyDeviceToDevice, s));
+    const float* X = X_dev;
+    int64_t ldx = N;
+    if (!kernel_accessible(X_dev, h->cfg.device)) {
+        CK(copy_batch(h, X_dev, N, s));
+        X = h->X.p;
+        ldx = h->ld;
+    }
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));
     // tiles, which the GEMM writes 64 bytes per thread at a time; one pass brings them into the caller's rows
-    int rc = run_scores(h, h->X.p, h->ld, N, h->B.p, s, nullptr, false, /*tiled=*/true);
+    const bool direct = kernel_accessible(B_dev, h->cfg.device);
+    int rc = run_scores(h, X, ldx, N, h->B.p, s, nullptr, false, /*tiled=*/direct);
     if (rc) return rc;
-    CK(launch_untile_scores(h->B.p, h->mp_perm.p, h->T, N, B_dev, N, s));
-    h->stats.launches += 1;
+    if (direct) {
+        CK(launch_untile_scores(h->B.p, h->mp_perm.p, h->T, N, B_dev, N, s));
+        h->stats.launches += 1;
+    } else {
+        CK(cudaMemcpy2DAsync(B_dev, N * sizeof(float), h->B.p, h->ld * sizeof(float), N * sizeof(float), h->T,
+                             cudaMemcpyDeviceToDevice, s));
+    }
     int32_t st = 0;
     CK(cudaMemcpyAsync(&st, h->status.p, sizeof(st), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1000,7 +1027,7 @@ int lss_scores(lss_handle* h, const float* X_dev, int64_t N, float* B_dev, void*
     return LSS_OK;
 }
 
-static int match_common(lss_handle* h, int64_t N, const float* Xsrc, int64_t* st_dev, float* amps_dev,
+static int match_common(lss_handle* h, int64_t N, const float* Xsrc, int64_t ldx, int64_t* st_dev, float* amps_dev,
                         float* xres_dev, int64_t capacity, int64_t* n_spikes, cudaStream_t s,
                         bool maxima_ready = false) {
     int32_t n = 0, rounds = 0;
@@ -1013,10 +1040,15 @@ static int match_common(lss_handle* h, int64_t N, const float* Xsrc, int64_t* st
         h->stats.launches += 1;
     }
     if (xres_dev && Xsrc) {
-        rc = run_xres(h, Xsrc, h->ld, N, rounds, h->Xres.p, h->ld, s);
-        if (rc) return rc;
-        CK(cudaMemcpy2DAsync(xres_dev, N * sizeof(float), h->Xres.p, h->ld * sizeof(float), N * sizeof(float), h->C,
-                             cudaMemcpyDeviceToDevice, s));
+        if (kernel_accessible(xres_dev, h->cfg.device)) {
+            rc = run_xres(h, Xsrc, ldx, N, rounds, xres_dev, N, s);
+            if (rc) return rc;
+        } else {
+            rc = run_xres(h, Xsrc, ldx, N, rounds, h->Xres.p, h->ld, s);
+            if (rc) return rc;
+            CK(cudaMemcpy2DAsync(xres_dev, N * sizeof(float), h->Xres.p, h->ld * sizeof(float), N * sizeof(float),
+                                 h->C, cudaMemcpyDeviceToDevice, s));
+        }
     }
     int32_t st = 0;
     CK(cudaMemcpyAsync(&st, h->status.p, sizeof(st), cudaMemcpyDeviceToHost, s));
@@ -1033,13 +1065,26 @@ int lss_match(lss_handle* h, const float* X_dev, int64_t N, int64_t* st_dev, flo
     CK(cudaSetDevice(h->cfg.device));
     cudaStream_t s = (cudaStream_t)stream;
     CK(wait_mixing(h, s));
-    CK(cudaMemcpy2DAsync(h->X.p, h->ld * sizeof(float), X_dev, N * sizeof(float), N * sizeof(float), h->C,
-                         cudaMemcpyDeviceToDevice, s));
+    const float* X = X_dev;
+    int64_t ldx = N;
+    // the batch is read again after the rounds: where an output shares its memory, from a copy
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(X_dev), x1 = x0 + sizeof(float) * (size_t)N * h->C;
+    auto shared = [&](const void* p, size_t bytes) {
+        const uintptr_t b = reinterpret_cast<uintptr_t>(p);
+        return p && b < x1 && x0 < b + bytes;
+    };
+    const size_t cap = capacity > 0 ? (size_t)capacity : 0;
+    if (!kernel_accessible(X_dev, h->cfg.device) || shared(xres_dev, x1 - x0) ||
+        (xres_dev && (shared(st_dev, 16 * cap) || shared(amps_dev, 4 * cap)))) {
+        CK(copy_batch(h, X_dev, N, s));
+        X = h->X.p;
+        ldx = h->ld;
+    }
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));
     bool ready = false;
-    int rc = run_scores(h, h->X.p, h->ld, N, h->B.p, s, &ready, false, h->mp_lazy);
+    int rc = run_scores(h, X, ldx, N, h->B.p, s, &ready, false, h->mp_lazy);
     if (rc) return rc;
-    return match_common(h, N, h->X.p, st_dev, amps_dev, xres_dev, capacity, n_spikes, s, ready);
+    return match_common(h, N, X, ldx, st_dev, amps_dev, xres_dev, capacity, n_spikes, s, ready);
 }
 
 int lss_match_scores(lss_handle* h, const float* B_dev, int64_t N, int64_t* st_dev, float* amps_dev,
@@ -1051,14 +1096,28 @@ int lss_match_scores(lss_handle* h, const float* B_dev, int64_t N, int64_t* st_d
     cudaStream_t s = (cudaStream_t)stream;
     CK(wait_mixing(h, s));
     if (h->mp_lazy) {  // the deferred rounds read the field as tiles
-        CK(launch_tile_scores(B_dev, N, h->mp_perm.p, h->T, N, h->B.p, s));
+        const float* B = B_dev;
+        float* tmp = nullptr;
+        if (!kernel_accessible(B_dev, h->cfg.device)) {
+            const size_t bytes = sizeof(float) * (size_t)N * h->T;
+            CK(cudaMallocAsync(reinterpret_cast<void**>(&tmp), bytes, s));
+            const cudaError_t e = cudaMemcpyAsync(tmp, B_dev, bytes, cudaMemcpyDeviceToDevice, s);
+            if (e != cudaSuccess) {
+                cudaFreeAsync(tmp, s);
+                CK(e);
+            }
+            B = tmp;
+        }
+        const cudaError_t e = launch_tile_scores(B, N, h->mp_perm.p, h->T, N, h->B.p, s);
+        if (tmp) cudaFreeAsync(tmp, s);
+        CK(e);
         h->stats.launches += 1;
     } else {
         CK(cudaMemcpy2DAsync(h->B.p, h->ld * sizeof(float), B_dev, N * sizeof(float), N * sizeof(float), h->T,
                              cudaMemcpyDeviceToDevice, s));
     }
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));
-    return match_common(h, N, nullptr, st_dev, amps_dev, nullptr, capacity, n_spikes, s);
+    return match_common(h, N, nullptr, 0, st_dev, amps_dev, nullptr, capacity, n_spikes, s);
 }
 
 static int sort_batch_impl(lss_handle* h, const int16_t* raw, int64_t n_rows, int64_t ibatch, int64_t n_batches,
@@ -1147,7 +1206,7 @@ static int sort_batch_impl(lss_handle* h, const int16_t* raw, int64_t n_rows, in
     // the whitening / drift matrix is folded into the templates (set_mixing), so
     // the scores come from the highpassed batch directly
     const float* Xh = nullptr;
-    int rc = run_filter(h, raw, n_rows, ibatch, n_batches, raw_on_device, nullptr, s, &Xh);
+    int rc = run_filter(h, raw, n_rows, ibatch, n_batches, raw_on_device, nullptr, 0, s, &Xh);
     if (rc) return rc;
     if (up_slot >= 0) CK(cudaEventRecord(h->raw_free[up_slot], s));
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));

@@ -200,7 +200,7 @@ namespace lss {
 
 // Ingest (channel sums, CAR, highpass; optional whitening into Xout) of the
 // batch whose raw rows `src` (device) are read through `map`.
-int run_ingest(lss_handle* h, const int16_t* src, const IngestMap& map, float* Xout, cudaStream_t s,
+int run_ingest(lss_handle* h, const int16_t* src, const IngestMap& map, float* Xout, int64_t ldo, cudaStream_t s,
                const float** pre_out);
 // Projection and score GEMM of X [C, ldx] into B; *maxima_ready when the
 // column maxima were fused into the GEMM. tiled: B as the deferred

@@ -225,8 +225,8 @@ cudaError_t launch_status_or(const int32_t* st, int32_t* acc, cudaStream_t s);
 // ---- residual and PC features (features.cu); n = spikes of the batch ----
 cudaError_t launch_xres(const float* X, int64_t ldx, int32_t C, int32_t N, int32_t nt, const float* wave,
                         const int32_t* sp_x, const int32_t* sp_y, const float* sp_amp,
-                        const int32_t* round_start, const int32_t* counters, int32_t rounds,
-                        float* Xres, int32_t* status, cudaStream_t s);
+                        const int32_t* round_start, int32_t rounds,
+                        float* Xres, int64_t ldr, int32_t* status, cudaStream_t s);
 // slot: scratch [n] for the output position of each spike
 struct RecordClock {
     int32_t presorted = 0;                 // output slots already computed (post-processing)

@@ -206,7 +206,7 @@ int enqueue_stream_batch(Probe* p) {
     map.base_dev = p->state.p + 1;
     map.ring_rows = p->R;
     const float* Xh = nullptr;
-    int rc = run_ingest(h, p->ring.p, map, nullptr, s, &Xh);
+    int rc = run_ingest(h, p->ring.p, map, nullptr, 0, s, &Xh);
     if (rc) return p->fail(rc, h->err);
     PCK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));
     bool ready = false;
