@@ -273,7 +273,7 @@ cudaError_t launch_highpass(const float* X1, int64_t ldx, int32_t C, int64_t N, 
 // once as the real and imaginary parts of a 4096-point complex signal (the
 // filter is real, so both come out of one transform): the block x[start-L ..
 // start-L+4096) (indices mod N) is transformed by a radix-16 Stockham FFT in
-// shared memory, multiplied by H = conj(FFT(g)) where g holds the taps wrapped
+// registers and shared memory, multiplied by H = conj(FFT(g)) where g holds the taps wrapped
 // around index 0 (a circular correlation), and transformed back; its outputs
 // L .. 4096-L-1 are exact (their taps never wrap inside the block).
 // ---------------------------------------------------------------------------
@@ -324,34 +324,56 @@ __device__ __forceinline__ void dft16(float2 v[16]) {
     for (int i = 0; i < 16; ++i) v[i] = t[i];
 }
 
-// One radix-16 Stockham pass (L = 1, 16, 256 known at compile time), in
-// place: one butterfly per thread (blockDim.x == HF / 16), every thread reads
-// its 16 inputs before any thread writes. One buffer instead of two lets four
-// CTAs share an SM.
+// The radix-16 Stockham passes (L = 1, 16, 256), one butterfly per thread
+// (blockDim.x == HF / 16), in place. Thread j takes the points j + 256 i of every
+// pass and leaves those of the last one, so the first pass starts from registers and
+// the last ends in them: the samples, the product with H and the outputs never pass
+// through shared memory, which a block crosses four times instead of sixteen. The
+// twiddle of point i is read from a table laid out [i][k] (i = 1..15, k < L),
+// neighbouring threads at neighbouring places; exp(-2 pi i n / 4096) by its n
+// put a warp's lanes on up to 30 lines per load.
 template <int L>
-__device__ __forceinline__ void fft16_pass(float2* a, const float2* __restrict__ tw) {
-    constexpr int step = HF / (16 * L);
-    constexpr int lg = (L == 1) ? 0 : (L == 16) ? 4 : 8;
-    const int j = threadIdx.x;
-    const int k = j & (L - 1), m = j >> lg;
-    float2 v[16];
+__device__ __forceinline__ void twiddle(float2 v[16], const float2* __restrict__ tw) {
+    const int k = threadIdx.x & (L - 1);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = a[pad16(j + (HF / 16) * i)];
-    if (L > 1) {
+    for (int i = 1; i < 16; ++i) v[i] = cmul(v[i], __ldg(tw + i * L + k));
+}
+
+template <int L>
+__device__ __forceinline__ void put(float2* a, const float2 v[16]) {
+    constexpr int lg = (L == 1) ? 0 : 4, step = (L == 1) ? 1 : 17;  // pad16(base + L * i) - pad16(base) = step * i
+    const int j = threadIdx.x, base = (j >> lg) * 16 * L + (j & (L - 1));
+    a += pad16(base);
 #pragma unroll
-        for (int i = 1; i < 16; ++i) v[i] = cmul(v[i], __ldg(tw + ((i * k * step) & (HF - 1))));
-    }
+    for (int i = 0; i < 16; ++i) a[step * i] = v[i];
+    __syncthreads();
+}
+
+__device__ __forceinline__ void get(const float2* a, float2 v[16]) {
+    a += pad16(threadIdx.x);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = a[pad16((HF / 16) * i)];
+}
+
+__device__ __forceinline__ void fft4096(float2 v[16], float2* a, const float2* __restrict__ tw) {
+    dft16(v);
+    put<1>(a, v);
+    get(a, v);
+    twiddle<16>(v, tw + 16 * 256);
     dft16(v);
     __syncthreads();
-    const int base = m * 16 * L + k;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) a[pad16(base + L * i)] = v[i];
-    __syncthreads();
+    put<16>(a, v);
+    get(a, v);
+    twiddle<256>(v, tw);
+    dft16(v);
 }
 
 constexpr int HF_THREADS = HF / 16;
 
-__global__ void __launch_bounds__(HF_THREADS, 4) k_highpass_fft(const float* __restrict__ X1, int64_t ldx, int32_t C,
+// Bound by its FP32 adds and multiplies (about 50 us at the full rate for 384 x 60122, L = 500) with the shared-memory
+// passes beside them: 93 us, against 242 with every pass through shared memory. Two CTAs per SM: the 16 points, their
+// twiddles and a butterfly's temporaries take 128 registers (118 and 116 us with four and three CTAs, which spill).
+__global__ void __launch_bounds__(HF_THREADS, 2) k_highpass_fft(const float* __restrict__ X1, int64_t ldx, int32_t C,
                                                                int64_t N, int32_t L, const float2* __restrict__ H,
                                                                const float2* __restrict__ tw, float* __restrict__ Xh) {
     extern __shared__ float2 A[];  // [HFP]: one padded 4096-point buffer, transformed in place
@@ -360,45 +382,42 @@ __global__ void __launch_bounds__(HF_THREADS, 4) k_highpass_fft(const float* __r
     const int64_t start = (int64_t)blockIdx.x * (HF - 2 * L);
     const float* x1 = X1 + (int64_t)c1 * ldx;
     const float* x2 = X1 + (int64_t)(two ? c2 : c1) * ldx;
-    // 4 samples per thread loaded before they are stored (8 loads in flight)
-    static_assert(HF % (4 * HF_THREADS) == 0, "whole groups of 4 samples per thread");
+    float2 v[16];
+    if (start - L >= 0 && start - L + HF <= N) {
+        x1 += start - L + threadIdx.x;
+        x2 += start - L + threadIdx.x;
 #pragma unroll
-    for (int i0 = 0; i0 < HF / HF_THREADS; i0 += 4) {
-        float v1[4], v2[4];
+        for (int i = 0; i < 16; ++i) v[i].x = x1[i * HF_THREADS];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int n = threadIdx.x + (i0 + u) * HF_THREADS;
-            int64_t g = start - L + n;  // circular index (the modulo only near the ends)
-            if (g < 0 || g >= N) {
-                g %= N;
-                if (g < 0) g += N;
-            }
-            v1[u] = x1[g];
-            v2[u] = two ? x2[g] : 0.f;
+        for (int i = 0; i < 16; ++i) v[i].y = two ? x2[i * HF_THREADS] : 0.f;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {  // the ends wrap around
+            int g = ((int)(start - L) + (int)threadIdx.x + i * HF_THREADS) % (int)N;
+            if (g < 0) g += (int)N;
+            v[i] = make_float2(x1[g], two ? x2[g] : 0.f);
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) A[pad16(threadIdx.x + (i0 + u) * HF_THREADS)] = make_float2(v1[u], v2[u]);
     }
-    __syncthreads();
-    fft16_pass<1>(A, tw);
-    fft16_pass<16>(A, tw);
-    fft16_pass<256>(A, tw);
+    fft4096(v, A, tw);
     // conj(Z * H): the second forward transform then gives conj(F * y)
-    for (int n = threadIdx.x; n < HF; n += HF_THREADS) {
-        const float2 z = cmul(A[pad16(n)], __ldg(H + n));
-        A[pad16(n)] = make_float2(z.x, -z.y);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float2 z = cmul(v[i], __ldg(H + threadIdx.x + i * HF_THREADS));
+        v[i] = make_float2(z.x, -z.y);
     }
     __syncthreads();
-    fft16_pass<1>(A, tw);
-    fft16_pass<16>(A, tw);
-    fft16_pass<256>(A, tw);
+    fft4096(v, A, tw);
     const float inv = 1.f / (float)HF;
-    for (int n = L + threadIdx.x; n < HF - L; n += HF_THREADS) {
-        const int64_t i = start + (n - L);
-        if (i >= N) break;
-        const float2 r = A[pad16(n)];
-        Xh[(int64_t)c1 * ldx + i] = r.x * inv;
-        if (two) Xh[(int64_t)c2 * ldx + i] = -r.y * inv;
+    const int nend = (int)min((int64_t)(HF - L), N - start + L);
+    float* y1 = Xh + (int64_t)c1 * ldx + (start - L + threadIdx.x);
+    float* y2 = y1 + ldx;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int n = threadIdx.x + i * HF_THREADS;
+        if (n >= L && n < nend) {
+            y1[i * HF_THREADS] = v[i].x * inv;
+            if (two) y2[i * HF_THREADS] = -v[i].y * inv;
+        }
     }
 }
 

@@ -417,7 +417,7 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
     const bool hp_fft = h->hpL >= 0 && h->hpL <= 1024;
     if (hp_fft) {
         ALLOC(hpH, 4096);
-        ALLOC(hpTw, 4096);
+        ALLOC(hpTw, 4096 + 256);
     }
     ALLOC(R, (size_t)K * K * (2 * nt - 1));
     ALLOC(B, (size_t)((T + MPB_ROWS - 1) / MPB_ROWS * MPB_ROWS) * ld);  // rows [T, ld], or tiles of whole row blocks
@@ -525,7 +525,13 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
             tv[k] = make_float2((float)std::cos(ang), (float)std::sin(ang));
         }
         CK(cudaMemcpy(h->hpH.p, hv.data(), F * sizeof(float2), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->hpTw.p, tv.data(), F * sizeof(float2), cudaMemcpyHostToDevice));
+        // the passes' order: [16][256] exp(-2 pi i (i k) / 4096), then [16][16] exp(-2 pi i (i k) / 256)
+        std::vector<float2> tp(F + 256);
+        for (int i = 0; i < 16; ++i) {
+            for (int k = 0; k < 256; ++k) tp[i * 256 + k] = tv[i * k];
+            for (int k = 0; k < 16; ++k) tp[F + i * 16 + k] = tv[i * k * 16];
+        }
+        CK(cudaMemcpy(h->hpTw.p, tp.data(), tp.size() * sizeof(float2), cudaMemcpyHostToDevice));
     }
     {
         // R[k, k', d] = sum_m wPCA[k, m] * wPCA[k', m + d], d = -(nt-1) .. nt-1

@@ -32,7 +32,8 @@ cudaError_t launch_car(const int16_t* raw, int32_t ld_raw, const int32_t* chan_m
                        int64_t ldx, cudaStream_t s);
 cudaError_t launch_highpass(const float* X1, int64_t ldx, int32_t C, int64_t N, const float* taps, int32_t L,
                             float* Xh, cudaStream_t s);
-// overlap-save FFT form (L <= 1024): H = conj(FFT_4096(taps wrapped around 0)), tw[k] = exp(-2 pi i k / 4096)
+// overlap-save FFT form (L <= 1024): H = conj(FFT_4096(taps wrapped around 0)), tw = [16][256] exp(-2 pi i (i k) / 4096) and
+// [16][16] exp(-2 pi i (i k) / 256)
 cudaError_t launch_highpass_fft(const float* X1, int64_t ldx, int32_t C, int64_t N, int32_t L, const float2* H,
                                 const float2* tw, float* Xh, cudaStream_t s);
 
