@@ -11,6 +11,7 @@
 // float [C, ldx] channel-major with time contiguous, so every later stage reads
 // 128-byte rows.
 #include "lss_kernels.cuh"
+#include "mp_common.cuh"
 
 namespace lss {
 
@@ -30,17 +31,19 @@ __device__ __forceinline__ int64_t src_row(int64_t s, const IngestMap& m, int64_
 
 // Per-channel integer sums over the padded batch (exact: raw samples are
 // integers, so the mean is the correctly rounded quotient of an exact sum).
-// Grid: one CTA per 256 columns; a warp per column at a time with channels
-// lane + 32q in registers (all of a column's loads in flight), per-lane int
-// sums combined across the CTA's warps in shared memory, one 64-bit atomic
-// per channel and CTA.
+// Grid: one CTA per `cols` columns (a multiple of 8); a warp per column at a time with
+// channels lane + 32q in registers (the loads of two columns in flight), per-lane int
+// sums combined across the CTA's warps in shared memory, one 64-bit atomic per channel
+// and CTA. Bound by the latency of its loads: 64 columns per CTA fill the chip in a
+// long batch, fewer in a short one (384 x 60122 in 19 us, 422 columns in 2.5 us, against 69 and 34 us with
+// 256 columns per CTA and a branch per load).
 template <int NQ>
 __global__ void __launch_bounds__(256) k_chan_sums(const int16_t* __restrict__ raw, int32_t ld_raw,
                                                    const int32_t* __restrict__ chan_map, int32_t C, int64_t N,
-                                                   IngestMap map, long long* __restrict__ sums) {
+                                                   IngestMap map, int cols, long long* __restrict__ sums) {
     __shared__ int part[8][NQ * 32];
-    const int64_t s0 = (int64_t)blockIdx.x * 256;
-    const int64_t s1 = min(N, s0 + 256);
+    const int64_t s0 = (int64_t)blockIdx.x * cols;
+    const int64_t s1 = min(N, s0 + cols);
     const int64_t base = map.base_dev ? *map.base_dev : 0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int acc[NQ];
@@ -51,13 +54,22 @@ __global__ void __launch_bounds__(256) k_chan_sums(const int16_t* __restrict__ r
         acc[q] = 0;
         ch[q] = (c < C) ? (chan_map ? chan_map[c] : c) : 0;
     }
-    for (int64_t sc = s0 + warp; sc < s1; sc += 8) {
-        const int64_t r = src_row(sc, map, base);
-        if (r < 0) continue;
-        const int16_t* row = raw + r * ld_raw;
+    constexpr int P = NQ <= 12 ? 2 : 1;  // columns in flight
+    for (int64_t sc = s0 + warp; sc < s1; sc += 8 * P) {
+        int16_t v[P][NQ];
+        int mask[P];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q)
-            if (lane + 32 * q < C) acc[q] += row[ch[q]];
+        for (int p = 0; p < P; ++p) {
+            const int64_t r = sc + 8 * p < s1 ? src_row(sc + 8 * p, map, base) : -1;
+            const int16_t* row = raw + max(r, (int64_t)0) * ld_raw;
+            mask[p] = r >= 0 ? -1 : 0;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) v[p][q] = row[ch[q]];  // no branch: all loads in flight (lanes past C: unused)
+        }
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) acc[q] += v[p][q] & mask[p];
     }
 #pragma unroll
     for (int q = 0; q < NQ; ++q) part[warp][lane + 32 * q] = acc[q];
@@ -73,8 +85,9 @@ __global__ void __launch_bounds__(256) k_chan_sums(const int16_t* __restrict__ r
 template <int NQ>
 static void launch_sums_t(const int16_t* raw, int32_t ld_raw, const int32_t* chan_map, int32_t C, int64_t N,
                           IngestMap map, long long* sums, cudaStream_t s) {
-    const int grid = (int)((N + 255) / 256);
-    k_chan_sums<NQ><<<grid, 256, 0, s>>>(raw, ld_raw, chan_map, C, N, map, sums);
+    const int cols = (int)std::min<int64_t>(64, std::max<int64_t>(8, N / (4 * 148) / 8 * 8));
+    const int grid = (int)((N + cols - 1) / cols);
+    k_chan_sums<NQ><<<grid, 256, 0, s>>>(raw, ld_raw, chan_map, C, N, map, cols, sums);
 }
 
 cudaError_t launch_chan_sums(const int16_t* raw, int32_t ld_raw, const int32_t* chan_map, int32_t C,
@@ -102,84 +115,187 @@ __device__ __forceinline__ float unkey(uint32_t k) {
     return __uint_as_float(u);
 }
 
-// CAR tile: 32 time columns x C channels staged in shared memory. Each warp
-// finds the lower median (sorted index (C-1)/2, torch.median's choice) of a
-// column by a 32-step bitwise select on order-preserving keys held in
-// registers (NQ = keys per lane >= C/32; padding keys are the largest value),
-// then the tile is written back as 128-byte channel rows.
-constexpr int CAR_COLS = 32;
+// Lower median (sorted index (C-1)/2, torch.median's choice) of a warp's C values,
+// v[q] of lane l being value l + 32 q (padding +inf; no NaN and no -0), found by
+// counting: two pivots about the mean, 1.7 standard errors of the median apart for
+// normal values, leave about 20 of 384 values between them; a further pair of pivots
+// tightens the bracket, by rank on even turns and halving the floats in it on odd
+// ones, until at most 32 values are left. Those are packed one per lane and each
+// counts the ones not above it. About 300 instructions per column of 384; a search
+// bit by bit over the floats takes 32 counts, 1150.
 template <int NQ>
-__global__ void __launch_bounds__(256) k_car(const int16_t* __restrict__ raw, int32_t ld_raw,
+__device__ __forceinline__ float lower_median(const float (&v)[NQ], int C, float mean, float& d0, float* cand,
+                                              int lane) {
+    const int kth = (C - 1) / 2;
+    const float big = 3.0e38f;  // above every value in magnitude
+    float flo = -big, fhi = big;
+    int clo = 0, chi = C;  // values not above flo, fhi; clo <= kth < chi
+    if (C > 32) {
+        if (d0 < 0.f) {  // the warp's first column
+            float dev = 0.f;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) dev += (lane + 32 * q < C) ? fabsf(v[q] - mean) : 0.f;
+            // sums of at most 32 values below 2^18, in eighths: 32 lanes of them fit
+            const float total = 0.125f * (float)__reduce_add_sync(0xffffffffu, (unsigned)(8.f * fminf(dev, 8388608.f)));
+            d0 = fmaxf(31.f * total / ((float)C * (float)C), 0.01f);
+        }
+        float d = d0;
+        float p1 = mean - d, p2 = mean + d;
+        for (int turn = 0; turn < 128; ++turn) {
+            unsigned cnt = 0;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) cnt += (v[q] <= p1 ? 1u : 0u) + (v[q] <= p2 ? 0x10000u : 0u);
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
+            const int n1 = (int)(cnt & 0xffffu), n2 = (int)(cnt >> 16);
+            if (n1 > kth) {
+                fhi = p1;
+                chi = n1;
+            } else {
+                flo = p1;
+                clo = n1;
+                if (n2 > kth) {
+                    fhi = p2;
+                    chi = n2;
+                } else {
+                    flo = p2;
+                    clo = n2;
+                }
+            }
+            if (chi - clo <= 32) break;
+            const uint32_t klo = fkey(flo), khi = fkey(fhi);
+            if (khi - klo <= 1) return fhi;  // nothing but fhi itself
+            if (flo == -big || fhi == big) {
+                d *= 3.f;
+                p1 = (flo == -big) ? fhi - d : flo + 0.4f * d;
+                p2 = (flo == -big) ? fhi - 0.4f * d : flo + d;
+            } else if (turn & 1) {
+                p1 = p2 = unkey(klo + (khi - klo) / 2);
+            } else {
+                const float w = (fhi - flo) / (float)(chi - clo);
+                const float est = flo + w * ((float)(kth - clo) + 0.5f);
+                p1 = est - 10.f * w;
+                p2 = est + 10.f * w;
+            }
+            // strictly inside the bracket, in order
+            p1 = fminf(fmaxf(p1, unkey(klo + 1)), unkey(khi - 1));
+            p2 = fminf(fmaxf(p2, p1), unkey(khi - 1));
+        }
+        if (chi - clo > 32) return fhi;  // (the bracket halves every other turn: not reached)
+    }
+    __syncwarp();
+    cand[lane] = big;
+    __syncwarp();
+    unsigned in = 0;  // of the chi - clo values in the bracket, this lane's
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) in |= (v[q] > flo && v[q] <= fhi) ? 1u << q : 0u;
+    const int mine = __popc(in);
+    float* dst = cand + warp_inc_scan(mine, lane) - mine;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+        if (in >> q & 1u) *dst++ = v[q];
+    __syncwarp();
+    const float x = cand[lane];
+    int le = 0;
+    for (int i = 0; i < chi - clo; i += 4) {
+        const float4 o = *reinterpret_cast<const float4*>(cand + i);
+        le += (o.x <= x) + (o.y <= x) + (o.z <= x) + (o.w <= x);
+    }
+    const uint32_t key = le > kth - clo ? fkey(x) : 0xFFFFFFFFu;
+    return unkey(__reduce_min_sync(0xffffffffu, key));
+}
+
+// CAR tile: COLS time columns x C channels staged in shared memory, a warp per column
+// at a time (NQ = values per lane >= C/32): its channels' loads in flight together, the
+// median taken off, then the tile is written back as rows of COLS samples. Tiles of 32
+// columns (128-byte rows); of 8 in batches that give the chip less than one CTA per SM
+// of those (384 x 60122 in 62 us, 422 columns in 4.9 us; bit-wise search and 32 columns: 169 and 28 us).
+template <int NQ, int COLS>
+__global__ void __launch_bounds__(256, NQ <= 12 ? 4 : 1) k_car(const int16_t* __restrict__ raw, int32_t ld_raw,
                                              const int32_t* __restrict__ chan_map, int32_t C,
                                              int64_t N, IngestMap map, float sign,
                                              const long long* __restrict__ sums, int do_car,
                                              float* __restrict__ X1, int64_t ldx) {
-    extern __shared__ float sm[];
-    float* tile = sm;                                  // [C][CAR_COLS + 1]
-    float* mean = sm + (size_t)C * (CAR_COLS + 1);     // [C]
-    const int64_t s0 = (int64_t)blockIdx.x * CAR_COLS;
-    const int ncol = (int)min((int64_t)CAR_COLS, N - s0);
+    extern __shared__ __align__(16) float sm[];
+    float* cand = sm + 32 * (threadIdx.x >> 5);  // [8 warps][32]
+    float* tile = sm + 8 * 32;                   // [C][COLS + 1]
+    float* mean = tile + (size_t)C * (COLS + 1);  // [NQ * 32]
+    int* chan = reinterpret_cast<int*>(mean + NQ * 32);  // [NQ * 32]
+    const int64_t s0 = (int64_t)blockIdx.x * COLS;
+    const int ncol = (int)min((int64_t)COLS, N - s0);
     const double invN = 1.0 / (double)N;
     const int64_t base = map.base_dev ? *map.base_dev : 0;
-    for (int c = threadIdx.x; c < C; c += blockDim.x)
-        mean[c] = (float)((double)sign * (double)sums[c] * invN);
+    for (int c = threadIdx.x; c < NQ * 32; c += 256) {
+        mean[c] = c < C ? (float)((double)sign * (double)sums[c] * invN) : 0.f;
+        chan[c] = c >= C ? 0 : chan_map ? chan_map[c] : c;
+    }
     __syncthreads();
-    // a warp per time column: its channels lane + 32q in registers (all loads
-    // of the column in flight at once), mean removed, the lower median found
-    // on the keys, and the referenced values parked in the tile for the
-    // channel-major write below
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t kth = (uint32_t)((C - 1) / 2);
-    for (int j = warp; j < CAR_COLS; j += blockDim.x >> 5) {
-        const int64_t r = (j < ncol) ? src_row(s0 + j, map, base) : -1;
+    const float invC = 1.f / (float)C;
+    float mbar = 0.f;  // mean of the channel means (where the search starts from)
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) mbar += mean[lane + 32 * q];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) mbar += __shfl_xor_sync(0xffffffffu, mbar, o);
+    mbar *= invC;
+    float d0 = -1.f;
+    for (int j = warp; j < ncol; j += 8) {
+        const int64_t r = src_row(s0 + j, map, base);
+        const int16_t* row = raw + max(r, (int64_t)0) * ld_raw;
+        const int mask = r >= 0 ? -1 : 0;
+        int16_t x[NQ];
         float v[NQ];
+        int sx = 0;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) x[q] = row[chan[lane + 32 * q]];  // (lanes past C: unused)
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
-            const int c = lane + 32 * q;
-            const int ch = (c < C) ? (chan_map ? chan_map[c] : c) : 0;
-            const float x = (c < C && r >= 0) ? sign * (float)raw[r * ld_raw + ch] : 0.f;
-            v[q] = (c < C && j < ncol) ? __fsub_rn(x, mean[c]) : 0.f;
+            const bool on = lane + 32 * q < C;
+            const int xi = x[q] & mask;
+            sx += on ? xi : 0;
+            v[q] = on ? __fsub_rn(sign * (float)xi, mean[lane + 32 * q]) : INFINITY;
         }
         float mj = 0.f;
-        if (do_car && j < ncol) {
-            uint32_t key[NQ];
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) key[q] = (lane + 32 * q < C) ? fkey(v[q]) : 0xFFFFFFFFu;
-            uint32_t res = 0;
-            for (int b = 31; b >= 0; --b) {
-                const uint32_t trial = res | ((1u << b) - 1u);
-                uint32_t cnt = 0;
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) cnt += (key[q] <= trial);
-                cnt = __reduce_add_sync(0xffffffffu, cnt);
-                if (cnt < kth + 1) res |= (1u << b);
-            }
-            mj = unkey(res);
+        if (do_car) {
+            sx = __reduce_add_sync(0xffffffffu, sx);
+            mj = lower_median<NQ>(v, C, sign * (float)sx * invC - mbar, d0, cand, lane);
         }
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
             const int c = lane + 32 * q;
-            if (c < C) tile[c * (CAR_COLS + 1) + j] = do_car ? __fsub_rn(v[q], mj) : v[q];
+            if (c < C) tile[c * (COLS + 1) + j] = do_car ? __fsub_rn(v[q], mj) : v[q];
         }
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < C * CAR_COLS; idx += blockDim.x) {
-        const int j = idx % CAR_COLS, c = idx / CAR_COLS;
-        if (j < ncol) {
-            X1[(int64_t)c * ldx + s0 + j] = tile[c * (CAR_COLS + 1) + j];
+    // rows of whole 16-byte pieces (ldx and s0 are multiples of 4)
+    for (int idx = threadIdx.x; idx < C * (COLS / 4); idx += 256) {
+        const int j = idx % (COLS / 4) * 4, c = idx / (COLS / 4);
+        const float* t = tile + c * (COLS + 1) + j;
+        float* o = X1 + (int64_t)c * ldx + s0 + j;
+        if (j + 4 <= ncol) {
+            *reinterpret_cast<float4*>(o) = make_float4(t[0], t[1], t[2], t[3]);
+        } else {
+            for (int u = 0; u < ncol - j; ++u) o[u] = t[u];
         }
     }
+}
+
+template <int NQ, int COLS>
+static cudaError_t launch_car_cols(const int16_t* raw, int32_t ld_raw, const int32_t* chan_map, int32_t C, int64_t N,
+                                   IngestMap map, float sign, const long long* sums, int do_car, float* X1, int64_t ldx,
+                                   cudaStream_t s) {
+    const size_t smem = sizeof(float) * (8 * 32 + (size_t)C * (COLS + 1) + 2 * NQ * 32);
+    cudaFuncSetAttribute(k_car<NQ, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    k_car<NQ, COLS><<<(unsigned)((N + COLS - 1) / COLS), 256, smem, s>>>(raw, ld_raw, chan_map, C, N, map, sign, sums,
+                                                                         do_car, X1, ldx);
+    return cudaGetLastError();
 }
 
 template <int NQ>
 static cudaError_t launch_car_t(const int16_t* raw, int32_t ld_raw, const int32_t* chan_map, int32_t C, int64_t N,
                                 IngestMap map, float sign, const long long* sums, int do_car, float* X1, int64_t ldx,
                                 cudaStream_t s) {
-    const size_t smem = sizeof(float) * ((size_t)C * (CAR_COLS + 1) + C + CAR_COLS);
-    cudaFuncSetAttribute(k_car<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    const int grid = (int)((N + CAR_COLS - 1) / CAR_COLS);
-    k_car<NQ><<<grid, 256, smem, s>>>(raw, ld_raw, chan_map, C, N, map, sign, sums, do_car, X1, ldx);
-    return cudaGetLastError();
+    if (N < 148 * 32) return launch_car_cols<NQ, 8>(raw, ld_raw, chan_map, C, N, map, sign, sums, do_car, X1, ldx, s);
+    return launch_car_cols<NQ, 32>(raw, ld_raw, chan_map, C, N, map, sign, sums, do_car, X1, ldx, s);
 }
 
 cudaError_t launch_car(const int16_t* raw, int32_t ld_raw, const int32_t* chan_map, int32_t C, int64_t N,
@@ -370,7 +486,7 @@ __device__ __forceinline__ void fft4096(float2 v[16], float2* a, const float2* _
 
 constexpr int HF_THREADS = HF / 16;
 
-// Bound by its FP32 adds and multiplies (about 50 us at the full rate for 384 x 60122, L = 500) with the shared-memory
+// Bound by its FP32 adds and multiplies (about 50 us at the full rate for 384 x 60122) with the shared-memory
 // passes beside them: 93 us, against 242 with every pass through shared memory. Two CTAs per SM: the 16 points, their
 // twiddles and a butterfly's temporaries take 128 registers (118 and 116 us with four and three CTAs, which spill).
 __global__ void __launch_bounds__(HF_THREADS, 2) k_highpass_fft(const float* __restrict__ X1, int64_t ldx, int32_t C,
