@@ -34,10 +34,11 @@
 
 namespace lss {
 
-constexpr int RF_COLS = 64;    // output columns per CTA (two warps of 32)
 constexpr int RF_CH = 128;     // channels per CTA (four groups of 32, one per warp)
 constexpr int RF_THREADS = 256;
-constexpr int RB_THREADS = 256;
+constexpr int RF_JC = 4;       // columns per lane
+constexpr int RB_THREADS = 512;
+constexpr int RB_WARPS = RB_THREADS / 32;
 constexpr int RB_SP = 64;      // spikes whose dL/da shares are kept before they are summed over the cluster
 constexpr int RB_MAXZ = 8;     // CTAs of a cluster (portable limit)
 
@@ -50,92 +51,162 @@ __device__ __forceinline__ int lower_bound_i(const int32_t* a, int n, int v) {
     return lo;
 }
 
-// xs/ys/as: spikes sorted by x. A warp owns 32 columns (lane = column) of 32
-// channels (in registers) and takes the tile's spikes in time order, skipping
-// the ones whose window misses its columns: acc[c] += U[y, k, c] * (a W[k, m]).
-// U rows of SP spikes at a time are staged in shared memory (broadcast reads, 16
-// bytes each), W is staged once with 32 zeros on either side.
-// Bound by the FP32 pipe and shared-memory reads about equally: 9000 spikes at
-// 384 channels x 60000 samples are 2.5 GFLOP that must be done and 3.9 GFLOP done
-// (a window covers 61 of the 92 columns it is taken over), over 92 MB written.
+// 8 channels by JC columns of sums: += u[c] * b[j], one FMA per term
+template <typename F, int JC>
+struct Outer {
+    F v[8][JC];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+#pragma unroll
+            for (int j = 0; j < JC; ++j) v[c][j] = F(0);
+    }
+    __device__ __forceinline__ void add(const F* u, const F (&b)[JC]) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+#pragma unroll
+            for (int j = 0; j < JC; ++j) v[c][j] += u[c] * b[j];
+    }
+    __device__ __forceinline__ F at(int c, int j) const { return v[c][j]; }
+};
+template <int JC>
+struct Outer<float, JC> {  // channels in pairs
+    unsigned long long v[4][JC];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int j = 0; j < JC; ++j) v[c][j] = 0ull;
+    }
+    __device__ __forceinline__ void add(const float* u, const float (&b)[JC]) {
+        const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(u), q = *reinterpret_cast<const ulonglong2*>(u + 4);
+#pragma unroll
+        for (int j = 0; j < JC; ++j) {
+            unsigned long long bb;
+            asm("mov.b64 %0, {%1, %1};" : "=l"(bb) : "f"(b[j]));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[0][j]) : "l"(p.x), "l"(bb));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[1][j]) : "l"(p.y), "l"(bb));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[2][j]) : "l"(q.x), "l"(bb));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[3][j]) : "l"(q.y), "l"(bb));
+        }
+    }
+    __device__ __forceinline__ float at(int c, int j) const {
+        float a, b;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v[c / 2][j]));
+        return c % 2 ? b : a;
+    }
+};
+
+// xs/ys/as: spikes sorted by x. A warp owns 32 columns of 32 channels, a lane 8
+// channels by 4 columns (8 apart) in registers, and takes the tile's spikes in time
+// order, skipping the ones whose window misses its columns:
+// acc[c, s] += U[y, k, c] * (a W[k, m]). U rows of SP spikes at a time are copied to
+// shared memory while the SP before them are added, W is staged once with 32 zeros
+// on either side. Shared memory returns 128 bytes per cycle to a warp also where
+// lanes read the same value: 8 x 4 outputs take 12 cycles of it beside 8 of FMAs (in
+// pairs of channels for floats); one column by 32 channels took 32 beside 8.
+// 9000 spikes at 384 channels x 60000 samples are 2.5 GFLOP that must be done and
+// 3.9 GFLOP done (a window covers 61 of the 92 columns it is taken over), over 92 MB
+// written: 182 us, against 296 us with one column per lane and 232 us with 8 x 8
+// outputs (two CTAs per SM instead of three, 61 of 124 columns).
 template <typename F, int SP>
-__global__ void __launch_bounds__(RF_THREADS) k_recon_fwd(const F* __restrict__ U, const F* __restrict__ W, int K,
-                                                          int C, int nt, const int32_t* __restrict__ xs,
-                                                          const int32_t* __restrict__ ys, const F* __restrict__ as,
-                                                          int n, F* __restrict__ R, int64_t N) {
+__global__ void __launch_bounds__(RF_THREADS, sizeof(F) == 4 ? 3 : 1)
+    k_recon_fwd(const F* __restrict__ U, const F* __restrict__ W, int K, int C, int nt, const int32_t* __restrict__ xs,
+                const int32_t* __restrict__ ys, const F* __restrict__ as, int n, F* __restrict__ R, int64_t N) {
+    constexpr int JC = RF_JC, CW = 8 * JC, COLS = 2 * CW;     // a warp's columns, the CTA's
     extern __shared__ __align__(16) unsigned char rf_smem[];
-    F* Us = reinterpret_cast<F*>(rf_smem);        // [SP][K][RF_CH]
-    F* Ws = Us + SP * K * RF_CH;                   // [K][nt + 64]
-    __shared__ int s_x[SP];
-    __shared__ F s_a[SP];
-    const int h = nt / 2, wp = nt + 64;
-    const int64_t t0 = (int64_t)blockIdx.x * RF_COLS;
+    F* Us = reinterpret_cast<F*>(rf_smem);        // [2][SP][K][RF_CH]
+    F* Ws = Us + 2 * SP * K * RF_CH;               // [K][nt + 2 CW]
+    __shared__ int s_x[2][SP];
+    __shared__ F s_a[2][SP];
+    const int h = nt / 2, wp = nt + 2 * CW;
+    const int64_t t0 = (int64_t)blockIdx.x * COLS;
     const int c0 = blockIdx.y * RF_CH;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wc = (warp >> 1) * 32;                       // the warp's channels, from c0
-    const int64_t w0 = t0 + (warp & 1) * 32;               // its first column
-    const int64_t col = w0 + lane;
-    const bool on = c0 + wc < C && w0 < N;
+    const int wc = (warp >> 1) * 32 + (lane >> 3) * 8;     // the lane's channels, from c0
+    const int64_t w0 = t0 + (warp & 1) * CW;               // the warp's first column
+    const int64_t col = w0 + (lane & 7);                   // the lane's
+    const bool on = c0 + (warp >> 1) * 32 < C && w0 < N;
     for (int e = threadIdx.x; e < K * wp; e += RF_THREADS) {
-        const int k = e / wp, m = e % wp - 32;
+        const int k = e / wp, m = e % wp - CW;
         Ws[e] = (m >= 0 && m < nt) ? W[k * nt + m] : F(0);
     }
-    // spikes whose window [x - h, x - h + nt) meets [t0, t0 + RF_COLS)
+    // spikes whose window [x - h, x - h + nt) meets [t0, t0 + COLS)
     const int lo = lower_bound_i(xs, n, (int)(t0 - (nt - 1 - h)));
-    const int hi = lower_bound_i(xs, n, (int)(t0 + RF_COLS + h));
-    F acc[32];
-#pragma unroll
-    for (int c = 0; c < 32; ++c) acc[c] = F(0);
-    for (int i0 = lo; i0 < hi; i0 += SP) {
+    const int hi = lower_bound_i(xs, n, (int)(t0 + COLS + h));
+    Outer<F, JC> acc;
+    acc.clear();
+    // SP spikes from i0 on: a warp per row (spike, component) of U, copied asynchronously (past C: zeros)
+    auto stage = [&](int i0, int buf) {
         const int ns = min(SP, hi - i0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < ns * K * RF_CH; e += RF_THREADS) {
-            const int q = e / (K * RF_CH), r = e - q * (K * RF_CH);
-            const int k = r / RF_CH, c = r % RF_CH;
-            Us[e] = (c0 + c < C) ? U[((int64_t)ys[i0 + q] * K + k) * C + c0 + c] : F(0);
+        for (int row = warp; row < ns * K; row += RF_THREADS / 32) {
+            const int q = row / K;
+            const F* src = U + ((int64_t)ys[i0 + q] * K + (row - q * K)) * C;
+            F* dst = Us + (buf * SP * K + row) * RF_CH;
+#pragma unroll
+            for (int c = lane; c < RF_CH; c += 32) {
+                const bool in = c0 + c < C;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(dst + c)),
+                             "l"(src + (in ? c0 + c : 0)), "n"((int)sizeof(F)), "r"(in ? (int)sizeof(F) : 0)
+                             : "memory");
+            }
         }
         if (threadIdx.x < ns) {
-            s_x[threadIdx.x] = xs[i0 + threadIdx.x];
-            s_a[threadIdx.x] = as[i0 + threadIdx.x];
+            s_x[buf][threadIdx.x] = xs[i0 + threadIdx.x];
+            s_a[buf][threadIdx.x] = as[i0 + threadIdx.x];
         }
-        __syncthreads();
+    };
+    if (lo < hi) stage(lo, 0);
+    int buf = 0;
+    for (int i0 = lo; i0 < hi; i0 += SP, buf ^= 1) {
+        const int ns = min(SP, hi - i0);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();  // the group is there; the one before it has been added, its buffer is free
+        if (i0 + SP < hi) stage(i0 + SP, buf ^ 1);
         if (!on) continue;
         for (int q = 0; q < ns; ++q) {
-            const int64_t d = w0 - s_x[q] + h;             // lag of the warp's first column
-            if (d <= -32 || d >= nt) continue;
-            const F a = s_a[q];
-            const F* wq = Ws + (int)d + lane + 32;
-            const F* uq = Us + q * K * RF_CH + wc;
+            const int64_t d = w0 - s_x[buf][q] + h;        // lag of the warp's first column
+            if (d <= -CW || d >= nt) continue;
+            const F a = s_a[buf][q];
+            const F* wq = Ws + (int)d + CW + (lane & 7);
+            const F* uq = Us + (buf * SP + q) * K * RF_CH + wc;
             for (int k = 0; k < K; ++k) {
-                const F b = a * wq[k * wp];
+                F b[JC];
 #pragma unroll
-                for (int c = 0; c < 32; ++c) acc[c] += uq[k * RF_CH + c] * b;
+                for (int j = 0; j < JC; ++j) b[j] = a * wq[k * wp + 8 * j];
+                acc.add(uq + k * RF_CH, b);
             }
         }
     }
-    if (on && col < N) {
+    if (on) {
         F* out = R + (int64_t)(c0 + wc) * N + col;
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
-            if (c0 + wc + c < C) out[(int64_t)c * N] = acc[c];
+        for (int c = 0; c < 8; ++c)
+#pragma unroll
+            for (int j = 0; j < JC; ++j)
+                if (c0 + wc + c < C && col + 8 * j < N) out[(int64_t)c * N + 8 * j] = acc.at(c, j);
     }
 }
 
+
 // A cluster of Z CTAs per template t; order[tstart[t] .. tstart[t+1]) are its
-// spikes. CTA z takes channel chunks z, z + Z, ...: a warp's channels w + 8j (j <
+// spikes. CTA z takes channel chunks z, z + Z, ...: a warp's channels w + 16 j (j <
 // CJ), lags lane + 32u (u < NM) of a window in registers, S and the template's
 // waveform beside them, so a spike costs one coalesced read and two FMAs per
-// element. The clusters' shared memories are then summed in rank order.
-// Bound by L2 reads of the windows (9000 spikes x 384 channels x 61 samples =
-// 843 MB; the 92 MB gradient stays in L2).
+// element; a spike's window is fetched while the one before it is added. The
+// clusters' shared memories are then summed in rank order. 9000 spikes x 384
+// channels x 61 samples are 843 MB of windows (the 92 MB gradient stays in L2), read
+// and added in 270 us; 470 us with 8 warps per CTA, no window ahead and a check per
+// element.
 template <typename F, int NM>
-__global__ void __launch_bounds__(RB_THREADS) k_recon_bwd(const F* __restrict__ U, const F* __restrict__ W, int K,
+__global__ void __launch_bounds__(RB_THREADS, sizeof(F) == 4 ? 2 : 1) k_recon_bwd(const F* __restrict__ U, const F* __restrict__ W, int K,
                                                           int C, int nt, const int32_t* __restrict__ x,
                                                           const F* __restrict__ amp, const int32_t* __restrict__ order,
                                                           const int32_t* __restrict__ tstart, const F* __restrict__ G,
                                                           int64_t N, F* __restrict__ dU, F* __restrict__ Qt,
                                                           F* __restrict__ damp) {
-    constexpr int CJ = 16 / NM, CH = 8 * CJ;
+    constexpr int CJ = 8 / NM, CH = RB_WARPS * CJ;
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char rb_smem[];
@@ -144,7 +215,7 @@ __global__ void __launch_bounds__(RB_THREADS) k_recon_bwd(const F* __restrict__ 
     F* Us = Ws + K * nt;                           // [K][CH]  U[t] of the chunk
     F* S = Us + K * CH;                            // [CH][ntp]
     F* Qp = S + CH * ntp;                          // [K][nt] this CTA's share of U[t] S_t
-    F* red = Qp + K * nt;                          // [RB_SP][8] shares of dL/da_i by warp
+    F* red = Qp + K * nt;                          // [RB_SP][RB_WARPS] shares of dL/da_i by warp
     __shared__ int s_i[RB_SP], s_x[RB_SP];
     __shared__ F s_a[RB_SP];
     const int Z = (int)cl.num_blocks(), z = (int)cl.block_rank();
@@ -173,7 +244,7 @@ __global__ void __launch_bounds__(RB_THREADS) k_recon_bwd(const F* __restrict__ 
                 const int m = lane + 32 * u;
                 F v = F(0);
                 if (m < nt)
-                    for (int k = 0; k < K; ++k) v += Us[k * CH + warp + 8 * j] * Ws[k * nt + m];
+                    for (int k = 0; k < K; ++k) v += Us[k * CH + warp + RB_WARPS * j] * Ws[k * nt + m];
                 wv[j][u] = v;
                 s[j][u] = F(0);
             }
@@ -187,20 +258,30 @@ __global__ void __launch_bounds__(RB_THREADS) k_recon_bwd(const F* __restrict__ 
                 s_a[threadIdx.x] = amp[i];
             }
             __syncthreads();
-            for (int q = 0; q < nb; ++q) {
+            // spike q's window of G in this warp's rows
+            auto load = [&](int q, F (&v)[CJ][NM]) {
+                if (q >= nb) return;
                 const int64_t x0 = (int64_t)s_x[q] - h;
-                const F a = s_a[q];
-                const bool whole = x0 >= 0 && x0 + nt <= N;
-                F v[CJ][NM];
                 const F* g = G + (int64_t)(c0 + warp) * N + x0 + lane;
+                if (x0 >= 0 && x0 + nt <= N && c0 + CH <= C) {
 #pragma unroll
-                for (int j = 0; j < CJ; ++j)
+                    for (int j = 0; j < CJ; ++j, g += RB_WARPS * N)
 #pragma unroll
-                    for (int u = 0; u < NM; ++u) {
-                        const int64_t p = x0 + lane + 32 * u;
-                        const bool in = lane + 32 * u < nt && c0 + warp + 8 * j < C && (whole || (p >= 0 && p < N));
-                        v[j][u] = in ? __ldg(g + (int64_t)(8 * j) * N + 32 * u) : F(0);
-                    }
+                        for (int u = 0; u < NM; ++u) v[j][u] = lane + 32 * u < nt ? __ldg(g + 32 * u) : F(0);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < CJ; ++j, g += RB_WARPS * N)
+#pragma unroll
+                        for (int u = 0; u < NM; ++u) {
+                            const int64_t p = x0 + lane + 32 * u;
+                            const bool in = lane + 32 * u < nt && c0 + warp + RB_WARPS * j < C && p >= 0 && p < N;
+                            v[j][u] = in ? __ldg(g + 32 * u) : F(0);
+                        }
+                }
+            };
+            // what it adds to the window sums; this lane's share of dL/da
+            auto add = [&](int q, const F (&v)[CJ][NM]) {
+                const F a = s_a[q];
                 F d = F(0);
 #pragma unroll
                 for (int j = 0; j < CJ; ++j)
@@ -209,10 +290,20 @@ __global__ void __launch_bounds__(RB_THREADS) k_recon_bwd(const F* __restrict__ 
                         s[j][u] += a * v[j][u];
                         d += wv[j][u] * v[j][u];
                     }
-                if (damp) {
+                return d;
+            };
+            F va[CJ][NM], vb[CJ][NM];  // the next spike's window is on its way while one is added
+            load(0, va);
+            for (int q = 0; q < nb; q += 2) {
+                load(q + 1, vb);
+                const F da = add(q, va);
+                load(q + 2, va);
+                const F db = q + 1 < nb ? add(q + 1, vb) : F(0);
+                if (damp) {  // both sums over the lanes: the lower half of the warp takes the first
+                    F d = (lane & 16 ? db : da) + __shfl_xor_sync(0xffffffffu, lane & 16 ? da : db, 16);
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-                    if (lane == 0) red[q * 8 + warp] = d;
+                    for (int o = 8; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+                    if ((lane & 15) == 0 && q + (lane >> 4) < nb) red[(q + (lane >> 4)) * RB_WARPS + warp] = d;
                 }
             }
             if (damp) {
@@ -221,8 +312,8 @@ __global__ void __launch_bounds__(RB_THREADS) k_recon_bwd(const F* __restrict__ 
                 if (z == 0 && threadIdx.x < nb) {
                     F d = it ? damp[s_i[threadIdx.x]] : F(0);
                     for (int r = 0; r < Z; ++r) {
-                        const F* rr = cl.map_shared_rank(red, r) + threadIdx.x * 8;
-                        for (int w = 0; w < 8; ++w) d += rr[w];
+                        const F* rr = cl.map_shared_rank(red, r) + threadIdx.x * RB_WARPS;
+                        for (int w = 0; w < RB_WARPS; ++w) d += rr[w];
                     }
                     damp[s_i[threadIdx.x]] = d;
                 }
@@ -233,7 +324,7 @@ __global__ void __launch_bounds__(RB_THREADS) k_recon_bwd(const F* __restrict__ 
         for (int j = 0; j < CJ; ++j)
 #pragma unroll
             for (int u = 0; u < NM; ++u)
-                if (lane + 32 * u < nt) S[(warp + 8 * j) * ntp + lane + 32 * u] = s[j][u];
+                if (lane + 32 * u < nt) S[(warp + RB_WARPS * j) * ntp + lane + 32 * u] = s[j][u];
         __syncthreads();
         for (int e = threadIdx.x; e < K * CH; e += RB_THREADS) {
             const int k = e / CH, c = e % CH;
@@ -279,13 +370,12 @@ __global__ void __launch_bounds__(256) k_reduce_templates(const F* __restrict__ 
 template <typename F>
 static cudaError_t recon_fwd(const void* U, const void* W, int K, int C, int nt, const int32_t* xs, const int32_t* ys,
                              const void* as, int n, void* R, int64_t N, cudaStream_t s) {
-    constexpr int SP = sizeof(F) == 4 ? 8 : 4;
-    const size_t smem = sizeof(F) * ((size_t)SP * K * RF_CH + (size_t)K * (nt + 64));
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_recon_fwd<F, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    dim3 grid((unsigned)((N + RF_COLS - 1) / RF_COLS), (unsigned)((C + RF_CH - 1) / RF_CH));
+    constexpr int SP = sizeof(F) == 4 ? 8 : 4, COLS = 16 * RF_JC;
+    const size_t smem = sizeof(F) * ((size_t)2 * SP * K * RF_CH + (size_t)K * (nt + COLS));
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_recon_fwd<F, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    dim3 grid((unsigned)((N + COLS - 1) / COLS), (unsigned)((C + RF_CH - 1) / RF_CH));
     k_recon_fwd<F, SP><<<grid, RF_THREADS, smem, s>>>(static_cast<const F*>(U), static_cast<const F*>(W), K, C, nt, xs,
                                                       ys, static_cast<const F*>(as), n, static_cast<F*>(R), N);
     return cudaGetLastError();
@@ -296,13 +386,12 @@ template <typename F, int NM>
 static cudaError_t recon_bwd_nm(const F* U, const F* W, int T, int K, int C, int nt, const int32_t* x, const F* amp,
                                 const int32_t* order, const int32_t* tstart, const F* G, int64_t N, F* dU, F* work,
                                 F* damp, cudaStream_t s) {
-    constexpr int CH = 8 * (16 / NM);
-    const size_t smem = sizeof(F) * (2 * (size_t)K * nt + (size_t)K * CH + (size_t)CH * (nt | 1) + RB_SP * 8);
+    constexpr int CH = RB_WARPS * (8 / NM);
+    const size_t smem = sizeof(F) * (2 * (size_t)K * nt + (size_t)K * CH + (size_t)CH * (nt | 1) + RB_SP * RB_WARPS);
     auto kern = k_recon_bwd<F, NM>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    // (always: with the static arrays a size just below 48 KB needs it too)
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
     const int Z = std::min(RB_MAXZ, (C + CH - 1) / CH);
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)T * (unsigned)Z);
