@@ -37,12 +37,20 @@
 // shared memory), so a tile is only ever read and written by its CTA. CTAs
 // exchange 64-bit words that carry their round's tag next to the data, so a
 // reader polls the data itself and no fence or barrier counter is needed:
-//   * per round, each CTA's peak count, which every CTA reads (the parity of
-//     a spike is its number in the whole round);
+//   * the column maxima within nt of a CTA's edge, read by its neighbours;
 //   * the peaks (x, y, a), read by the CTAs whose columns they reach;
-//   * the column maxima within nt of a CTA's edge, read by its neighbours.
-// Peaks and counts are double-buffered by round parity: a CTA can be at most
-// one round ahead of another, because every round needs every CTA's count.
+//   * each CTA's peak count, read by those, and a round later by every CTA: the
+//     round's total ends the loop and numbers the records.
+// The parity of a spike is its number in the whole round, but it only orders
+// spikes whose windows overlap: a CTA near peaks closer than 2nt reads the counts
+// to its left in the same round, the others wait for their neighbours alone.
+// (Every CTA reading every count at once cost 10 us of a round's 31 at 800
+// templates, the skew between them: 2.23 ms of rounds against 2.00, 0.81 against
+// 0.72 at 400. Counts two or three rounds late gain nothing more.)
+// Peaks and counts are double-buffered by round parity: before a CTA sends those
+// of round r + 2 it has read every CTA's count of round r + 1, each sent after
+// its sender had read the peaks and all counts of round r. Column maxima need one
+// buffer: their readers' counts are read before the next ones are sent.
 // Every wait is bounded (STATUS_TIMEOUT).
 #include "lss_kernels.cuh"
 #include "mp_common.cuh"
@@ -55,7 +63,7 @@ namespace lss {
 
 constexpr int MPL_THREADS = 1024;
 constexpr int MPL_WARPS = MPL_THREADS / 32;
-constexpr int MPL_MAX_GRID = 1024;
+constexpr int MPL_MAX_GRID = 1024;  // (MPL_WARPS warps' lanes: collect)
 constexpr int MPL_LOG = 512;          // least log capacity (spikes)
 constexpr unsigned MPL_SPIN_LIMIT = 1u << 21;  // polls of a word (about 1.5 s)
 constexpr int MPL_REGIONS = 40;       // CTAs whose peaks reach one CTA's columns
@@ -138,7 +146,7 @@ __device__ __forceinline__ bool reaches(float ub, float th2) {
 template <bool KSMEM>
 __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_total, s_pref, s_nnew, s_qn, s_qold, s_qnext;
+    __shared__ int s_total, s_pref, s_own, s_base, s_nnew, s_qn, s_qold, s_qnext;
     __shared__ int s_rcnt[MPL_REGIONS];
     __shared__ unsigned long long s_clk[PhaseClock::WORDS];
 
@@ -207,7 +215,7 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
     }
     for (int q = tid; q < ntile; q += MPL_THREADS) s_app[q] = -1;
     for (int c = tid; c < cpc; c += MPL_THREADS) s_touch[c] = 1;
-    if (tid == 0) s_qn = s_qold = s_qnext = 0;
+    if (tid == 0) s_qn = s_qold = s_qnext = s_total = s_pref = s_base = 0;
     __syncthreads();
     int n_app = 0, n_items = 0;  // (spike, tile) updates applied (per warp) and met (per lane)
 
@@ -334,7 +342,57 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
         }
     };
     PhaseClock clk{s_clk};
-    int base = 0, r = 0, nlog = 0;
+    int r = 0, nlog = 0;
+    // counts of the CTAs [from, to) in the round of `tag`, summed over one warp
+    auto sum_counts = [&](int from, int to, unsigned tag, bool& bad) {
+        const unsigned long long* w = x_cnt + ((tag - 1u) & 1u) * G;
+        int sum = 0;
+        for (int i = from + lane; i < to; i += 32) {
+            unsigned long long wv;
+            bad |= !poll_word(w + i, tag, wv, a.status);
+            sum += (int)(unsigned)wv;
+        }
+        return __reduce_add_sync(FULL, sum);
+    };
+    // ... of round rr, added up: the number of this CTA's first peak and the
+    // total. The last warps take 32 words each (polled one after the other,
+    // every word would take the latency of a load)
+    auto collect = [&](int rr) {
+        bool bad = false;
+        const int i = (MPL_WARPS - 1 - warp) * 32 + lane;
+        if (i - lane < G) {
+            unsigned long long wv = 0ull;
+            if (i < G) bad = !poll_word(x_cnt + (rr & 1) * G + i, (unsigned)rr + 1u, wv, a.status);
+            const int tot = __reduce_add_sync(FULL, (int)(unsigned)wv);
+            const int before = __reduce_add_sync(FULL, i < b ? (int)(unsigned)wv : 0);
+            if (lane == 0) {
+                atomicAdd(&s_total, tot);
+                atomicAdd(&s_pref, before);
+            }
+        }
+        return bad;
+    };
+    // Round rr is counted: its peaks' records, unless it was the last one
+    // (none found) or overflows the list (every CTA sees the same total)
+    auto finish = [&](int rr) {
+        const int total = s_total, base = s_base;
+        if (total == 0) return false;
+        if (base + total > a.capacity) {
+            if (tid == 0) atomicOr(a.status, STATUS_CAPACITY);
+            return false;
+        }
+        const unsigned long long* pk = x_pk + 2 * ((int64_t)(rr & 1) * G * W + lo);
+        for (int k = MPL_THREADS - 1 - tid; k < s_own; k += MPL_THREADS) {
+            const unsigned long long w0 = ld_word(pk + 2 * k), w1 = ld_word(pk + 2 * k + 1);
+            const int i = base + s_pref + k;
+            a.sp_x[i] = (int)((w1 >> 24) & 0xFFFFFFFull);
+            a.sp_y[i] = (int)(w1 & 0xFFFFFFull);
+            a.sp_amp[i] = __uint_as_float((unsigned)w0);
+            if (a.sp_round) a.sp_round[i] = rr;
+        }
+        if (b == 0 && tid == 0) a.round_start[rr] = base;
+        return true;
+    };
     int todo_all = 1;  // every tile is due: 1 at the start (keys of the initial field), 2 when the log is full
     for (;; ++r) {
         // ---- the tiles that are due, one warp each
@@ -356,38 +414,53 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
             if (!grid_sync(a.bar, a.status)) return;
             if (tid == 0) clk.start();
         }
-        if (r >= a.max_rounds) break;
+        if (r >= a.max_rounds) {  // the last round's counts
+            bool bad = false;
+            if (r > 0) bad = collect(r - 1);
+            if (__syncthreads_or(bad)) return;
+            if (r == 0) break;
+            const bool found = finish(r - 1);
+            __syncthreads();
+            if (!found) --r;
+            else if (tid == 0) s_base += s_total;
+            break;
+        }
         const unsigned tag = (unsigned)r + 1u;
         unsigned long long* cnt_w = x_cnt + (r & 1) * G;                      // this round's counts
         unsigned long long* pk_w = x_pk + 2 * (int64_t)(r & 1) * G * W;       // ... and peaks
         bool bad = false;
-        // ---- column maxima (of the chunks that the last round touched) from
-        // the tiles' keys (a tile with pending spikes has old ones, below the
-        // threshold); the ones within nt of the edges go to the neighbours
+        // ---- column maxima (of the chunks that the last round touched) from the
+        // keys of the tiles whose bound reaches the threshold (the others', old
+        // ones among them, are below it and change no decision); the ones
+        // within nt of the edges go to the neighbours
         for (int c = warp; c < nchunk; c += MPL_WARPS) {
             const int s = lo + c * 32 + lane;
-            if (s < N) {
-                float v;
-                if (s_touch[c]) {
-                    unsigned long long k = 0ull;
-                    for (int b0 = 0; b0 < nb; b0 += 8) {
-                        unsigned long long kk[8];
+            float v;
+            if (s_touch[c]) {
+                unsigned long long k = 0ull;
+                for (int b0 = 0; b0 < nb; b0 += 32) {
+                    unsigned loud = __ballot_sync(FULL, b0 + lane < nb && reaches(s_ub[c * nb + b0 + lane], a.th2));
+                    while (loud) {
+                        unsigned long long kk[4];
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) kk[u] = (b0 + u < nb) ? ld_key(b0 + u, c) : 0ull;
+                        for (int u = 0; u < 4; ++u) {
+                            const int blk = b0 + __ffs(loud) - 1;
+                            kk[u] = loud && s < N ? ld_key(blk, c) : 0ull;
+                            loud &= loud - 1u;
+                        }
 #pragma unroll
-                        for (int u = 0; u < 8; ++u)
-                            k = max(k, kk[u]);
+                        for (int u = 0; u < 4; ++u) k = max(k, kk[u]);
                     }
-                    v = __uint_as_float((unsigned)(k >> 32));
-                    s_vals[nt + c * 32 + lane] = v;
-                    s_ival[c * 32 + lane] = (int)(0xFFFFFFFFu - (unsigned)k);
-                } else {
-                    v = s_vals[nt + c * 32 + lane];
                 }
-                if (s < lo + nt || s >= hi - nt)
-                    st_word(x_val + s, ((unsigned long long)tag << 32) | __float_as_uint(v));
+                v = __uint_as_float((unsigned)(k >> 32));
+                s_vals[nt + c * 32 + lane] = v;
+                s_ival[c * 32 + lane] = (int)(0xFFFFFFFFu - (unsigned)k);
+            } else {
+                v = s_vals[nt + c * 32 + lane];
             }
+            if (s < N && (s < lo + nt || s >= hi - nt)) st_word(x_val + s, ((unsigned long long)tag << 32) | __float_as_uint(v));
         }
+        __syncwarp();
         for (int p = tid; p < 2 * nt; p += MPL_THREADS) {
             const int s = p < nt ? lo - nt + p : hi + p - nt;
             float v = 0.f;
@@ -398,7 +471,13 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
             }
             s_vals[p < nt ? p : (hi - lo) + p] = v;
         }
+        // the last round's counts, which the others have had this long to send
+        if (r > 0) bad |= collect(r - 1);
         if (__syncthreads_or(bad)) return;
+        if (r > 0 && !finish(r - 1)) {
+            --r;
+            break;
+        }
         // ---- P: peaks = (Cmax > Th^2) & (|Cmax - Cfmax| < 1e-9), Cmax the
         // maximum over +-nt. Only a column at the threshold and not below its
         // direct neighbours (less margins above the 1e-9) can pass; for those
@@ -446,31 +525,25 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
             own += __shfl_sync(FULL, inc, 31);
         }
         if (tid == 0) {
+            s_base += s_total;  // (the round before's, recorded)
+            s_total = s_pref = 0;
+            s_own = own;
             st_word(cnt_w + b, ((unsigned long long)tag << 32) | (unsigned)own);
             clk.lap(0);
         }
-        // ---- warp 0: every CTA's count (the round's total, the number of this
-        // CTA's first peak), then the peaks that reach its columns, the
-        // round's even-numbered ones first
+        // ---- warp 0: the peaks that reach this CTA's columns, the round's
+        // even-numbered ones first. Only peaks within 2nt of one another care
+        // about their numbers; elsewhere the counts of the CTAs nearby will do
         if (warp == 0) {
             const int r_lo = max(0, b - (nt + W - 1) / W), r_hi = min(G - 1, b + (3 * nt + W - 1) / W);
-            int before = 0, tot = 0, left = 0, near_n = 0;
-            for (int i = lane; i < G; i += 32) {
+            int left = 0, near_n = 0;
+            for (int i = r_lo + lane; i <= r_hi; i += 32) {
                 unsigned long long wv;
                 bad |= !poll_word(cnt_w + i, tag, wv, a.status);
-                const int cnt = (int)(unsigned)wv;
-                tot += cnt;
-                if (i < b) before += cnt;
-                if (i < r_lo) left += cnt;
-                if (i >= r_lo && i <= r_hi) {
-                    near_n += cnt;
-                    s_rcnt[i - r_lo] = cnt;
-                }
+                near_n += (int)(unsigned)wv;
+                s_rcnt[i - r_lo] = (int)(unsigned)wv;
             }
             bad = __any_sync(FULL, bad);
-            tot = __reduce_add_sync(FULL, tot);
-            before = __reduce_add_sync(FULL, before);
-            left = __reduce_add_sync(FULL, left);
             near_n = __reduce_add_sync(FULL, near_n);
             if (lane == 0) clk.lap(1);
             int n_new = 0;
@@ -480,10 +553,10 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
                 while (i >= s_rcnt[reg - r_lo]) i -= s_rcnt[reg++ - r_lo];
                 const unsigned long long* p = pk_w + 2 * ((int64_t)reg * W + i);
                 unsigned long long w0 = 0, w1 = 0;
-                if (!poll_word(p, tag, w0, a.status)) bad = true;
                 for (unsigned sp = 0; !bad; ++sp) {
+                    w0 = ld_word(p);
                     w1 = ld_word(p + 1);
-                    if ((unsigned)(w1 >> 52) == (tag & 0xFFFu)) break;
+                    if ((unsigned)(w0 >> 32) == tag && (unsigned)(w1 >> 52) == (tag & 0xFFFu)) break;
                     if (sp > MPL_SPIN_LIMIT) {
                         atomicOr(a.status, STATUS_TIMEOUT);
                         bad = true;
@@ -506,21 +579,36 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
                 n_new += __popc(bal);
             };
             __syncwarp();
-            if (!bad && near_n > 0) {
+            if (!bad && near_n > 0 && near_n <= 30) {  // one group
+                int x = INT_MAX / 2, y = 0;
+                float am = 0.f;
+                if (lane < near_n) entry(lane, x, y, am);
+                const int x1 = __shfl_down_sync(FULL, x, 1);
+                const bool close = __any_sync(FULL, lane + 1 < near_n && x1 - x <= 2 * nt);
+                if (close) left = sum_counts(0, r_lo, tag, bad);
+                const int x2 = __shfl_down_sync(FULL, x, 2);
+                const int ehi = min(min(x + nt, N - 1), x2 - nt - 1);
+                const bool mine = lane < near_n && x - nt < hi && ehi >= lo && ehi >= x - nt, odd = (left + lane) & 1;
+                const unsigned me = __ballot_sync(FULL, mine && !odd), mo = __ballot_sync(FULL, mine && odd);
+                const unsigned below = (1u << lane) - 1u;
+                const int dst = odd ? __popc(me) + __popc(mo & below) : __popc(me & below);
+                if (mine && dst < a.new_cap) s_new[dst] = make_int4(x, ehi, y, __float_as_int(am));
+                n_new = __popc(me | mo);
+            } else if (!bad && near_n > 0) {
+                left = sum_counts(0, r_lo, tag, bad);
+                __syncwarp();
+                const int before = left + sum_counts(r_lo, b, tag, bad), tot = left + sum_counts(r_lo, G, tag, bad);
                 for (int pass = 0; pass < 2; ++pass)
                     for (int i0 = 0; i0 < near_n; i0 += 30) {
                         int x = INT_MAX / 2, y = 0;
                         float am = 0.f;
                         if (i0 + lane < near_n) entry(i0 + lane, x, y, am);
                         emit(pass, i0, x, y, am);
-                        if (near_n <= 30) {  // one group: its words are read once for both parities
-                            emit(1, i0, x, y, am);
-                            pass = 1;
-                        } else if (pass == 0) {
+                        if (pass == 0) {
                             // more than MP_LIST peaks within 2nt of one another are refused, as by
                             // the other rounds kernel (whose lists they would overflow)
                             const int i = i0 + lane;
-                            if (lane < 30 && left + i >= before && left + i < before + own && i + MP_LIST - 1 < near_n &&
+                            if (lane < 30 && left + i >= before && left + i < before + s_own && i + MP_LIST - 1 < near_n &&
                                 left + i + MP_LIST < tot) {
                                 int xq = 0, yq = 0;
                                 float aq = 0.f;
@@ -531,33 +619,11 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
                         }
                     }
             }
-            bad = __any_sync(FULL, bad);
-            if (lane == 0) {
-                s_total = bad ? -1 : tot;
-                s_pref = before;
-                s_nnew = n_new;
-            }
+            if (lane == 0) s_nnew = n_new;
         }
-        __syncthreads();
-        const int total = s_total, n_new = min(s_nnew, a.new_cap);
-        if (total < 0) return;
-        if (total == 0) break;
-        if (base + total > a.capacity) {  // every CTA sees the same total
-            if (tid == 0) atomicOr(a.status, STATUS_CAPACITY);
-            break;
-        }
+        if (__syncthreads_or(bad)) return;
+        const int n_new = min(s_nnew, a.new_cap);
         if (s_nnew > a.new_cap && tid == 0) atomicOr(a.status, STATUS_LIST);
-        // ---- records of this CTA's peaks; the round's spikes into the log
-        for (int k = tid; k < own; k += MPL_THREADS) {
-            const unsigned long long* p = pk_w + 2 * ((int64_t)lo + k);
-            const unsigned long long w0 = ld_word(p), w1 = ld_word(p + 1);
-            const int i = base + s_pref + k;
-            a.sp_x[i] = (int)((w1 >> 24) & 0xFFFFFFFull);
-            a.sp_y[i] = (int)(w1 & 0xFFFFFFull);
-            a.sp_amp[i] = __uint_as_float((unsigned)w0);
-            if (a.sp_round) a.sp_round[i] = r;
-        }
-        if (b == 0 && tid == 0) a.round_start[r] = base;
         for (int e = tid; e < n_new; e += MPL_THREADS) s_log[nlog + e] = s_new[e];
         // ---- the tiles the spikes reach (a warp per chunk and group of 32
         // blocks, lane = block): a spike that changes the tile, or any spike on
@@ -611,7 +677,6 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
             }
         }
         nlog += n_new;
-        base += total;
         // a log that the next round may overflow: every pending spike is applied
         todo_all = nlog + a.new_cap > a.log_cap ? 2 : 0;
         __syncthreads();
@@ -626,9 +691,9 @@ __global__ void __launch_bounds__(MPL_THREADS, 1) k_mp_lazy(MPArgs a) {
         clk.flush(a.phase);
     }
     if (b == 0 && tid == 0) {
-        a.counters[0] = base;
+        a.counters[0] = s_base;
         a.counters[1] = r;
-        a.round_start[r] = base;
+        a.round_start[r] = s_base;
     }
 }
 
