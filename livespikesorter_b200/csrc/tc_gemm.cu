@@ -32,6 +32,7 @@ namespace tc {
 
 constexpr int BM = 128;               // samples per tile
 constexpr int MAX_NP = 512;           // templates per pass (TMEM columns)
+constexpr int MAX_STAGES = 6;
 constexpr int SPLIT_W = 128;          // templates per work item in split mode
 constexpr int MAPPED_SPLIT_W = 64;    // ... for a re-check of a few mapped rows
 constexpr int THREADS = 192;
@@ -60,7 +61,7 @@ struct Kind {
 
 struct Args {
     int N, T, Tpad, KB;
-    int box_rows, nbox_max, stages, b_rows;
+    int stages, b_rows;
     int nacc;                 // accumulator buffers in TMEM (2 when a pass fits in 256 columns)
     float* Bout;
     int64_t ldb;
@@ -132,8 +133,8 @@ __device__ __forceinline__ uint64_t globaltimer() {
 
 // Bounded wait (about 2 s of wall time); false when the CTA is aborting or
 // the budget expired (then the abort flag and STATUS_TIMEOUT are raised).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int32_t* status) {
+static __device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                                   int32_t* status) {
     const uint64_t t0 = globaltimer();
     for (uint32_t i = 0;; ++i) {
         if (mbar_try(bar, parity)) return true;
@@ -145,6 +146,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     *abort_flag = 1;
     atomicOr(status, STATUS_TIMEOUT);
     return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
+    return mbar_try(bar, parity) || mbar_wait_long(bar, parity, abort_flag, status);
 }
 
 // Wait (bounded, no abort check) for a phase that is known to complete.
@@ -161,12 +165,18 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
-// K-major operand with swizzled rows: 8-row atoms of ATOM bytes.
+// K-major operand with swizzled rows: 8-row atoms of ATOM bytes. The low word holds
+// the address in 16-byte units, so that an operand elsewhere in shared memory is one
+// addition away.
 template <int OP>
-__device__ __forceinline__ uint64_t operand_desc(uint32_t addr) {
+__device__ __forceinline__ uint32_t operand_desc(uint32_t addr) {
+    return ((addr >> 4) & 0x3FFFu) | (1u << 16);
+}
+template <int OP>
+__device__ __forceinline__ uint64_t operand_at(uint32_t desc, uint32_t bytes) {
     using KD = Kind<OP>;
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(KD::ATOM >> 4) << 32) |
-           ((uint64_t)1 << 46) | (KD::LAYOUT << 61);
+    constexpr uint32_t hi = (KD::ATOM >> 4) | (1u << 14) | (uint32_t)(KD::LAYOUT << 29);
+    return (uint64_t)hi << 32 | (desc + (bytes >> 4));
 }
 
 // Instruction descriptor: F32 accumulator, BF16 (1) or TF32 (2) operands,
@@ -329,29 +339,25 @@ __global__ void __launch_bounds__(THREADS, 1)
             // ---------------- TMA producer
             int stage = 0;
             uint32_t ph = 0;
-            uint32_t last_ph[8];
-            bool pending[8] = {false, false, false, false, false, false, false, false};
+            uint32_t last_ph[MAX_STAGES];
+            bool pending[MAX_STAGES] = {};
             bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
                 const int tile = split ? it / npass : it;
                 const int pb = split ? it % npass : 0, pe = split ? pb + 1 : npass;
                 for (int p = pb; p < pe && ok; ++p) {
-                    const int np = min(PW, a.Tpad - p * PW);
-                    const int nbox = (np + a.box_rows - 1) / a.box_rows;
-                    const uint32_t bytes = KD::PARTS * (KD::A_TILE + (uint32_t)nbox * a.box_rows * KD::ROW);
-                    for (int kb = 0; kb < a.KB; ++kb) {
+                    const int row = p * PW;
+                    int kx = 0;
+                    for (int kb = 0; kb < a.KB; ++kb, kx += KD::BKE) {
+                        const uint32_t full = full_bar(stage);
                         if (!mbar_wait(empty_bar(stage), ph ^ 1u, abort_flag, a.status)) { ok = false; break; }
                         const uint32_t sa = s0 + stage * stage_bytes;
                         const uint32_t sb = sa + a_bytes;
-                        const int kx = kb * KD::BKE;
-                        mbar_expect_tx(full_bar(stage), bytes);
-                        tma_load_2d(sa, &tmA, kx, tile * BM, full_bar(stage));
-                        if (KD::SPLIT) tma_load_2d(sa + KD::A_TILE, &tmAlo, kx, tile * BM, full_bar(stage));
-                        for (int bx = 0; bx < nbox; ++bx) {
-                            const int row = p * PW + bx * a.box_rows;
-                            tma_load_2d(sb + bx * a.box_rows * KD::ROW, &tmB, kx, row, full_bar(stage));
-                            if (KD::SPLIT) tma_load_2d(sb + b_part + bx * a.box_rows * KD::ROW, &tmBlo, kx, row, full_bar(stage));
-                        }
+                        mbar_expect_tx(full, stage_bytes);
+                        tma_load_2d(sa, &tmA, kx, tile * BM, full);
+                        if (KD::SPLIT) tma_load_2d(sa + KD::A_TILE, &tmAlo, kx, tile * BM, full);
+                        tma_load_2d(sb, &tmB, kx, row, full);
+                        if (KD::SPLIT) tma_load_2d(sb + b_part, &tmBlo, kx, row, full);
                         last_ph[stage] = ph;
                         pending[stage] = true;
                         if (++stage == a.stages) { stage = 0; ph ^= 1u; }
@@ -366,7 +372,14 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            // ---------------- MMA issuer
+            // ---------------- MMA issuer. A k-block's six MMAs of 208 templates
+            // take 650 cycles; waiting, building every MMA's descriptors and
+            // issuing took this thread 830 at any width. With the descriptors'
+            // low words kept, the waits' timers out of line and a fifth stage a
+            // block takes 770 (400 templates x 60122 samples, 3xTF32: 518 -> 438
+            // us, 418 at the measured peak; BF16x3 at 800: 682 -> 654 us, where
+            // the error bounds' epilogue waits beside it).
+            const uint32_t desc_a = operand_desc<OP>(s0), desc_b = operand_desc<OP>(s0 + a_bytes);
             int stage = 0;
             uint32_t ph = 0;
             uint32_t acc_ph[2] = {0, 0};
@@ -379,29 +392,23 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (!mbar_wait(acce_bar(acc), acc_ph[acc] ^ 1u, abort_flag, a.status)) { ok = false; break; }
                     fence_after();
                     const uint32_t dcol = tmem + (uint32_t)(acc * 256);
+                    const uint32_t idesc = instr_desc<OP>(np);
                     for (int kb = 0; kb < a.KB; ++kb) {
                         if (!mbar_wait(full_bar(stage), ph, abort_flag, a.status)) { ok = false; break; }
                         fence_after();
-                        const uint32_t sa = s0 + stage * stage_bytes;
-                        const uint32_t sb = sa + a_bytes;
+                        const uint32_t da = desc_a + stage * (stage_bytes >> 4), db = desc_b + stage * (stage_bytes >> 4);
 #pragma unroll
                         for (int ks = 0; ks < KD::SUB; ++ks) {
-                            const uint32_t ko = ks * 32;
-                            const uint64_t ad = operand_desc<OP>(sa + ko);
-                            for (int c = 0; c < np; c += 256) {
-                                const int n = min(256, np - c);
-                                const uint32_t idesc = instr_desc<OP>(n);
-                                const uint64_t bd = operand_desc<OP>(sb + (uint32_t)c * KD::ROW + ko);
-                                const uint32_t acc_on = (kb | ks) != 0;
-                                if (KD::SPLIT) {
-                                    const uint64_t adl = operand_desc<OP>(sa + KD::A_TILE + ko);
-                                    const uint64_t bdl = operand_desc<OP>(sb + b_part + (uint32_t)c * KD::ROW + ko);
-                                    mma<OP>(dcol + (uint32_t)c, adl, bd, idesc, acc_on);   // A_lo B_hi
-                                    mma<OP>(dcol + (uint32_t)c, ad, bdl, idesc, 1u);      // A_hi B_lo
-                                    mma<OP>(dcol + (uint32_t)c, ad, bd, idesc, 1u);       // A_hi B_hi
-                                } else {
-                                    mma<OP>(dcol + (uint32_t)c, ad, bd, idesc, acc_on);
-                                }
+                            const uint64_t ad = operand_at<OP>(da, ks * 32), bd = operand_at<OP>(db, ks * 32);
+                            const uint32_t acc_on = (kb | ks) != 0;
+                            if (KD::SPLIT) {
+                                const uint64_t adl = operand_at<OP>(da, KD::A_TILE + ks * 32);
+                                const uint64_t bdl = operand_at<OP>(db + (b_part >> 4), ks * 32);
+                                mma<OP>(dcol, adl, bd, idesc, acc_on);  // A_lo B_hi
+                                mma<OP>(dcol, ad, bdl, idesc, 1u);      // A_hi B_lo
+                                mma<OP>(dcol, ad, bd, idesc, 1u);       // A_hi B_hi
+                            } else {
+                                mma<OP>(dcol, ad, bd, idesc, acc_on);
                             }
                         }
                         mma_commit(empty_bar(stage));
@@ -673,11 +680,13 @@ TcPlan tc_plan(int T, int op, int pass_w) {
     p.b_rows = b_rows;
     const size_t row = op == TC_BF16 ? 128 : 64, parts = op == TC_BF16 ? 1 : 2;
     const size_t stage = parts * (tc::BM * row + (size_t)b_rows * row);
+    auto bytes = [&](int stages) { return 1024 + stages * stage + 8 * (2 * stages + 5) + 16 + 12 * (size_t)p.Tpad; };
     const size_t tail = 8 * (2 * 4 + 5) + 16 + 12 * (size_t)p.Tpad;
     const size_t budget = 227 * 1024 - 1024 - tail;
     p.stages = (int)std::min<size_t>(4, budget / stage);
+    while (p.stages >= 4 && p.stages < tc::MAX_STAGES && bytes(p.stages + 1) <= 227 * 1024) ++p.stages;
     p.nacc = (np0 <= 256) ? 2 : 1;
-    p.smem = 1024 + (size_t)p.stages * stage + 8 * (2 * p.stages + 5) + 16 + 12 * (size_t)p.Tpad;
+    p.smem = bytes(p.stages);
     p.kblock = op == TC_TF32X3 ? 16 : (op == TC_BF16X3 ? 32 : 64);
     return p;
 }
@@ -688,7 +697,9 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
                              int32_t* status, int grid, cudaStream_t s, const TcExtra& ex) {
     // Few sample tiles (short streaming batches): one work item per (tile,
     // pass of SPLIT_W templates) so that more SMs share the templates; the
-    // column maxima are then combined through 64-bit keys.
+    // column maxima are then combined through 64-bit keys. (Passes as narrow as
+    // give every SM one take as long for one probe, 57 us for 422 samples x 800
+    // templates, and slow four probes that share the device down by a sixth.)
     // A re-check of mapped rows (rowmap, count on the device) is usually one
     // or two tiles: its templates are split the same way, in narrower passes.
     const int ntiles = (N + tc::BM - 1) / tc::BM;
@@ -713,7 +724,7 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     const bool split = split_map || split_short || split_pass;
     const bool part_mode = split_pass && bounds_part;
     const TcPlan p = tc_plan(T, OP, split_map ? tc::MAPPED_SPLIT_W : (split_short ? tc::SPLIT_W : even_w));
-    if (p.stages < 2 || CKpad % p.kblock) return cudaErrorInvalidValue;
+    if (p.stages < 2 || p.b_rows > 256 || CKpad % p.kblock) return cudaErrorInvalidValue;
     CUtensorMap ma, malo, mb, mblo;
     if (!make_map(&ma, A, N, CKpad, ldk, tc::BM, OP) || !make_map(&mb, Bm, p.Tpad, CKpad, CKpad, p.box_rows, OP))
         return cudaErrorInvalidValue;
@@ -730,7 +741,6 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     a.T = T;
     a.Tpad = p.Tpad;
     a.KB = CKpad / p.kblock;
-    a.box_rows = p.box_rows;
     a.stages = p.stages;
     a.b_rows = p.b_rows;
     a.nacc = p.nacc;
