@@ -435,8 +435,8 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
     ALLOC(colkey, 2 * ld);
     h->mp_nb = (T + MPB_ROWS - 1) / MPB_ROWS;
     // The deferred rounds are the faster ones at every size measured (B200, rounds of one batch, against
-    // updating every row): 2.72 vs 7.68 ms at 384 channels, 800 templates, 60000 samples, 0.90 vs 2.06 at 400
-    // templates, 0.122 vs 0.160 at 64 channels and 32 templates, 0.038 vs 0.047 there on 300 samples. Slices
+    // updating every row): 2.00 vs 7.67 ms at 384 channels, 800 templates, 60000 samples, 0.72 vs 2.06 at 400
+    // templates, 0.107 vs 0.159 at 64 channels and 32 templates, 0.038 vs 0.043 there on 300 samples. Slices
     // too wide for their shared memory (batches of millions of samples) update every row.
     h->mp_lazy = mp_lazy_fits(h->N, h->mp_grid, T, nt);
     h->mp_switch = T >= 600;
