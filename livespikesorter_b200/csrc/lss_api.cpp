@@ -506,6 +506,7 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
     }
     CK(cudaMemcpy(h->nm.p, nmv.data(), T * sizeof(float), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->wave.p, wave.data(), wave.size() * sizeof(float), cudaMemcpyHostToDevice));
+    h->h_wpca.assign(t->wpca, t->wpca + (size_t)K * nt);
     CK(cudaMemcpy(h->wpca.p, t->wpca, (size_t)K * nt * sizeof(float), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->U.p, t->wall3, (size_t)T * K * C * sizeof(float), cudaMemcpyHostToDevice));
     if (hp_fft) {
@@ -702,7 +703,7 @@ int lss::run_scores(lss_handle* h, const float* X, int64_t ldx, int64_t N, float
                    bool* maxima_ready, bool folded, bool tiled) {
     const int tiles = tiled ? h->mp_nb : 0;
     if (h->cfg.precision == LSS_PREC_BF16_RECHECK) {
-        CK(launch_pca_proj_t(X, ldx, h->C, N, h->wpca.p, h->K, h->nt, h->B0T.p, h->B0T16lo.p, h->CKpad, s, h->pn2.p));
+        CK(launch_pca_proj_t(X, ldx, h->C, N, h->wpca.p, h->h_wpca.data(), h->K, h->nt, h->B0T.p, h->B0T16lo.p, h->CKpad, s, h->pn2.p));
         h->mark(5, s);
         TcExtra ex;
         ex.cf2 = h->cf2.p;
@@ -755,7 +756,7 @@ int lss::run_scores(lss_handle* h, const float* X, int64_t ldx, int64_t N, float
         if (maxima_ready) *maxima_ready = true;
         return LSS_OK;
     }
-    CK(launch_pca_proj_t_tf32(X, ldx, h->C, N, h->wpca.p, h->K, h->nt, h->B0T_hi.p, h->B0T_lo.p, h->CKpad, s));
+    CK(launch_pca_proj_t_tf32(X, ldx, h->C, N, h->wpca.p, h->h_wpca.data(), h->K, h->nt, h->B0T_hi.p, h->B0T_lo.p, h->CKpad, s));
     h->mark(5, s);
     TcExtra ex;
     ex.keys = h->colkey.p;  // free until the rounds start (they clear it)

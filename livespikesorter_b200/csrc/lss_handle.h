@@ -44,6 +44,7 @@ struct lss_handle {
     int mp_grid = 0;
     size_t dev_bytes = 0;                        // device memory allocated by lss_create
     std::vector<float> h_hp;
+    std::vector<float> h_wpca;                   // [K, nt] basis (kernel arguments of the projection)
     lss_stats stats{};
     bool prof = false;
     bool capturing = false;                      // inside a graph capture: no host-side copies or timing events

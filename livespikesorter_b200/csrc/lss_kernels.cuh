@@ -49,7 +49,8 @@ cudaError_t launch_sgemm_folded(const float* U, const float* Mw, int32_t T, int3
 // transposed bf16 variant for the tensor-core GEMM: B0T[s, c*K + k], row stride ldk
 // bf16 split (hi, lo = bf16(x - hi)) of the projection for the BF16x3 GEMM;
 // norm2 (optional, [N]): ||B0T[s, :]||^2 of the FP32 values before rounding
-cudaError_t launch_pca_proj_t(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t K,
+cudaError_t launch_pca_proj_t(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca,
+                              const float* wpca_host, int32_t K,
                               int32_t nt, __nv_bfloat16* B0T_hi, __nv_bfloat16* B0T_lo, int64_t ldk, cudaStream_t s,
                               float* norm2 = nullptr);
 
@@ -116,7 +117,8 @@ cudaError_t launch_score_tc_tf32x3(const float* B0T_hi, const float* B0T_lo, int
                                    float* cfmax, int32_t* imax, int nt, int32_t* status, int grid, cudaStream_t s,
                                    const TcExtra& ex = TcExtra());
 // transposed projection split into tf32 hi/lo parts (fp32 containers) for the 3xTF32 GEMM
-cudaError_t launch_pca_proj_t_tf32(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t K,
+cudaError_t launch_pca_proj_t_tf32(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca,
+                                   const float* wpca_host, int32_t K,
                                    int32_t nt, float* hi, float* lo, int64_t ldk, cudaStream_t s);
 
 // U_w[t, c'*K + k] = sum_c U[t,k,c] Mw[c,c'] in GEMM layout: bf16 split (out16, out16lo) and/or tf32

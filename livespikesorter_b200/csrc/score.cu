@@ -6,6 +6,8 @@
 // template matrix permuted once at set-up to U_p[t, c*K + k] = U[t, k, c].
 #include "lss_kernels.cuh"
 
+#include <cstring>
+
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -43,34 +45,43 @@ __device__ __forceinline__ unsigned long long dup2(float x) {
     return v;
 }
 
+// A basis of up to 64 taps as kernel arguments: pairs of components by tap (zero
+// past nt and K), which the packed FMAs read from the constant bank.
+struct PcaTaps {
+    unsigned long long w[64 * 4];
+};
+
 // Thread = (channel, 8-sample group) with the channel fastest across a warp,
 // so the K values a thread writes per sample land next to its neighbours'
 // and a warp writes 32*K contiguous outputs per sample row. The FP32 pipe bounds
-// it (17 GFLOP at 384 channels x 60122 samples, K = 6, nt = 61: 0.24 ms at the FP32
-// peak), so components go in pairs through packed FMAs and one sample load, one
-// duplication and K/4 weight loads serve 8K of them: 0.43 ms with the tf32 split
-// (0.49 with one FMA per instruction; a packed one takes the pipe two cycles, what
-// it saves is issue slots). A walk over several tiles per CTA with the next one's
-// samples copied ahead and rows staged per warp was slower (0.45 ms).
+// it (17 GFLOP at 384 channels x 60122 samples, K = 6, nt = 61: 0.23 ms at the FP32
+// peak), so components go in pairs through packed FMAs and one sample load and one
+// duplication serve 8K of them. Up to 64 taps the weights come from the kernel's
+// arguments: 0.36 ms with the tf32 split, 0.42 with two weight loads from shared
+// memory per tap (0.49 with one FMA per instruction; a packed one takes the pipe
+// two cycles and more, what it saves is issue slots). A walk over several tiles per
+// CTA with the next one's samples copied ahead and rows staged per warp was slower.
 template <int KPC, int PC, bool TF32, int NTP>
 __global__ void __launch_bounds__(256, KPC <= 6 ? 3 : 2) k_pca_proj_t(const float* __restrict__ X, int64_t ldx, int32_t C, int64_t N,
                                                     const float* __restrict__ wpca, int32_t nt, void* __restrict__ out0,
                                                     void* __restrict__ out_lo, int64_t ldk,
-                                                    float* __restrict__ norm2) {
+                                                    float* __restrict__ norm2, const __grid_constant__ PcaTaps taps) {
     extern __shared__ __align__(16) float sm[];
     const int64_t s0 = (int64_t)blockIdx.x * PT_S;
     const int ntp = NTP ? NTP : (nt + 7) & ~7;     // taps padded to 8 (zero weights)
     const int xw = PT_S + ntp + 9;                 // staged samples per channel row (odd: no bank conflicts)
     constexpr int KP = (KPC + 1) / 2;              // pairs of components (the last may be half empty)
-    float* ws = sm;                                // [ntp][2 KP]: a tap's components
-    float* xs = ws + 2 * KP * ntp;                 // [PC][xw]
-    float* stage = sm + ((2 * KP * ntp + PC * xw + 3) & ~3);  // [PT_S][PC*KPC], 16-byte aligned
+    float* ws = sm;                                // [ntp][2 KP]: a tap's components (no fixed tap count)
+    float* xs = ws + (NTP ? 0 : 2 * KP * ntp);     // [PC][xw]
+    float* stage = sm + (((NTP ? 0 : 2 * KP * ntp) + PC * xw + 3) & ~3);  // [PT_S][PC*KPC], 16-byte aligned
     const int c0 = blockIdx.y * PC;
     const int nc = min(PC, C - c0);
     const int half = nt / 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    for (int k = warp; k < 2 * KP; k += nwarps)
-        for (int m = lane; m < ntp; m += 32) ws[m * 2 * KP + k] = (m < nt && k < KPC) ? wpca[k * nt + m] : 0.f;
+    if constexpr (NTP == 0) {
+        for (int k = warp; k < 2 * KP; k += nwarps)
+            for (int m = lane; m < ntp; m += 32) ws[m * 2 * KP + k] = (m < nt && k < KPC) ? wpca[k * nt + m] : 0.f;
+    }
     if constexpr (NTP > 0 && PC % 8 == 0) {
         // fixed tap count: a warp's channel rows loaded into registers first, so
         // that all of them are in flight at once, then stored (256 threads)
@@ -124,12 +135,17 @@ __global__ void __launch_bounds__(256, KPC <= 6 ? 3 : 2) k_pca_proj_t(const floa
             for (int u = 0; u < 8; u += 2) {
                 // the weights of two taps (whole 16-byte pieces)
                 unsigned long long wt[2 * KP];
-                const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(ws + (mb + u) * 2 * KP);
+                if constexpr (NTP > 0) {
 #pragma unroll
-                for (int k = 0; k < KP; ++k) {
-                    const ulonglong2 p = wp[k];
-                    wt[2 * k] = p.x;
-                    wt[2 * k + 1] = p.y;
+                    for (int k = 0; k < 2 * KP; ++k) wt[k] = taps.w[(mb + u) * KP + k];
+                } else {
+                    const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(ws + (mb + u) * 2 * KP);
+#pragma unroll
+                    for (int k = 0; k < KP; ++k) {
+                        const ulonglong2 p = wp[k];
+                        wt[2 * k] = p.x;
+                        wt[2 * k + 1] = p.y;
+                    }
                 }
 #pragma unroll
                 for (int v = 0; v < 2; ++v) {
@@ -215,53 +231,62 @@ __global__ void __launch_bounds__(256, KPC <= 6 ? 3 : 2) k_pca_proj_t(const floa
 }
 
 template <int KPC, bool TF32>
-static cudaError_t launch_pjt(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t nt,
-                              void* out0, void* out_lo, int64_t ldk, float* norm2, cudaStream_t s) {
+static cudaError_t launch_pjt(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, const float* wpca_host,
+                              int32_t nt, void* out0, void* out_lo, int64_t ldk, float* norm2, cudaStream_t s) {
     constexpr int PC = 32;
     const int ntp = (nt + 7) & ~7;
-    const size_t smem = sizeof(float) * ((size_t)(KPC + 1) / 2 * 2 * ntp + (size_t)PC * (PT_S + ntp + 9) + 4 + (size_t)PT_S * PC * KPC);
+    const size_t smem = sizeof(float) * ((ntp == 64 ? 0 : (size_t)(KPC + 1) / 2 * 2 * ntp) + (size_t)PC * (PT_S + ntp + 9) + 4 + (size_t)PT_S * PC * KPC);
     dim3 grid((unsigned)((N + PT_S - 1) / PT_S), (unsigned)((C + PC - 1) / PC));
+    PcaTaps taps{};
+    if (ntp == 64) {
+        constexpr int KP = (KPC + 1) / 2;
+        for (int m = 0; m < nt; ++m)
+            for (int k = 0; k < KPC; ++k)
+                std::memcpy(reinterpret_cast<float*>(&taps.w[m * KP + k / 2]) + k % 2, wpca_host + (int64_t)k * nt + m, 4);
+    }
     if (ntp == 64) {  // nt = 57..64 (Kilosort's 61): taps fully unrolled
         auto kern = k_pca_proj_t<KPC, PC, TF32, 64>;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2);
+        kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, taps);
     } else {
         auto kern = k_pca_proj_t<KPC, PC, TF32, 0>;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2);
+        kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, taps);
     }
     return cudaGetLastError();
 }
 
 template <bool TF32>
-static cudaError_t pjt_dispatch(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t K,
+static cudaError_t pjt_dispatch(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, const float* wpca_host, int32_t K,
                                 int32_t nt, void* out0, void* out_lo, int64_t ldk, float* norm2, cudaStream_t s) {
     if (norm2) {
         const cudaError_t e = cudaMemsetAsync(norm2, 0, sizeof(float) * N, s);
         if (e != cudaSuccess) return e;
     }
     switch (K) {
-        case 1: return launch_pjt<1, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
-        case 2: return launch_pjt<2, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
-        case 3: return launch_pjt<3, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
-        case 4: return launch_pjt<4, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
-        case 5: return launch_pjt<5, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
-        case 6: return launch_pjt<6, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
-        case 7: return launch_pjt<7, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
-        case 8: return launch_pjt<8, TF32>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, s);
+        case 1: return launch_pjt<1, TF32>(X, ldx, C, N, wpca, wpca_host, nt, out0, out_lo, ldk, norm2, s);
+        case 2: return launch_pjt<2, TF32>(X, ldx, C, N, wpca, wpca_host, nt, out0, out_lo, ldk, norm2, s);
+        case 3: return launch_pjt<3, TF32>(X, ldx, C, N, wpca, wpca_host, nt, out0, out_lo, ldk, norm2, s);
+        case 4: return launch_pjt<4, TF32>(X, ldx, C, N, wpca, wpca_host, nt, out0, out_lo, ldk, norm2, s);
+        case 5: return launch_pjt<5, TF32>(X, ldx, C, N, wpca, wpca_host, nt, out0, out_lo, ldk, norm2, s);
+        case 6: return launch_pjt<6, TF32>(X, ldx, C, N, wpca, wpca_host, nt, out0, out_lo, ldk, norm2, s);
+        case 7: return launch_pjt<7, TF32>(X, ldx, C, N, wpca, wpca_host, nt, out0, out_lo, ldk, norm2, s);
+        case 8: return launch_pjt<8, TF32>(X, ldx, C, N, wpca, wpca_host, nt, out0, out_lo, ldk, norm2, s);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t launch_pca_proj_t(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t K,
+cudaError_t launch_pca_proj_t(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca,
+                              const float* wpca_host, int32_t K,
                               int32_t nt, __nv_bfloat16* B0T_hi, __nv_bfloat16* B0T_lo, int64_t ldk, cudaStream_t s,
                               float* norm2) {
-    return pjt_dispatch<false>(X, ldx, C, N, wpca, K, nt, B0T_hi, B0T_lo, ldk, norm2, s);
+    return pjt_dispatch<false>(X, ldx, C, N, wpca, wpca_host, K, nt, B0T_hi, B0T_lo, ldk, norm2, s);
 }
 
-cudaError_t launch_pca_proj_t_tf32(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca, int32_t K,
+cudaError_t launch_pca_proj_t_tf32(const float* X, int64_t ldx, int32_t C, int64_t N, const float* wpca,
+                                   const float* wpca_host, int32_t K,
                                    int32_t nt, float* hi, float* lo, int64_t ldk, cudaStream_t s) {
-    return pjt_dispatch<true>(X, ldx, C, N, wpca, K, nt, hi, lo, ldk, nullptr, s);
+    return pjt_dispatch<true>(X, ldx, C, N, wpca, wpca_host, K, nt, hi, lo, ldk, nullptr, s);
 }
 
 
