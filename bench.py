@@ -312,15 +312,17 @@ def run_b200(args):
     tfl = peaks.get('bf16_tflops', 1590.0)
     src = 'measured' if peaks else 'fallback'
     if top == 'mp_ms':
-        ach = mp_bytes / (mean_st['mp_ms'] / 1e3) / 1e9
         kname, prof = 'k_mp_lazy (matching pursuit, deferred updates)', f'k_mp_lazy_384ch_{T}t.md'
-        roof = {'kernel': kname, 'bound': 'hbm', 'achieved': ach, 'peak': hbm, 'unit': 'GB/s',
-                'frac': ach / hbm, 'traffic': profile_traffic(prof),
+        traffic = profile_traffic(prof)
+        ach = (traffic or mp_bytes) / (mean_st['mp_ms'] / 1e3) / 1e9
+        roof = {'kernel': kname, 'bound': 'latency', 'achieved': ach, 'peak': hbm, 'unit': 'GB/s',
+                'frac': ach / hbm, 'traffic': traffic,
                 'traffic_source': 'ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload '
                                   f'(profiles/{prof})',
                 'algorithmic_bytes': mp_bytes, 'peak_source': src,
-                'note': 'achieved counts the algorithmic bytes of every row update; the deferred rounds make only '
-                        'the updates that can matter to a decision and move only `traffic`'}
+                'note': 'achieved counts `traffic` (every row updated where it is not recorded); the deferred rounds '
+                        'make only the updates that can matter to a decision, updating every row would move '
+                        '`algorithmic_bytes`'}
     else:
         ach = gemm_flops / (mean_st['score_ms'] / 1e3) / 1e12
         roof = {'kernel': 'k_score_tc (tcgen05 3xTF32 score GEMM)' if args.precision == 'fp32'
