@@ -302,7 +302,11 @@ int lss_set_templates(lss_handle* h, const float* U, const float* wPCA) {
     const int L2 = 2 * nt + 1, nd = 2 * nt - 1;
     cudaStream_t s = 0;
     SCK(cudaMemcpy(h->U.p, U, (size_t)T * K * C * sizeof(float), cudaMemcpyHostToDevice));
-    if (wPCA) SCK(cudaMemcpy(h->wpca.p, wPCA, (size_t)K * nt * sizeof(float), cudaMemcpyHostToDevice));
+    if (wPCA) {
+        SCK(cudaMemcpy(h->wpca.p, wPCA, (size_t)K * nt * sizeof(float), cudaMemcpyHostToDevice));
+        // the projection's kernel arguments are made from this copy
+        SCK(cudaMemcpy(h->h_wpca.data(), h->wpca.p, (size_t)K * nt * sizeof(float), cudaMemcpyDeviceToHost));
+    }
     Tmp<double> wtw, utu;
     SCK(wtw.alloc((size_t)K * K * L2));
     SCK(utu.alloc((size_t)T * K * T * K));
