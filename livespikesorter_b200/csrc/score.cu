@@ -295,7 +295,7 @@ cudaError_t launch_pca_proj_t_tf32(const float* X, int64_t ldx, int32_t C, int64
 // so that sum_kk U_w[t, kk] * P[s, kk] over the projection P of the
 // un-whitened batch equals the score of the whitened batch. Stored as bf16
 // (BF16 path) or as a tf32 hi/lo split (FP32 path), rows [Tpad, ldk]. The
-// product is the 64x64-tile FP32 GEMM with a store into that layout; every
+// product is the 64x128-tile FP32 GEMM with a store into that layout; every
 // output sums over c in order.
 cudaError_t launch_build_uw(const float* U, const float* Mw, int32_t T, int32_t K, int32_t C, int64_t ldk,
                             __nv_bfloat16* out16, __nv_bfloat16* out16lo, float* hi, float* lo, cudaStream_t s) {

@@ -6,7 +6,7 @@
 // myGPUhelpers.cu:262-336, in the reference).
 //
 // Shape: samples are the MMA's M (128 per tile, one TMEM lane each), templates
-// its N (up to 512 TMEM columns per pass; several passes when T > 512), the
+// its N (up to 256 TMEM columns per pass, two accumulators in turn), the
 // (channel, component) pairs its K (64 per pipeline stage = one 128-byte
 // swizzle row of bf16). Both operands are K-major, loaded by TMA with 128B
 // swizzle into a multi-stage shared-memory ring guarded by mbarriers.
@@ -705,7 +705,7 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     const int ntiles = (N + tc::BM - 1) / tc::BM;
     // templates in passes of at most 256 TMEM columns (equal widths): two
     // accumulators alternate, so one pass's epilogue drains while the next
-    // pass's MMAs run, and the smaller stages leave room for four of them
+    // pass's MMAs run, and the smaller stages leave room for five of them
     const int tpad = (T + 15) / 16 * 16;
     const int npass = (tpad + 255) / 256;
     const int even_w = ((tpad + npass - 1) / npass + 15) / 16 * 16;
