@@ -97,6 +97,23 @@ struct Outer<float, JC> {  // channels in pairs
     }
 };
 
+// R[c, col] by the definition, over the spikes [lo, hi), none of which adds to a
+// column outside its window.
+template <typename F>
+__device__ __noinline__ F recon_one(const F* __restrict__ U, const F* __restrict__ W, int K, int C, int nt,
+                                    const int32_t* __restrict__ xs, const int32_t* __restrict__ ys,
+                                    const F* __restrict__ as, int lo, int hi, int c, int64_t col) {
+    F acc = F(0);
+    for (int i = lo; i < hi; ++i) {
+        const int64_t m = col - xs[i] + nt / 2;
+        if (m < 0 || m >= nt) continue;
+        F w = F(0);
+        for (int k = 0; k < K; ++k) w += U[((int64_t)ys[i] * K + k) * C + c] * W[k * nt + m];
+        acc += as[i] * w;
+    }
+    return acc;
+}
+
 // xs/ys/as: spikes sorted by x. A warp owns 32 columns of 32 channels, a lane 8
 // channels by 4 columns (8 apart) in registers, and takes the tile's spikes in time
 // order, skipping the ones whose window misses its columns:
@@ -109,6 +126,8 @@ struct Outer<float, JC> {  // channels in pairs
 // 3.9 GFLOP done (a window covers 61 of the 92 columns it is taken over), over 92 MB
 // written: 182 us, against 296 us with one column per lane and 232 us with 8 x 8
 // outputs (two CTAs per SM instead of three, 61 of 124 columns).
+// The zeros beside W are no zeros beside an infinite or NaN amplitude or template
+// value: a sum that is not finite at the end is taken again by the definition.
 template <typename F, int SP>
 __global__ void __launch_bounds__(RF_THREADS, sizeof(F) == 4 ? 3 : 1)
     k_recon_fwd(const F* __restrict__ U, const F* __restrict__ W, int K, int C, int nt, const int32_t* __restrict__ xs,
@@ -181,11 +200,25 @@ __global__ void __launch_bounds__(RF_THREADS, sizeof(F) == 4 ? 3 : 1)
     }
     if (on) {
         F* out = R + (int64_t)(c0 + wc) * N + col;
+        F z = F(0);  // NaN once an output is not finite
 #pragma unroll
         for (int c = 0; c < 8; ++c)
 #pragma unroll
             for (int j = 0; j < JC; ++j)
-                if (c0 + wc + c < C && col + 8 * j < N) out[(int64_t)c * N + 8 * j] = acc.at(c, j);
+                if (c0 + wc + c < C && col + 8 * j < N) {
+                    const F v = acc.at(c, j);
+                    out[(int64_t)c * N + 8 * j] = v;
+                    z += F(0) * v;
+                }
+        if (z != F(0)) {
+#pragma unroll 1
+            for (int e = 0; e < 8 * JC; ++e) {
+                const int c = e / JC, j = e % JC;
+                if (c0 + wc + c >= C || col + 8 * j >= N) continue;
+                F* p = out + (int64_t)c * N + 8 * j;
+                if (!isfinite(*p)) *p = recon_one(U, W, K, C, nt, xs, ys, as, lo, hi, c0 + wc + c, col + 8 * j);
+            }
+        }
     }
 }
 
