@@ -416,11 +416,14 @@ __device__ __forceinline__ void pc_features_one(
 }
 
 // Projection-row path for ten nearest channels, K = KPC components known at
-// compile time. A CTA (one per SM) takes the spikes of `cols` columns: it first lists, in
-// matching order, every spike within nt of them (one pass over the spikes' columns
-// instead of a search of every round per spike); then a warp takes a spike at a
-// time. Lanes own quads of channels (whole lines of P and of the Mw rows per
-// load; a lane per feature reads ten lines per load and was bound by the L1) and
+// compile time. A CTA (one per SM) takes the spikes of `cols` columns, a piece of
+// them at a time: it first lists, in matching order, every spike within nt of the
+// piece (a round's spikes are in time order: a thread finds a round's share by
+// bisection, a warp copies it); then a warp takes a spike at a time. A piece whose
+// list would not fit is halved, a sparse one is followed by a wider one, so that the
+// time grows with the spikes whatever the length of the batch. Lanes own quads of
+// channels (whole lines of P and of the Mw rows per load, three quads in flight; a
+// lane per feature reads ten lines per load and was bound by the L1) and
 // sum all ten channels' features over them; the partial sums are combined and
 // dealt out together, a lane keeping half the features at every step (the same
 // additions as a butterfly per feature: 62 shuffles instead of 300 for 60
@@ -429,13 +432,17 @@ __device__ __forceinline__ void pc_features_one(
 // neighbour whose template is exactly zero on all of the spike's channels (urange:
 // a template's first and last channel that is not) subtracts nothing and is not
 // loaded; templates are local, on a 384-channel probe three of four are skipped.
-// 384 channels, 19.3k spikes of 800 templates: 0.16 ms (0.40 with a search of
-// every round per spike, five butterfly steps per feature and a neighbour at a time).
-constexpr int FS_LIST = 1024;   // spikes listed per CTA (more: the warps read the spikes themselves)
+// 384 channels, 19.9k spikes of 800 templates: 0.17 ms with the BF16 path's rows, 0.21
+// with the FP32 path's (0.40 with a search of every round per spike, five butterfly
+// steps per feature and a neighbour at a time). 32 channels, 0.68 spikes per sample:
+// 0.5 ms at 60000 samples, 2.4 at 300000, 9.0 at 1200000 (with one list for the CTA's
+// whole slice, and every spike read where it did not fit: 0.5, 176 and 2660).
+constexpr int FS_LIST = 1024;   // spikes listed per piece (more than a spike's neighbours may be: see fw_list)
 constexpr int FS_WARPS = 16;    // most warps of a CTA
 constexpr int FS_MIN_COLS = 16; // least columns of a CTA
 // neighbours per spike (all rounds, within +-nt), more are refused
 constexpr int fw_list(int K) { return K == 6 ? 256 : FT_LIST; }
+static_assert(FT_LIST < FS_LIST, "one column's list holds every spike's neighbours, or the batch is refused");
 constexpr int FS_NC = 10;
 constexpr int FS_NB = 4;        // neighbours whose templates are loaded together
 
@@ -460,282 +467,286 @@ __device__ __forceinline__ void halve(float* v, int lane) {
     }
 }
 
+// Of a round's spikes [lo, hi), in time order, the ones in columns [s0, s1): both ends
+// at once, since a load of either chain takes 300 cycles.
+__device__ __forceinline__ void columns_of(const int32_t* __restrict__ sp_x, int s0, int s1, int& lo, int& hi) {
+    int a0 = lo, b0 = hi, a1 = lo, b1 = hi;  // the first spike at or after s0 (s1) is in [a0, b0] ([a1, b1])
+    while (a0 < b0 || a1 < b1) {
+        const int m0 = (a0 + b0) >> 1, m1 = (a1 + b1) >> 1;
+        const int x0 = a0 < b0 ? __ldg(sp_x + m0) : 0, x1 = a1 < b1 ? __ldg(sp_x + m1) : 0;
+        if (a0 < b0) {
+            if (x0 < s0) a0 = m0 + 1; else b0 = m0;
+        }
+        if (a1 < b1) {
+            if (x1 < s1) a1 = m1 + 1; else b1 = m1;
+        }
+    }
+    lo = a0;
+    hi = a1;
+}
+
 template <int KPC, typename PT>
 __global__ void __launch_bounds__(32 * FS_WARPS, 1) k_pc_features(
     int32_t C, int32_t nt, int32_t T, const float* __restrict__ Mw, const float* __restrict__ Ut,
     const int2* __restrict__ urange, const float* __restrict__ R, const int64_t* __restrict__ iCC,
     const int64_t* __restrict__ iU, const float* __restrict__ Ucc, const int32_t* __restrict__ sp_x,
-    const int32_t* __restrict__ sp_y, const float* __restrict__ sp_amp, int32_t n, const int32_t* __restrict__ counters, float* __restrict__ tF,
+    const int32_t* __restrict__ sp_y, const float* __restrict__ sp_amp, const int32_t* __restrict__ round_start,
+    int32_t rounds, const int32_t* __restrict__ counters, float* __restrict__ tF,
     int32_t* status, const PT* __restrict__ Phi, const PT* __restrict__ Plo, int64_t ldp, int32_t cols) {
     constexpr int NC = FS_NC, F = NC * KPC, FP = (F + 31) / 32;
     constexpr bool ONE_J = KPC % FP == 0;  // a lane's features belong to one channel
     constexpr int NB = ONE_J ? FS_NB : FS_NB / 2;  // (registers)
     extern __shared__ __align__(16) float fs_sm[];
-    constexpr int NW = FS_WARPS;
+    constexpr int NW = FS_WARPS, NT = 32 * NW;
     float* Rs = fs_sm;  // [lag][k'][k]: R[k, k', lag]
     __shared__ int l_x[FS_LIST], l_y[FS_LIST], l_i[FS_LIST], l_own[FS_LIST];
     __shared__ float l_a[FS_LIST];
-    __shared__ int s_cnt[FS_WARPS], s_ocnt[FS_WARPS], s_next;
+    __shared__ int s_lo[NT], s_off[NT + 1], s_wtot[NW];  // of a round: its first listed spike, where it goes
+    __shared__ int s_at, s_w;  // the piece
+    __shared__ int s_n, s_own, s_next;  // its spikes listed and owned, the next to take
     __shared__ int s_ch[FS_WARPS][NC];  // the spike's channels
-    if (counters) n = counters[0];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const int nd = 2 * nt - 1;
-    const int s0 = blockIdx.x * cols;
-    // ---- the spikes near the CTA's columns, in matching order: every warp
-    // counts its share of the spikes, then writes it
-    const int per = (((n + NW - 1) / NW) + 3) & ~3;  // whole groups of 4
-    const int i_lo = min(n, wl * per), i_hi = min(n, i_lo + per);
-    int n_list = 0, n_own = 0;
-    for (int pass = 0; pass < 2; ++pass) {
-        int c_all = 0, c_own = 0;
-        if (pass)
-            for (int w = 0; w < NW; ++w) {
-                if (w < wl) {
-                    c_all += s_cnt[w];
-                    c_own += s_ocnt[w];
-                }
-                n_list += s_cnt[w];
-                n_own += s_ocnt[w];
-            }
-        if (pass && n_list > FS_LIST) break;
-        for (int ib = i_lo; ib < i_hi; ib += 512) {
-            int xs[4][4];  // four groups of 128 spikes in flight
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                const int i = ib + 128 * v + 4 * lane;
-                if (i + 4 <= i_hi) {
-                    const int4 q = __ldg(reinterpret_cast<const int4*>(sp_x + i));
-                    xs[v][0] = q.x;
-                    xs[v][1] = q.y;
-                    xs[v][2] = q.z;
-                    xs[v][3] = q.w;
-                } else {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) xs[v][u] = i + u < i_hi ? __ldg(sp_x + i + u) : INT_MIN;
-                }
-            }
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-            const int i = ib + 128 * v + 4 * lane;
-            const int(&xv)[4] = xs[v];
-            int m = 0, own = 0;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (xv[u] > s0 - nt && xv[u] < s0 + cols - 1 + nt) m |= 1 << u;
-                if (xv[u] >= s0 && xv[u] < s0 + cols) own |= 1 << u;
-            }
-            if (!__any_sync(0xffffffffu, m)) continue;
-            int inc = __popc(m), oinc = __popc(own);
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int a = __shfl_up_sync(0xffffffffu, inc, o), b = __shfl_up_sync(0xffffffffu, oinc, o);
-                if (lane >= o) {
-                    inc += a;
-                    oinc += b;
-                }
-            }
-            if (pass) {
-                int at = c_all + inc - __popc(m), oat = c_own + oinc - __popc(own);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if ((m >> u) & 1) {
-                        l_x[at] = xv[u];
-                        l_y[at] = __ldg(sp_y + i + u);
-                        l_a[at] = __ldg(sp_amp + i + u);
-                        l_i[at] = i + u;
-                        if ((own >> u) & 1) l_own[oat++] = at;
-                        ++at;
-                    }
-            }
-            c_all += __shfl_sync(0xffffffffu, inc, 31);
-            c_own += __shfl_sync(0xffffffffu, oinc, 31);
-            }
-        }
-        if (!pass) {
-            if (lane == 0) {
-                s_cnt[wl] = c_all;
-                s_ocnt[wl] = c_own;
-            }
-            if (threadIdx.x == 0) s_next = NW;
-            __syncthreads();
-            int any = 0;
-            for (int w = 0; w < NW; ++w) any += s_ocnt[w];
-            if (!any) return;  // no spike in these columns
-            for (int p = wl; p < KPC * KPC; p += NW)  // a warp per pair of components
-#pragma unroll 4
-                for (int d = lane; d < nd; d += 32)
-                    Rs[d * (KPC * KPC) + (p % KPC) * KPC + p / KPC] = __ldg(R + (int64_t)p * nd + d);
-        }
+    if (counters) rounds = counters[1];
+    if (threadIdx.x == 0) {
+        s_at = blockIdx.x * cols;
+        s_w = cols;
     }
+    for (int p = wl; p < KPC * KPC; p += NW)  // a warp per pair of components; they arrive while the spikes are listed
+        for (int d = lane; d < nd; d += 32)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(Rs + d * (KPC * KPC) + (p % KPC) * KPC + p / KPC)),
+                         "l"(R + (int64_t)p * nd + d)
+                         : "memory");
     __syncthreads();
-    const bool listed = n_list <= FS_LIST;
-    // spikes to scan for neighbours: the list, or (a list that is too long) all of them
-    const int n_scan = listed ? n_list : n;
-    for (int o = wl;;) {
-        // the o-th spike of the CTA's columns
-        int i = -1, x = 0, y = 0;
-        float amp = 0.f;
-        if (listed) {
-            if (o >= n_own) break;
-            const int e = l_own[o];
-            i = l_i[e];
-            x = l_x[e];
-            y = l_y[e];
-            amp = l_a[e];
-        } else {
-            if (o >= n) break;
-            i = o;
-            x = __ldg(sp_x + o);
-            y = __ldg(sp_y + o);
-            amp = __ldg(sp_amp + o);
+    // (what a piece is lives in shared memory: no register is held for it while spikes are worked on)
+    for (;;) {
+        const int s0 = s_at, w = min(s_w, (int)(blockIdx.x + 1) * cols - s0);
+        if (w <= 0) break;
+        if (threadIdx.x == 0) {
+            s_own = 0;
+            s_next = NW;
         }
-        int nx = 0;
-        if (lane == 0) nx = atomicAdd(&s_next, 1);
-        o = __shfl_sync(0xffffffffu, nx, 0);
-        if (x < s0 || x >= s0 + cols) continue;
-        const int64_t u = iU[y];
-        int chl = 0;  // lane j < NC holds channel j's index
-        if (lane < NC) chl = (int)iCC[(int64_t)lane * C + u];
-        const int ch_min = __reduce_min_sync(0xffffffffu, lane < NC ? chl : INT_MAX);
-        const int ch_max = __reduce_max_sync(0xffffffffu, lane < NC ? chl : -1);
-        __syncwarp();
-        if (lane < NC) s_ch[wl][lane] = chl;
-        __syncwarp();
-        // ---- sums over channels: acc[j * K + k] = sum_c Mw[ch_j, c] * P[x, c*K + k]
-        float acc[32 * FP];
+        // ---- the spikes near the piece's columns, in matching order
+        int n_list = 0;
+        for (int rb = 0; rb < rounds; rb += NT) {
+            const int r = rb + threadIdx.x;
+            int lo = 0, cnt = 0;
+            if (r < rounds) {
+                lo = __ldg(round_start + r);
+                cnt = __ldg(round_start + r + 1);
+                columns_of(sp_x, s0 - nt + 1, s0 + w - 1 + nt, lo, cnt);
+                cnt -= lo;
+            }
+            const int inc = warp_inc_scan(cnt, lane);
+            if (lane == 31) s_wtot[wl] = inc;
+            __syncthreads();
+            int before = n_list, total = n_list;
 #pragma unroll
-        for (int f = 0; f < 32 * FP; ++f) acc[f] = 0.f;
-        {
-            const PT* ph = Phi + (int64_t)x * ldp;
-            const PT* pl = Plo + (int64_t)x * ldp;
-            if ((C & 3) == 0) {  // (rows of P and Mw are then whole 16-byte pieces)
-                for (int c = 4 * lane; c < C; c += 128) {
-                    float pv[4 * KPC];
+            for (int v = 0; v < NW; ++v) {
+                if (v < wl) before += s_wtot[v];
+                total += s_wtot[v];
+            }
+            s_lo[threadIdx.x] = lo;
+            s_off[threadIdx.x] = before + inc - cnt;
+            if (threadIdx.x == 0) s_off[NT] = total;
+            __syncthreads();
+            n_list = total;
+            if (n_list > FS_LIST) break;
+            for (int q = wl; q < min(NT, rounds - rb); q += NW) {  // a warp per round
+                const int at = s_off[q], ne = s_off[q + 1] - at, i0 = s_lo[q];
+                for (int e = lane; e < ne; e += 32) {
+                    const int i = i0 + e, xe = __ldg(sp_x + i);
+                    l_x[at + e] = xe;
+                    l_y[at + e] = __ldg(sp_y + i);
+                    l_a[at + e] = __ldg(sp_amp + i);
+                    l_i[at + e] = i;
+                    if (xe >= s0 && xe < s0 + w) l_own[atomicAdd(&s_own, 1)] = at + e;
+                }
+            }
+            __syncthreads();
+        }
+        if (n_list > FS_LIST) {
+            if (w == 1) {  // a spike of this column has more neighbours than may be
+                bool own = false;
+                for (int r = threadIdx.x; r < rounds; r += NT) {
+                    int lo = __ldg(round_start + r), hi = __ldg(round_start + r + 1);
+                    columns_of(sp_x, s0, s0 + 1, lo, hi);
+                    own |= lo < hi;
+                }
+                if (own) atomicOr(status, STATUS_LIST);
+            }
+            if (threadIdx.x == 0) {
+                if (w == 1) ++s_at;
+                s_w = (w + 1) / 2;
+            }
+            __syncthreads();
+            continue;
+        }
+        if (threadIdx.x == 0) s_n = n_list;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        for (int o = wl; o < s_own;) {
+            // the o-th spike of these columns
+            const int e = l_own[o], i = l_i[e], x = l_x[e], y = l_y[e];
+            const float amp = l_a[e];
+            int nx = 0;
+            if (lane == 0) nx = atomicAdd(&s_next, 1);
+            o = __shfl_sync(0xffffffffu, nx, 0);
+            const int64_t u = iU[y];
+            int chl = 0;  // lane j < NC holds channel j's index
+            if (lane < NC) chl = (int)iCC[(int64_t)lane * C + u];
+            const int ch_min = __reduce_min_sync(0xffffffffu, lane < NC ? chl : INT_MAX);
+            const int ch_max = __reduce_max_sync(0xffffffffu, lane < NC ? chl : -1);
+            __syncwarp();
+            if (lane < NC) s_ch[wl][lane] = chl;
+            __syncwarp();
+            // ---- sums over channels: acc[j * K + k] = sum_c Mw[ch_j, c] * P[x, c*K + k]
+            float acc[32 * FP];
 #pragma unroll
-                    for (int e = 0; e < 4 * KPC; e += 4) {
-                        const float4 h = ld4(ph + c * KPC + e), l = ld4(pl + c * KPC + e);
-                        pv[e] = __fadd_rn(h.x, l.x);
-                        pv[e + 1] = __fadd_rn(h.y, l.y);
-                        pv[e + 2] = __fadd_rn(h.z, l.z);
-                        pv[e + 3] = __fadd_rn(h.w, l.w);
-                    }
+            for (int f = 0; f < 32 * FP; ++f) acc[f] = 0.f;
+            {
+                const PT* ph = Phi + (int64_t)x * ldp;
+                const PT* pl = Plo + (int64_t)x * ldp;
+                if ((C & 3) == 0) {  // (rows of P and Mw are then whole 16-byte pieces)
+#pragma unroll 3
+                    for (int c = 4 * lane; c < C; c += 128) {
+                        float pv[4 * KPC];
 #pragma unroll
-                    for (int j = 0; j < NC; ++j) {
-                        const float4 mv = ld4(Mw + (int64_t)s_ch[wl][j] * C + c);
-#pragma unroll
-                        for (int k = 0; k < KPC; ++k) {
-                            float v = acc[j * KPC + k];
-                            v = fmaf(mv.x, pv[k], v);
-                            v = fmaf(mv.y, pv[KPC + k], v);
-                            v = fmaf(mv.z, pv[2 * KPC + k], v);
-                            acc[j * KPC + k] = fmaf(mv.w, pv[3 * KPC + k], v);
+                        for (int e = 0; e < 4 * KPC; e += 4) {
+                            const float4 h = ld4(ph + c * KPC + e), l = ld4(pl + c * KPC + e);
+                            pv[e] = __fadd_rn(h.x, l.x);
+                            pv[e + 1] = __fadd_rn(h.y, l.y);
+                            pv[e + 2] = __fadd_rn(h.z, l.z);
+                            pv[e + 3] = __fadd_rn(h.w, l.w);
                         }
-                    }
-                }
-            } else {
-                for (int c = lane; c < C; c += 32) {
-                    float pv[KPC];
 #pragma unroll
-                    for (int k = 0; k < KPC; ++k) pv[k] = __fadd_rn(pval(ph + c * KPC + k), pval(pl + c * KPC + k));
+                        for (int j = 0; j < NC; ++j) {
+                            const float4 mv = ld4(Mw + (int64_t)s_ch[wl][j] * C + c);
 #pragma unroll
-                    for (int j = 0; j < NC; ++j) {
-                        const float mv = __ldg(Mw + (int64_t)s_ch[wl][j] * C + c);
-#pragma unroll
-                        for (int k = 0; k < KPC; ++k) acc[j * KPC + k] = fmaf(mv, pv[k], acc[j * KPC + k]);
-                    }
-                }
-            }
-        }
-        halve<16 * FP, 16>(acc, lane);
-        halve<8 * FP, 8>(acc, lane);
-        halve<4 * FP, 4>(acc, lane);
-        halve<2 * FP, 2>(acc, lane);
-        halve<FP, 1>(acc, lane);
-        // ---- this lane's features f = lane * FP + q
-        int jf[FP], kf[FP], cf[FP];
-#pragma unroll
-        for (int q = 0; q < FP; ++q) {
-            const int f = min(lane * FP + q, F - 1);
-            jf[q] = f / KPC;
-            kf[q] = f % KPC;
-            cf[q] = s_ch[wl][jf[q]];
-        }
-        // ---- neighbours (any round, matching order) whose window overlaps x's
-        int nl = 0;
-        for (int b0 = 0; b0 < n_scan; b0 += 32) {
-            const int e = b0 + lane;
-            int xq = INT_MIN, yq = 0;
-            float aq = 0.f;
-            if (e < n_scan) {
-                xq = listed ? l_x[e] : __ldg(sp_x + e);
-                if (xq > x - nt && xq < x + nt) {
-                    yq = listed ? l_y[e] : __ldg(sp_y + e);
-                    aq = listed ? l_a[e] : __ldg(sp_amp + e);
-                }
-            }
-            const bool near = xq > x - nt && xq < x + nt;
-            nl += __popc(__ballot_sync(0xffffffffu, near));
-            bool some = near;  // (an infinite amplitude times zero is not zero)
-            if (near && fabsf(aq) < INFINITY) {
-                const int2 ur = __ldg(urange + yq);
-                some = ur.x <= ch_max && ur.y >= ch_min;
-            }
-            unsigned m = __ballot_sync(0xffffffffu, some);
-            while (m) {
-                // the next NB neighbours (an = 0 past the last: it subtracts nothing)
-                int d[NB];
-                float an[NB], uv[NB][ONE_J ? 1 : FP][KPC];
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    const int src = m ? __ffs(m) - 1 : 0;
-                    const int yn = __shfl_sync(0xffffffffu, yq, src);
-                    const float ab = __shfl_sync(0xffffffffu, aq, src);
-                    const int xb = __shfl_sync(0xffffffffu, xq, src);
-                    const bool on = m != 0u;
-                    m &= m - 1u;
-                    d[b] = on ? x - xb + nt - 1 : -1;
-                    an[b] = ab;
-                    if (on) {
-#pragma unroll
-                        for (int q = 0; q < (ONE_J ? 1 : FP); ++q) {
-                            const float* uy = Ut + ((int64_t)yn * C + cf[q]) * KPC;
-                            if constexpr (KPC % 2 == 0) {
-#pragma unroll
-                                for (int kk = 0; kk < KPC; kk += 2) {
-                                    const float2 t = __ldg(reinterpret_cast<const float2*>(uy + kk));
-                                    uv[b][q][kk] = t.x;
-                                    uv[b][q][kk + 1] = t.y;
-                                }
-                            } else {
-#pragma unroll
-                                for (int kk = 0; kk < KPC; ++kk) uv[b][q][kk] = __ldg(uy + kk);
+                            for (int k = 0; k < KPC; ++k) {
+                                float v = acc[j * KPC + k];
+                                v = fmaf(mv.x, pv[k], v);
+                                v = fmaf(mv.y, pv[KPC + k], v);
+                                v = fmaf(mv.z, pv[2 * KPC + k], v);
+                                acc[j * KPC + k] = fmaf(mv.w, pv[3 * KPC + k], v);
                             }
                         }
                     }
-                }
+                } else {
+                    for (int c = lane; c < C; c += 32) {
+                        float pv[KPC];
 #pragma unroll
-                for (int b = 0; b < NB; ++b)
-                    if (d[b] >= 0) {
+                        for (int k = 0; k < KPC; ++k) pv[k] = __fadd_rn(pval(ph + c * KPC + k), pval(pl + c * KPC + k));
 #pragma unroll
-                        for (int q = 0; q < FP; ++q) {
-                            const float* rk = Rs + d[b] * (KPC * KPC) + kf[q];
-                            float sub = 0.f;
+                        for (int j = 0; j < NC; ++j) {
+                            const float mv = __ldg(Mw + (int64_t)s_ch[wl][j] * C + c);
 #pragma unroll
-                            for (int kk = 0; kk < KPC; ++kk) sub = fmaf(uv[b][ONE_J ? 0 : q][kk], rk[kk * KPC], sub);
-                            acc[q] = __fsub_rn(acc[q], __fmul_rn(an[b], sub));
+                            for (int k = 0; k < KPC; ++k) acc[j * KPC + k] = fmaf(mv, pv[k], acc[j * KPC + k]);
                         }
                     }
+                }
+            }
+            halve<16 * FP, 16>(acc, lane);
+            halve<8 * FP, 8>(acc, lane);
+            halve<4 * FP, 4>(acc, lane);
+            halve<2 * FP, 2>(acc, lane);
+            halve<FP, 1>(acc, lane);
+            // ---- this lane's features f = lane * FP + q
+            int jf[FP], kf[FP], cf[FP];
+#pragma unroll
+            for (int q = 0; q < FP; ++q) {
+                const int f = min(lane * FP + q, F - 1);
+                jf[q] = f / KPC;
+                kf[q] = f % KPC;
+                cf[q] = s_ch[wl][jf[q]];
+            }
+            // ---- neighbours (any round, matching order) whose window overlaps x's
+            int nl = 0;
+            const int n_list = s_n;
+            for (int b0 = 0; b0 < n_list; b0 += 32) {
+                const int q = b0 + lane;
+                int xq = INT_MIN, yq = 0;
+                float aq = 0.f;
+                if (q < n_list) {
+                    xq = l_x[q];
+                    if (xq > x - nt && xq < x + nt) {
+                        yq = l_y[q];
+                        aq = l_a[q];
+                    }
+                }
+                const bool near = xq > x - nt && xq < x + nt;
+                nl += __popc(__ballot_sync(0xffffffffu, near));
+                bool some = near;  // (an infinite amplitude times zero is not zero)
+                if (near && fabsf(aq) < INFINITY) {
+                    const int2 ur = __ldg(urange + yq);
+                    some = ur.x <= ch_max && ur.y >= ch_min;
+                }
+                unsigned m = __ballot_sync(0xffffffffu, some);
+                while (m) {
+                    // the next NB neighbours (an = 0 past the last: it subtracts nothing)
+                    int d[NB];
+                    float an[NB], uv[NB][ONE_J ? 1 : FP][KPC];
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        const int src = m ? __ffs(m) - 1 : 0;
+                        const int yn = __shfl_sync(0xffffffffu, yq, src);
+                        const float ab = __shfl_sync(0xffffffffu, aq, src);
+                        const int xb = __shfl_sync(0xffffffffu, xq, src);
+                        const bool on = m != 0u;
+                        m &= m - 1u;
+                        d[b] = on ? x - xb + nt - 1 : -1;
+                        an[b] = ab;
+                        if (on) {
+#pragma unroll
+                            for (int q = 0; q < (ONE_J ? 1 : FP); ++q) {
+                                const float* uy = Ut + ((int64_t)yn * C + cf[q]) * KPC;
+                                if constexpr (KPC % 2 == 0) {
+#pragma unroll
+                                    for (int kk = 0; kk < KPC; kk += 2) {
+                                        const float2 t = __ldg(reinterpret_cast<const float2*>(uy + kk));
+                                        uv[b][q][kk] = t.x;
+                                        uv[b][q][kk + 1] = t.y;
+                                    }
+                                } else {
+#pragma unroll
+                                    for (int kk = 0; kk < KPC; ++kk) uv[b][q][kk] = __ldg(uy + kk);
+                                }
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int b = 0; b < NB; ++b)
+                        if (d[b] >= 0) {
+#pragma unroll
+                            for (int q = 0; q < FP; ++q) {
+                                const float* rk = Rs + d[b] * (KPC * KPC) + kf[q];
+                                float sub = 0.f;
+#pragma unroll
+                                for (int kk = 0; kk < KPC; ++kk) sub = fmaf(uv[b][ONE_J ? 0 : q][kk], rk[kk * KPC], sub);
+                                acc[q] = __fsub_rn(acc[q], __fmul_rn(an[b], sub));
+                            }
+                        }
+                }
+            }
+            if (nl > fw_list(KPC) && lane == 0) atomicOr(status, STATUS_LIST);
+#pragma unroll
+            for (int q = 0; q < FP; ++q) {
+                const int f = lane * FP + q;
+                if (f < F)
+                    tF[(int64_t)i * F + f] =
+                        __fadd_rn(acc[q], __fmul_rn(amp, Ucc[((int64_t)jf[q] * T + y) * KPC + kf[q]]));
             }
         }
-        if (nl > fw_list(KPC) && lane == 0) atomicOr(status, STATUS_LIST);
-#pragma unroll
-        for (int q = 0; q < FP; ++q) {
-            const int f = lane * FP + q;
-            if (f < F)
-                tF[(int64_t)i * F + f] =
-                    __fadd_rn(acc[q], __fmul_rn(amp, Ucc[((int64_t)jf[q] * T + y) * KPC + kf[q]]));
+        __syncthreads();  // the list has been read
+        if (threadIdx.x == 0) {
+            const int done = min(s_w, (int)(blockIdx.x + 1) * cols - s_at);
+            s_at += done;
+            s_w = s_n < FS_LIST / 2 ? min(2 * done, cols) : done;
         }
+        __syncthreads();
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // CTA per spike, grid-stride over the spikes; with counters != null the spike
@@ -764,7 +775,8 @@ __global__ void __launch_bounds__(256) k_pc_features_folded(
 template <int KPC, typename PT>
 static cudaError_t launch_pcs(int32_t C, int32_t N, int32_t nt, int32_t T, const float* Mw, const float* Ut, const int2* urange, const float* R,
                               const int64_t* iCC, const int64_t* iU, const float* Ucc, const int32_t* sp_x,
-                              const int32_t* sp_y, const float* sp_amp, int32_t n, const int32_t* counters, float* tF,
+                              const int32_t* sp_y, const float* sp_amp, const int32_t* round_start, int32_t rounds,
+                              const int32_t* counters, float* tF,
                               int32_t* status, const PT* Phi, const PT* Plo, int64_t ldp, size_t smem, cudaStream_t s) {
     const cudaError_t e = cudaFuncSetAttribute(k_pc_features<KPC, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -774,8 +786,8 @@ static cudaError_t launch_pcs(int32_t C, int32_t N, int32_t nt, int32_t T, const
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int cols = std::max(FS_MIN_COLS, (N + sms - 1) / std::max(sms, 1));
     k_pc_features<KPC, PT><<<(N + cols - 1) / cols, 32 * FS_WARPS, smem, s>>>(C, nt, T, Mw, Ut, urange, R, iCC, iU, Ucc, sp_x, sp_y,
-                                                                          sp_amp, n, counters, tF, status, Phi, Plo, ldp,
-                                                                          cols);
+                                                                          sp_amp, round_start, rounds, counters, tF, status,
+                                                                          Phi, Plo, ldp, cols);
     return cudaGetLastError();
 }
 
@@ -794,8 +806,8 @@ static cudaError_t launch_pcf(const float* Xh, int64_t ldx, int32_t C, int32_t n
     if (Phi && nC == FS_NC && K >= 1 && K <= 8 && rs <= 180 * 1024) {
 #define LSS_PCS(k)                                                                                                       \
     case k:                                                                                                              \
-        return launch_pcs<k, PT>(C, N, nt, T, Mw, Ut, urange, R, iCC, iU, Ucc, sp_x, sp_y, sp_amp, n, counters, tF, status, Phi, \
-                                 Plo, ldp, rs, s)
+        return launch_pcs<k, PT>(C, N, nt, T, Mw, Ut, urange, R, iCC, iU, Ucc, sp_x, sp_y, sp_amp, round_start, rounds, counters, \
+                                 tF, status, Phi, Plo, ldp, rs, s)
         switch (K) {
             LSS_PCS(1);
             LSS_PCS(2);
