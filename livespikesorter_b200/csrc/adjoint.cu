@@ -405,8 +405,7 @@ static cudaError_t recon_fwd(const void* U, const void* W, int K, int C, int nt,
                              const void* as, int n, void* R, int64_t N, cudaStream_t s) {
     constexpr int SP = sizeof(F) == 4 ? 8 : 4, COLS = 16 * RF_JC;
     const size_t smem = sizeof(F) * ((size_t)2 * SP * K * RF_CH + (size_t)K * (nt + COLS));
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_recon_fwd<F, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_shared_memory<k_recon_fwd<F, SP>>();
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((N + COLS - 1) / COLS), (unsigned)((C + RF_CH - 1) / RF_CH));
     k_recon_fwd<F, SP><<<grid, RF_THREADS, smem, s>>>(static_cast<const F*>(U), static_cast<const F*>(W), K, C, nt, xs,
@@ -421,9 +420,8 @@ static cudaError_t recon_bwd_nm(const F* U, const F* W, int T, int K, int C, int
                                 F* damp, cudaStream_t s) {
     constexpr int CH = RB_WARPS * (8 / NM);
     const size_t smem = sizeof(F) * (2 * (size_t)K * nt + (size_t)K * CH + (size_t)CH * (nt | 1) + RB_SP * RB_WARPS);
-    auto kern = k_recon_bwd<F, NM>;
     // (always: with the static arrays a size just below 48 KB needs it too)
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_shared_memory<k_recon_bwd<F, NM>>();
     if (e != cudaSuccess) return e;
     const int Z = std::min(RB_MAXZ, (C + CH - 1) / CH);
     cudaLaunchConfig_t lc = {};
@@ -438,7 +436,7 @@ static cudaError_t recon_bwd_nm(const F* U, const F* W, int T, int K, int C, int
     attr[0].val.clusterDim.z = 1;
     lc.attrs = attr;
     lc.numAttrs = 1;
-    return cudaLaunchKernelEx(&lc, kern, U, W, K, C, nt, x, amp, order, tstart, G, N, dU, work, damp);
+    return cudaLaunchKernelEx(&lc, k_recon_bwd<F, NM>, U, W, K, C, nt, x, amp, order, tstart, G, N, dU, work, damp);
 }
 
 template <typename F>

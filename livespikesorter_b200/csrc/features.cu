@@ -778,7 +778,7 @@ static cudaError_t launch_pcs(int32_t C, int32_t N, int32_t nt, int32_t T, const
                               const int32_t* sp_y, const float* sp_amp, const int32_t* round_start, int32_t rounds,
                               const int32_t* counters, float* tF,
                               int32_t* status, const PT* Phi, const PT* Plo, int64_t ldp, size_t smem, cudaStream_t s) {
-    const cudaError_t e = cudaFuncSetAttribute(k_pc_features<KPC, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_shared_memory<k_pc_features<KPC, PT>>();
     if (e != cudaSuccess) return e;
     // one CTA per SM
     int dev = 0, sms = 0;
@@ -825,8 +825,10 @@ static cudaError_t launch_pcf(const float* Xh, int64_t ldx, int32_t C, int32_t n
                                               (size_t)nC * FT_CH,
                                           (size_t)C * K + (size_t)nC * C + 4 * (size_t)nC * K);
     const size_t smem = sizeof(float) * (front + (size_t)nC * K + (size_t)FT_NQ * nC * K);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_pc_features_folded<PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) {
+        const cudaError_t e = allow_shared_memory<k_pc_features_folded<PT>>();
+        if (e != cudaSuccess) return e;
+    }
     // n: the spike count, or (counters != null) the grid size
     k_pc_features_folded<PT><<<n, 256, smem, s>>>(Xh, ldx, C, nt, K, nC, T, wpca, Mw, U, R, iCC, iU, Ucc, sp_x,
                                                   sp_y, sp_amp, round_start, rounds, n, counters, tF, status, Phi, Plo,

@@ -284,7 +284,8 @@ static cudaError_t launch_car_cols(const int16_t* raw, int32_t ld_raw, const int
                                    IngestMap map, float sign, const long long* sums, int do_car, float* X1, int64_t ldx,
                                    cudaStream_t s) {
     const size_t smem = sizeof(float) * (8 * 32 + (size_t)C * (COLS + 1) + 2 * NQ * 32);
-    cudaFuncSetAttribute(k_car<NQ, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    const cudaError_t e = allow_shared_memory<k_car<NQ, COLS>>();
+    if (e != cudaSuccess) return e;
     k_car<NQ, COLS><<<(unsigned)((N + COLS - 1) / COLS), 256, smem, s>>>(raw, ld_raw, chan_map, C, N, map, sign, sums,
                                                                          do_car, X1, ldx);
     return cudaGetLastError();
@@ -371,11 +372,8 @@ cudaError_t launch_highpass(const float* X1, int64_t ldx, int32_t C, int64_t N, 
                             float* Xh, cudaStream_t s) {
     const int ntap_pad = ((2 * L + 1) + 7) & ~7;
     const size_t smem = sizeof(float) * ((size_t)ntap_pad + HP_TILE + ntap_pad + 8);
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(k_highpass, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr_done = true;
-    }
+    const cudaError_t e = allow_shared_memory<k_highpass>();
+    if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((N + HP_TILE - 1) / HP_TILE), (unsigned)C);
     k_highpass<<<grid, HP_THREADS, smem, s>>>(X1, ldx, N, taps, L, Xh);
     return cudaGetLastError();
@@ -541,7 +539,8 @@ cudaError_t launch_highpass_fft(const float* X1, int64_t ldx, int32_t C, int64_t
                                 const float2* tw, float* Xh, cudaStream_t s) {
     if (L > 1024) return cudaErrorInvalidValue;
     const size_t smem = HFP * sizeof(float2);
-    cudaFuncSetAttribute(k_highpass_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_shared_memory<k_highpass_fft>();
+    if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((N + (HF - 2 * L) - 1) / (HF - 2 * L)), (unsigned)((C + 1) / 2));
     k_highpass_fft<<<grid, HF_THREADS, smem, s>>>(X1, ldx, C, N, L, H, tw, Xh);
     return cudaGetLastError();

@@ -5,7 +5,36 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace lss {
+
+// Dynamic shared memory that a block of this kernel may have on the current device
+// (0: not known).
+template <auto Kernel>
+size_t shared_memory_room() {
+    static std::atomic<size_t> room{0};
+    size_t r = room.load(std::memory_order_relaxed);
+    if (!r) {
+        int dev = 0, optin = 0;
+        cudaFuncAttributes fa{};
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+            cudaFuncGetAttributes(&fa, Kernel) != cudaSuccess)
+            return 0;
+        r = (size_t)optin - fa.sharedSizeBytes;
+        room.store(r, std::memory_order_relaxed);
+    }
+    return r;
+}
+// ... and leave to take it. The limit belongs to the kernel, not to a launch: set from
+// one call's sizes, it may be lowered by another thread's call before the launch, which
+// is then refused.
+template <auto Kernel>
+cudaError_t allow_shared_memory() {
+    const size_t r = shared_memory_room<Kernel>();
+    return r ? cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r) : cudaErrorUnknown;
+}
 
 // Where column s of the padded batch X [C, N] comes from in the raw rows
 // (kilosort/io.py:584-637): row = clamp(s - lead, 0, nsamp-1); columns at or

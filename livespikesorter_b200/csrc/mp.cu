@@ -365,7 +365,7 @@ cudaError_t launch_mp(MPArgs a, int grid, cudaStream_t s) {
     if (grid > MP_MAX_GRID) return cudaErrorInvalidValue;
     const size_t smem = mp_smem_bytes(a.cols_per_blk, a.nt, a.T);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_mp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_shared_memory<k_mp>();
         if (e != cudaSuccess) return e;
     }
     cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned int), s);

@@ -735,11 +735,7 @@ __global__ void __launch_bounds__(128) k_tile_ctc(const float* __restrict__ ctcP
 
 cudaError_t launch_tile_ctc(const float* ctcP, const int32_t* perm, const float* nm, int32_t T, int32_t L2, float* ctct,
                             float2* hg, cudaStream_t s) {
-    const size_t smem = sizeof(float) * MPB_ROWS * (size_t)(L2 | 1);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(k_tile_ctc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const size_t smem = sizeof(float) * MPB_ROWS * (size_t)(L2 | 1);  // at most 33 KB (511 lags)
     k_tile_ctc<<<dim3((unsigned)T, (unsigned)((T + MPB_ROWS - 1) / MPB_ROWS)), 128, smem, s>>>(ctcP, perm, nm, T, L2, ctct, hg);
     return cudaGetLastError();
 }
@@ -843,15 +839,7 @@ static size_t mpl_smem_bytes(int W, int nt, int T, bool ksmem) {
            4 * (3 * w + 2 * nt_ + 3 * nb * MPB_ROWS + T + nb + 4 * cpc * nb + 2 * cpc);
 }
 
-static size_t mpl_room() {
-    int dev = 0, optin = 0;
-    cudaFuncAttributes fa{};
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa, k_mp_lazy<true>) != cudaSuccess)
-        return 0;
-    return (size_t)optin - fa.sharedSizeBytes;
-}
+static size_t mpl_room() { return std::min(shared_memory_room<k_mp_lazy<true>>(), shared_memory_room<k_mp_lazy<false>>()); }
 
 bool mp_lazy_fits(int64_t N, int grid, int T, int nt) {
     if (N >= (1 << 28) || T >= (1 << 24) || grid < 1 || grid > MPL_MAX_GRID) return false;
@@ -862,7 +850,7 @@ int64_t mp_lazy_words(int64_t N) { return 2 * MPL_MAX_GRID + 5 * (2 * N + 64); }
 
 template <bool KSMEM>
 static cudaError_t launch_lazy(const MPArgs& a, int grid, size_t smem, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(k_mp_lazy<KSMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_shared_memory<k_mp_lazy<KSMEM>>();
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(grid);

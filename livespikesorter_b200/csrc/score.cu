@@ -245,12 +245,14 @@ static cudaError_t launch_pjt(const float* X, int64_t ldx, int32_t C, int64_t N,
                 std::memcpy(reinterpret_cast<float*>(&taps.w[m * KP + k / 2]) + k % 2, wpca_host + (int64_t)k * nt + m, 4);
     }
     if (ntp == 64) {  // nt = 57..64 (Kilosort's 61): taps fully unrolled
-        auto kern = k_pca_proj_t<KPC, PC, TF32, 64>;
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        constexpr auto kern = k_pca_proj_t<KPC, PC, TF32, 64>;
+        const cudaError_t e = allow_shared_memory<kern>();
+        if (e != cudaSuccess) return e;
         kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, taps);
     } else {
-        auto kern = k_pca_proj_t<KPC, PC, TF32, 0>;
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        constexpr auto kern = k_pca_proj_t<KPC, PC, TF32, 0>;
+        const cudaError_t e = allow_shared_memory<kern>();
+        if (e != cudaSuccess) return e;
         kern<<<grid, 256, smem, s>>>(X, ldx, C, N, wpca, nt, out0, out_lo, ldk, norm2, taps);
     }
     return cudaGetLastError();

@@ -319,7 +319,7 @@ int lss_set_templates(lss_handle* h, const float* U, const float* wPCA) {
     const int M = T * K;
     k_utu<<<dim3((M + UT - 1) / UT, (M + UT - 1) / UT), 256, 0, s>>>(h->U.p, M, C, utu.p);
     const size_t smem = sizeof(double) * ((size_t)K * K * L2 + (size_t)CJ * K * K);
-    if (smem > 48 * 1024) SCK(cudaFuncSetAttribute(k_ctc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) SCK(allow_shared_memory<k_ctc>());
     k_ctc<<<dim3((T + CJ - 1) / CJ, T), 128, smem, s>>>(utu.p, wtw.p, T, K, nt, h->ctcP.p);
     SCK(cudaGetLastError());
     h->stats.launches += 6 + (nC > 0);

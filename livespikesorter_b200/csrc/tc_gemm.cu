@@ -770,7 +770,7 @@ static cudaError_t launch_tc(const void* A, const void* Alo, int64_t ldk, int N,
     a.cf_lo = ex.cf_lo;
     a.cf_hi = ex.cf_hi;
     if (a.un && (!a.pn2 || !a.cf2 || !a.cf_lo || !a.cf_hi || ex.rowmap)) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(tc::k_score_tc<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    cudaError_t e = allow_shared_memory<tc::k_score_tc<OP>>();
     if (e != cudaSuccess) return e;
     const int items = split ? ntiles * ((p.Tpad + p.pass_w - 1) / p.pass_w) : ntiles;
     if (split && !part_mode && maxima) {
