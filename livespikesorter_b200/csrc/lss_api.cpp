@@ -969,10 +969,18 @@ int lss_set_postprocess(lss_handle* h, const lss_post_config* pc) {
     return lss_reset_postprocess(h);
 }
 
-// May a kernel on `device` read or write p's floats in place? Else a copy is made, which takes whatever
-// cudaMemcpy takes (another device's memory, odd addresses) and refuses the rest with an error.
-static bool kernel_accessible(const void* p, int device) {
-    return (reinterpret_cast<uintptr_t>(p) & 3) == 0 && lss::device_accessible(p, device);
+// Is p memory of `device` whose floats kernels may work on in place? Else a copy is made, which takes whatever
+// cudaMemcpy takes (another device's memory, odd addresses) and refuses the rest with an error. Pinned host memory
+// is copied too: the projection reads a sample twice and the residual once more, and kernels cross the bus in
+// pieces (384 channels x 60122 samples, in place against copied: a pinned batch matched in 7.6 against 2.7 ms,
+// filtered into pinned memory in 12.8 against 2.3).
+static bool in_place(const void* p, int device) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return (reinterpret_cast<uintptr_t>(p) & 3) == 0 && a.type == cudaMemoryTypeDevice && a.device == device;
 }
 
 // The caller's batch [C, N] in the handle's buffer, rows of ld.
@@ -988,7 +996,7 @@ int lss_filter(lss_handle* h, const int16_t* raw, int64_t n_rows, int64_t ibatch
     CK(cudaSetDevice(h->cfg.device));
     cudaStream_t s = (cudaStream_t)stream;
     CK(wait_mixing(h, s));
-    if (kernel_accessible(X_dev, h->cfg.device)) {
+    if (in_place(X_dev, h->cfg.device)) {
         int rc = run_filter(h, raw, n_rows, ibatch, n_batches, raw_on_device, X_dev, h->N, s);
         if (rc) return rc;
     } else {
@@ -1010,14 +1018,14 @@ int lss_scores(lss_handle* h, const float* X_dev, int64_t N, float* B_dev, void*
     CK(wait_mixing(h, s));
     const float* X = X_dev;
     int64_t ldx = N;
-    if (!kernel_accessible(X_dev, h->cfg.device)) {
+    if (!in_place(X_dev, h->cfg.device)) {
         CK(copy_batch(h, X_dev, N, s));
         X = h->X.p;
         ldx = h->ld;
     }
     CK(cudaMemsetAsync(h->status.p, 0, sizeof(int32_t), s));
     // tiles, which the GEMM writes 64 bytes per thread at a time; one pass brings them into the caller's rows
-    const bool direct = kernel_accessible(B_dev, h->cfg.device);
+    const bool direct = in_place(B_dev, h->cfg.device);
     int rc = run_scores(h, X, ldx, N, h->B.p, s, nullptr, false, /*tiled=*/direct);
     if (rc) return rc;
     if (direct) {
@@ -1047,7 +1055,7 @@ static int match_common(lss_handle* h, int64_t N, const float* Xsrc, int64_t ldx
         h->stats.launches += 1;
     }
     if (xres_dev && Xsrc) {
-        if (kernel_accessible(xres_dev, h->cfg.device)) {
+        if (in_place(xres_dev, h->cfg.device)) {
             rc = run_xres(h, Xsrc, ldx, N, rounds, xres_dev, N, s);
             if (rc) return rc;
         } else {
@@ -1081,7 +1089,7 @@ int lss_match(lss_handle* h, const float* X_dev, int64_t N, int64_t* st_dev, flo
         return p && b < x1 && x0 < b + bytes;
     };
     const size_t cap = capacity > 0 ? (size_t)capacity : 0;
-    if (!kernel_accessible(X_dev, h->cfg.device) || shared(xres_dev, x1 - x0) ||
+    if (!in_place(X_dev, h->cfg.device) || shared(xres_dev, x1 - x0) ||
         (xres_dev && (shared(st_dev, 16 * cap) || shared(amps_dev, 4 * cap)))) {
         CK(copy_batch(h, X_dev, N, s));
         X = h->X.p;
@@ -1105,7 +1113,8 @@ int lss_match_scores(lss_handle* h, const float* B_dev, int64_t N, int64_t* st_d
     if (h->mp_lazy) {  // the deferred rounds read the field as tiles
         const float* B = B_dev;
         float* tmp = nullptr;
-        if (!kernel_accessible(B_dev, h->cfg.device)) {
+        // (read once, in whole lines: pinned memory in place as well)
+        if ((reinterpret_cast<uintptr_t>(B_dev) & 3) || !lss::device_accessible(B_dev, h->cfg.device)) {
             const size_t bytes = sizeof(float) * (size_t)N * h->T;
             CK(cudaMallocAsync(reinterpret_cast<void**>(&tmp), bytes, s));
             const cudaError_t e = cudaMemcpyAsync(tmp, B_dev, bytes, cudaMemcpyDeviceToDevice, s);
