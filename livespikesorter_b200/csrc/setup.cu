@@ -332,7 +332,10 @@ int lss_set_templates(lss_handle* h, const float* U, const float* wPCA) {
             return h->fail(LSS_ERR_ARG, "template " + std::to_string(i) + " has zero or non-finite energy");
     // the templates' probe order and what is laid out in it, and the
     // whitening-folded operands, follow the new templates
-    const int rc = rebuild_probe_order(h, U);
+    // (U read back: like wPCA it may be whatever cudaMemcpy takes, device memory included)
+    std::vector<float> u((size_t)T * K * C);
+    SCK(cudaMemcpy(u.data(), h->U.p, u.size() * sizeof(float), cudaMemcpyDeviceToHost));
+    const int rc = rebuild_probe_order(h, u.data());
     if (rc) return rc;
     return rebuild_uw(h);
 }
