@@ -171,11 +171,13 @@ int  lss_match_scores(lss_handle* h, const float* B_dev, int64_t N, int64_t* st_
  * reference): 0 = every template row of every spike window is updated in its
  * round; 1 = template rows are grouped in blocks along the probe and a block of
  * the score field is updated only once it can take part in a decision (a bound
- * of its scores reaches the threshold). A handle that was not told runs the
- * deferred updates (measured on a B200, 384 channels, 2-s batches: 2.0 vs 7.7 ms
- * of rounds at 800 templates, 0.72 vs 2.06 ms at 400). */
+ * of its scores reaches the threshold). A handle told 1, and one that was not
+ * told, defers unless its batches are too long for that (hundreds of thousands of
+ * samples: a slice's state no longer fits in shared memory). Measured on a B200,
+ * 384 channels, 2-s batches: 2.0 vs 7.7 ms of rounds at 800 templates, 0.72 vs
+ * 2.06 ms at 400. */
 int  lss_set_round_kernel(lss_handle* h, int32_t skip_blocks);
-/* The value last set; before that, 1 from 600 templates up, else 0. */
+/* Which of the two runs; setting what it returns changes nothing. */
 int  lss_get_round_kernel(const lss_handle* h, int32_t* skip_blocks);
 
 /* The same matching-pursuit rounds for callers that cannot allocate device

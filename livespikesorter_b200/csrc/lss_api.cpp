@@ -439,7 +439,6 @@ int lss_create(const lss_config* cfg, const lss_tensors* t, lss_handle** out) {
     // templates, 0.107 vs 0.159 at 64 channels and 32 templates, 0.038 vs 0.043 there on 300 samples. Slices
     // too wide for their shared memory (batches of millions of samples) update every row.
     h->mp_lazy = mp_lazy_fits(h->N, h->mp_grid, T, nt);
-    h->mp_switch = T >= 600;
     ALLOC(mp_perm, (size_t)h->mp_nb * MPB_ROWS);
     ALLOC(mp_hg, (size_t)T * h->mp_nb * mp_lag_groups((int)L2));
     ALLOC(Uq, (size_t)T * K * C);
@@ -606,14 +605,13 @@ int lss_get_stats(const lss_handle* h, lss_stats* out) {
 int lss_set_round_kernel(lss_handle* h, int32_t skip_blocks) {
     if (!h || (skip_blocks != 0 && skip_blocks != 1)) return LSS_ERR_ARG;
     if (h->streaming) return h->fail(LSS_ERR_STATE, "handle is owned by a serving loop");
-    h->mp_switch = skip_blocks != 0;
-    h->mp_lazy = h->mp_switch && mp_lazy_fits(h->N, h->mp_grid, h->T, h->nt);
+    h->mp_lazy = skip_blocks != 0 && mp_lazy_fits(h->N, h->mp_grid, h->T, h->nt);
     return LSS_OK;
 }
 
 int lss_get_round_kernel(const lss_handle* h, int32_t* skip_blocks) {
     if (!h || !skip_blocks) return LSS_ERR_ARG;
-    *skip_blocks = h->mp_switch ? 1 : 0;
+    *skip_blocks = h->mp_lazy ? 1 : 0;
     return LSS_OK;
 }
 

@@ -69,7 +69,6 @@ struct lss_handle {
     // ordered along the probe, bounds of their ctc rows, the CTAs' exchange words
     bool un_p_stale = true;                      // plain-template norms (BF16 bound) need recomputing
     bool mp_lazy = false;                        // rounds kernel: deferred (mp_lazy.cu) or every row (mp.cu)
-    bool mp_switch = false;                      // lss_get_round_kernel's answer
     int mp_nb = 0;
     DevBuf<int32_t> mp_perm;
     DevBuf<float2> mp_hg;

@@ -341,9 +341,17 @@ class Sorter:
         part in a decision (True) or every row in its round (False); the
         results are identical. A sorter that was not told defers."""
         self._check(self._lib.lss_set_round_kernel(self._h, int(bool(skip_blocks))))
+        self._rounds_told = bool(skip_blocks)
 
     def round_kernel(self) -> bool:
-        """The value last set; before that, True from 600 templates up."""
+        """What ``set_round_kernel`` was last given; before that, True from 600
+        templates up. Which rounds run is ``rounds_deferred``."""
+        told = getattr(self, '_rounds_told', None)
+        return self.T >= 600 if told is None else told
+
+    def rounds_deferred(self) -> bool:
+        """True when this sorter's rounds defer (not where its slices are too
+        wide for that); given to ``set_round_kernel`` it changes nothing."""
         import ctypes
         v = ctypes.c_int32(0)
         self._check(self._lib.lss_get_round_kernel(self._h, ctypes.byref(v)))
