@@ -811,10 +811,12 @@ int lss::enqueue_mp(lss_handle* h, int64_t N, cudaStream_t s, bool maxima_ready)
         a.bkey = h->mp_bkey.p;
         a.ctcP = h->mp_ctct.p;
         a.xch = h->mp_xch.p;
+        h->mp_ctas = mp_lazy_grid(N, G);
         CK(launch_mp_lazy(a, G, s));
     } else {
         a.init_cols = maxima_ready ? 0 : 1;
         CK(cudaMemsetAsync(h->colkey.p, 0, 2 * h->ld * sizeof(unsigned long long), s));
+        h->mp_ctas = G;
         CK(launch_mp(a, G, s));
     }
     h->stats.launches += 1;

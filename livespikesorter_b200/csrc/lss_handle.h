@@ -41,7 +41,8 @@ struct lss_handle {
     int C = 0, Cbin = 0, T = 0, K = 0, nt = 0, nC = 0, NT = 0, N = 0;
     int64_t ld = 0;
     int hpL = -1;  // FIR half length; -1 = no highpass
-    int mp_grid = 0;
+    int mp_grid = 0;                             // most CTAs of a rounds kernel
+    int mp_ctas = 0;                             // ... of the last one launched
     size_t dev_bytes = 0;                        // device memory allocated by lss_create
     std::vector<float> h_hp;
     std::vector<float> h_wpca;                   // [K, nt] basis (kernel arguments of the projection)
@@ -133,7 +134,7 @@ struct lss_handle {
 
     unsigned long long mp_phase_host[6] = {};    // host copy of mp_phase after a synchronous batch
     void set_phase_stats() {
-        const int64_t g = std::max(1, mp_grid);
+        const int64_t g = std::max(1, mp_ctas);
         stats.mp_peak_ns = (int64_t)(mp_phase_host[0] / g);
         stats.mp_peak_wait_ns = (int64_t)(mp_phase_host[1] / g);
         stats.mp_update_ns = (int64_t)(mp_phase_host[2] / g);

@@ -226,6 +226,8 @@ constexpr int MPB_ROWS = 16;  // template rows of a tile
 constexpr int MPB_LAGS = 8;   // lags of a group of the bounds
 inline int mp_lag_groups(int L2) { return (L2 + MPB_LAGS - 1) / MPB_LAGS; }
 cudaError_t launch_mp_lazy(MPArgs a, int max_grid, cudaStream_t s);
+// the CTAs that it launches: slices are whole chunks of 32 columns
+int mp_lazy_grid(int64_t N, int max_grid);
 // whether the deferred rounds can run a batch of N columns on at most grid CTAs
 bool mp_lazy_fits(int64_t N, int grid, int T, int nt);
 // 64-bit words of MPArgs::xch for batches of at most N columns

@@ -827,6 +827,11 @@ static int mpl_width(int64_t N, int grid) {
     return 32 * (int)((nchunk + grid - 1) / grid);
 }
 
+int mp_lazy_grid(int64_t N, int max_grid) {
+    const int W = mpl_width(N, max_grid);
+    return (int)((N + W - 1) / W);
+}
+
 // most spikes one round adds to a CTA's log before STATUS_LIST: MP_LIST per
 // 2nt+1 columns over its slice and the nt columns on either side, and the last
 // MP_LIST of the round, which no limit watches
@@ -871,7 +876,7 @@ cudaError_t launch_mp_lazy(MPArgs a, int max_grid, cudaStream_t s) {
         !mp_lazy_fits(a.N, max_grid, a.T, a.nt))
         return cudaErrorInvalidValue;
     const int W = mpl_width(a.N, max_grid);
-    const int grid = (a.N + W - 1) / W;
+    const int grid = mp_lazy_grid(a.N, max_grid);
     if ((3 * a.nt + W - 1) / W + (a.nt + W - 1) / W + 1 > MPL_REGIONS) return cudaErrorInvalidValue;
     a.cols_per_blk = W;
     a.new_cap = mpl_new_cap(W, a.nt);
