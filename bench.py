@@ -312,17 +312,7 @@ def run_b200(args):
     tfl = peaks.get('bf16_tflops', 1590.0)
     src = 'measured' if peaks else 'fallback'
     if top == 'mp_ms':
-        kname, prof = 'k_mp_lazy (matching pursuit, deferred updates)', f'k_mp_lazy_384ch_{T}t.md'
-        traffic = profile_traffic(prof)
-        ach = (traffic or mp_bytes) / (mean_st['mp_ms'] / 1e3) / 1e9
-        roof = {'kernel': kname, 'bound': 'latency', 'achieved': ach, 'peak': hbm, 'unit': 'GB/s',
-                'frac': ach / hbm, 'traffic': traffic,
-                'traffic_source': 'ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload '
-                                  f'(profiles/{prof})',
-                'algorithmic_bytes': mp_bytes, 'peak_source': src,
-                'note': 'achieved counts `traffic` (every row updated where it is not recorded); the deferred rounds '
-                        'make only the updates that can matter to a decision, updating every row would move '
-                        '`algorithmic_bytes`'}
+        roof = rounds_roofline(T, mean_st['mp_ms'], mp_bytes, hbm, src)
     else:
         ach = gemm_flops / (mean_st['score_ms'] / 1e3) / 1e12
         roof = {'kernel': 'k_score_tc (tcgen05 3xTF32 score GEMM)' if args.precision == 'fp32'
@@ -345,7 +335,8 @@ def run_b200(args):
                      'latency_ms_p50': float(np.percentile(per_s, 50)),
                      'latency_ms_p99': float(np.percentile(per_s, 99))},
         'latency_ms_p50': float(np.percentile(per, 50)), 'latency_ms_p99': float(np.percentile(per, 99)),
-        'roofline': roof, 'roofline_path': path_roofline(setup, float(np.mean(spikes)), T, value / world, hbm, tfl, src),
+        'roofline': roof, 'roofline_path': path_roofline(setup, float(np.mean(spikes)), T, value / world, hbm, tfl, src,
+                                                             rounds_traffic(T)),
         'gpu_launches': int(launches), 'clocks': clocks,
         'stage_ms': mean_st, 'mp_phases_ms': phases,
         'spikes_per_batch': float(np.mean(spikes)), 'rounds_per_batch': float(np.mean(rounds)),
@@ -474,23 +465,46 @@ def max_over_ranks(x: float, dist, device) -> float:
     return float(t.item())
 
 
-def path_roofline(setup, spikes_per_batch, T, rec_s_per_s, hbm_gbs, tensor_tflops, src):
-    """The whole path against both bounds: algorithmic FLOPs and bytes per
-    recording-second (whitening/drift C^2, temporal basis C*K*nt, score GEMM
-    T*K*C per sample, plus 2*T*(2nt+1) FLOPs and 12*T*(2nt+1) bytes per
-    accepted spike; int16 in and the score field written and read once),
-    times the measured rate."""
+def path_roofline(setup, spikes_per_batch, T, rec_s_per_s, hbm_gbs, tensor_tflops, src, mp_traffic):
+    """The whole path against both bounds: algorithmic FLOPs per recording-second
+    (whitening/drift C^2, temporal basis C*K*nt, score GEMM T*K*C per sample, plus
+    2*T*(2nt+1) per accepted spike) and bytes (int16 in, the score field written
+    once, and what the rounds move: `mp_traffic` DRAM bytes per batch, as recorded
+    for this template count), times the measured rate. No bytes where the rounds'
+    are not recorded."""
     C, K, nt = setup.C, setup.K, setup.nt
     L2 = 2 * nt + 1
-    S = spikes_per_batch / (setup.NT / FS)  # accepted spikes per recording-second
-    flops = 2.0 * FS * (C * C + C * K * nt + T * K * C) + S * 2.0 * T * L2
-    nbytes = 2.0 * C * FS + 8.0 * T * FS + S * 12.0 * T * L2
+    batches = FS / setup.NT                 # per recording-second
+    flops = 2.0 * FS * (C * C + C * K * nt + T * K * C) + spikes_per_batch * batches * 2.0 * T * L2
+    nbytes = None if mp_traffic is None else 2.0 * C * FS + 4.0 * T * FS + mp_traffic * batches
     f_t = flops * rec_s_per_s / 1e12 / tensor_tflops
-    f_h = nbytes * rec_s_per_s / 1e9 / hbm_gbs
+    gbs = None if nbytes is None else nbytes * rec_s_per_s / 1e9
+    f_h = None if gbs is None else gbs / hbm_gbs
     return {'flops_per_rec_s': flops, 'bytes_per_rec_s': nbytes,
-            'tflops': flops * rec_s_per_s / 1e12, 'gbs': nbytes * rec_s_per_s / 1e9,
-            'frac_tensor': f_t, 'frac_hbm': f_h, 'bound': 'hbm' if f_h >= f_t else 'tensor',
-            'frac': max(f_t, f_h), 'peaks': f'{src}: HBM {hbm_gbs} GB/s, dense bf16 {tensor_tflops} TFLOP/s'}
+            'tflops': flops * rec_s_per_s / 1e12, 'gbs': gbs,
+            'frac_tensor': f_t, 'frac_hbm': f_h, 'bound': 'hbm' if f_h is not None and f_h >= f_t else 'tensor',
+            'frac': max(f_t, f_h or 0.0), 'peaks': f'{src}: HBM {hbm_gbs} GB/s, dense bf16 {tensor_tflops} TFLOP/s'}
+
+
+def rounds_traffic(T):
+    """DRAM bytes of one batch's rounds on the 384-channel workload (None if not recorded)."""
+    return profile_traffic(f'k_mp_lazy_384ch_{T}t.md')
+
+
+def rounds_roofline(T, mp_ms, mp_bytes, hbm, src):
+    """The rounds against the copy bandwidth, by their recorded DRAM traffic; no
+    rate where none is recorded for this template count (the bytes of updating every
+    row are not what the deferred rounds move)."""
+    traffic = rounds_traffic(T)
+    ach = None if traffic is None else traffic / (mp_ms / 1e3) / 1e9
+    return {'kernel': 'k_mp_lazy (matching pursuit, deferred updates)', 'bound': 'latency', 'achieved': ach,
+            'peak': hbm, 'unit': 'GB/s', 'frac': None if ach is None else ach / hbm, 'traffic': traffic,
+            'traffic_source': None if traffic is None else
+            'ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload '
+            f'(profiles/k_mp_lazy_384ch_{T}t.md)',
+            'algorithmic_bytes': mp_bytes, 'peak_source': src,
+            'note': 'achieved counts `traffic`; the deferred rounds make only the updates that can matter to a '
+                    'decision, updating every row would move `algorithmic_bytes`'}
 
 
 def profile_traffic(name):
