@@ -347,30 +347,22 @@ __device__ __forceinline__ void pc_features_one(
     for (int c0 = 0; c0 < (Phi ? 0 : C); c0 += FT_CH) {
         const int nc = min(FT_CH, C - c0);
         __syncthreads();
-        if (Phi) {
-            // projection row of the score GEMM: P[x, c*K + k] = hi + lo (to 2^-23 relative)
-            const int64_t o = (int64_t)x * ldp + (int64_t)c0 * K;
-            for (int e = threadIdx.x; e < nc * K; e += blockDim.x) pc[e] = __fadd_rn(pval(Phi + o + e), pval(Plo + o + e));
-        } else {
-            for (int e = threadIdx.x; e < nc * nt; e += blockDim.x) {
-                const int c = e / nt, m = e % nt;
-                xs[c * ntp + m] = Xh[(int64_t)(c0 + c) * ldx + x - h + m];
-            }
+        for (int e = threadIdx.x; e < nc * nt; e += blockDim.x) {
+            const int c = e / nt, m = e % nt;
+            xs[c * ntp + m] = Xh[(int64_t)(c0 + c) * ldx + x - h + m];
         }
         for (int e = threadIdx.x; e < nC * nc; e += blockDim.x) {
             const int j = e / nc, c = e % nc;
             mw[j * FT_CH + c] = Mw[(int64_t)s_ch[j] * C + c0 + c];
         }
         __syncthreads();
-        if (!Phi) {
-            for (int e = threadIdx.x; e < nc * K; e += blockDim.x) {
-                const int c = e / K, k = e % K;
-                float p = 0.f;
-                for (int m = 0; m < nt; ++m) p = fmaf(ws[k * nt + m], xs[c * ntp + m], p);
-                pc[c * K + k] = p;
-            }
-            __syncthreads();
+        for (int e = threadIdx.x; e < nc * K; e += blockDim.x) {
+            const int c = e / K, k = e % K;
+            float p = 0.f;
+            for (int m = 0; m < nt; ++m) p = fmaf(ws[k * nt + m], xs[c * ntp + m], p);
+            pc[c * K + k] = p;
         }
+        __syncthreads();
         for (int e = threadIdx.x; e < nC * K; e += blockDim.x) {
             const int j = e / K, k = e % K;
             float v = acc[e];
