@@ -45,8 +45,9 @@ __device__ __forceinline__ unsigned long long dup2(float x) {
     return v;
 }
 
-// A basis of up to 64 taps as kernel arguments: pairs of components by tap (zero
-// past nt and K), which the packed FMAs read from the constant bank.
+// A basis of 57 to 63 taps (64 with its padding) as kernel arguments: pairs of
+// components by tap (zero past nt and K), which the packed FMAs read from the
+// constant bank.
 struct PcaTaps {
     unsigned long long w[64 * 4];
 };
@@ -56,9 +57,9 @@ struct PcaTaps {
 // and a warp writes 32*K contiguous outputs per sample row. The FP32 pipe bounds
 // it (17 GFLOP at 384 channels x 60122 samples, K = 6, nt = 61: 0.23 ms at the FP32
 // peak), so components go in pairs through packed FMAs and one sample load and one
-// duplication serve 8K of them. Up to 64 taps the weights come from the kernel's
-// arguments: 0.36 ms with the tf32 split, 0.42 with two weight loads from shared
-// memory per tap (0.49 with one FMA per instruction; a packed one takes the pipe
+// duplication serve 8K of them. With 57 to 63 taps, which are unrolled, the weights
+// come from the kernel's arguments: 0.36 ms with the tf32 split, 0.42 with two weight
+// loads from shared memory per tap, as other lengths take them (0.49 with one FMA per instruction; a packed one takes the pipe
 // two cycles and more, what it saves is issue slots). A walk over several tiles per
 // CTA with the next one's samples copied ahead and rows staged per warp was slower.
 template <int KPC, int PC, bool TF32, int NTP>
@@ -244,7 +245,7 @@ static cudaError_t launch_pjt(const float* X, int64_t ldx, int32_t C, int64_t N,
             for (int k = 0; k < KPC; ++k)
                 std::memcpy(reinterpret_cast<float*>(&taps.w[m * KP + k / 2]) + k % 2, wpca_host + (int64_t)k * nt + m, 4);
     }
-    if (ntp == 64) {  // nt = 57..64 (Kilosort's 61): taps fully unrolled
+    if (ntp == 64) {  // taps unrolled; a shorter basis would pay for zeros (41 taps, padded to 48 below: a third more)
         constexpr auto kern = k_pca_proj_t<KPC, PC, TF32, 64>;
         const cudaError_t e = allow_shared_memory<kern>();
         if (e != cudaSuccess) return e;

@@ -31,7 +31,7 @@ namespace lss {
 namespace tc {
 
 constexpr int BM = 128;               // samples per tile
-constexpr int MAX_NP = 512;           // templates per pass (TMEM columns)
+constexpr int MAX_NP = 512;           // TMEM columns: two accumulators of up to 256 templates
 constexpr int MAX_STAGES = 6;
 constexpr int SPLIT_W = 128;          // templates per work item in split mode
 constexpr int MAPPED_SPLIT_W = 64;    // ... for a re-check of a few mapped rows
@@ -62,7 +62,7 @@ struct Kind {
 struct Args {
     int N, T, Tpad, KB;
     int stages, b_rows;
-    int nacc;                 // accumulator buffers in TMEM (2 when a pass fits in 256 columns)
+    int nacc;                 // accumulator buffers in TMEM
     float* Bout;
     int64_t ldb;
     const float* nm;
@@ -77,7 +77,7 @@ struct Args {
     int tile_blocks;          // > 0: Bout as the deferred rounds' tiles, that many row blocks
     int ncols;                // samples in the batch (edge columns are the first/last nt)
     float* cf2;               // (error bounds) largest upper bound of any other template
-    int pass_w;               // templates per pass (<= MAX_NP)
+    int pass_w;               // templates per pass (at most 256)
     bool split;               // one work item per (sample tile, pass) instead of per tile
     bool maxima;              // column maxima are wanted (the deferred rounds take theirs from the tiles)
     unsigned long long* keys; // split mode: one work item per (sample tile, pass); column maxima are
@@ -666,6 +666,8 @@ static bool make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t col
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// A pass wider than 256 templates (two boxes, one accumulator) is planned only by
+// lss_create's check of the template count; launch_tc refuses it.
 TcPlan tc_plan(int T, int op, int pass_w) {
     TcPlan p{};
     p.Tpad = (T + 15) / 16 * 16;
