@@ -223,6 +223,56 @@ __global__ void __launch_bounds__(RF_THREADS, sizeof(F) == 4 ? 3 : 1)
 }
 
 
+// A template's gradients again where the sums over its spikes were NaN: by the
+// definition, which contracts a spike's window before its amplitude is taken (an
+// infinite amplitude times a window of both signs is a NaN in S_t, and an infinite
+// gradient). A sum that turns NaN here too is not taken further. One CTA; 0.8 us of the
+// backward pass below when nothing is redone.
+template <typename F>
+__device__ __noinline__ void redo_nan(const F* __restrict__ U, const F* __restrict__ W, int K, int C, int nt,
+                                      const int32_t* __restrict__ x, const F* __restrict__ amp,
+                                      const int32_t* __restrict__ order, const int32_t* __restrict__ tstart,
+                                      const F* __restrict__ G, int64_t N, F* dU, F* Qt, F* damp, int t) {
+    const int j0 = tstart[t], j1 = tstart[t + 1];
+    auto g = [&](int i, int c, int m) {  // G in spike i's window
+        const int64_t s = (int64_t)x[i] + m - nt / 2;
+        return s >= 0 && s < N ? G[(int64_t)c * N + s] : F(0);
+    };
+    auto dot = [&](int i, int k, int c) {  // P_i[k, c]
+        F p = F(0);
+        for (int m = 0; m < nt && p == p; ++m) p += W[k * nt + m] * g(i, c, m);
+        return p;
+    };
+    const F* Ut = U + (int64_t)t * K * C;
+    for (int e = threadIdx.x; e < K * C; e += RB_THREADS) {
+        F* p = dU + (int64_t)t * K * C + e;
+        if (*p == *p) continue;
+        F v = F(0);
+        for (int j = j0; j < j1 && v == v; ++j) v += amp[order[j]] * dot(order[j], e / C, e % C);
+        *p = v;
+    }
+    for (int e = threadIdx.x; e < K * nt; e += RB_THREADS) {
+        F* p = Qt + (int64_t)t * K * nt + e;
+        if (*p == *p) continue;
+        F v = F(0);
+        for (int j = j0; j < j1 && v == v; ++j) {
+            F q = F(0);
+            for (int c = 0; c < C && q == q; ++c) q += Ut[e / nt * C + c] * g(order[j], c, e % nt);
+            v += amp[order[j]] * q;
+        }
+        *p = v;
+    }
+    const int lane = threadIdx.x & 31;
+    for (int j = j0 + threadIdx.x / 32; damp && j < j1; j += RB_WARPS) {  // a warp per spike
+        F* p = damp + order[j];
+        if (*p == *p) continue;
+        F v = F(0);
+        for (int e = lane; e < K * C && v == v; e += 32) v += Ut[e] * dot(order[j], e / C, e % C);
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) *p = v;
+    }
+}
+
 // A cluster of Z CTAs per template t; order[tstart[t] .. tstart[t+1]) are its
 // spikes. CTA z takes channel chunks z, z + Z, ...: a warp's channels w + 16 j (j <
 // CJ), lags lane + 32u (u < NM) of a window in registers, S and the template's
@@ -374,13 +424,17 @@ __global__ void __launch_bounds__(RB_THREADS, sizeof(F) == 4 ? 2 : 1) k_recon_bw
         }
     }
     cl.sync();
+    bool odd = false;
     if (z == 0)
         for (int e = threadIdx.x; e < K * nt; e += RB_THREADS) {
             F v = F(0);
             for (int r = 0; r < Z; ++r) v += cl.map_shared_rank(Qp, r)[e];
             Qt[(int64_t)t * K * nt + e] = v;
+            odd |= !isfinite(v);
         }
     cl.sync();  // the other ranks' shared memory is read until here
+    // (what is not finite in S_t or in the template is in Qt, which sums over all channels)
+    if (z == 0 && __syncthreads_or(odd)) redo_nan(U, W, K, C, nt, x, amp, order, tstart, G, N, dU, Qt, damp, t);
 }
 
 // dW[e] = sum_t Qt[t, e]: 32 columns per CTA, the templates strided over 8 rows
