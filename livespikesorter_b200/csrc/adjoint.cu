@@ -124,7 +124,7 @@ __device__ __noinline__ F recon_one(const F* __restrict__ U, const F* __restrict
 // pairs of channels for floats); one column by 32 channels took 32 beside 8.
 // 9000 spikes at 384 channels x 60000 samples are 2.5 GFLOP that must be done and
 // 3.9 GFLOP done (a window covers 61 of the 92 columns it is taken over), over 92 MB
-// written: 182 us, against 296 us with one column per lane and 232 us with 8 x 8
+// written: 180 us, against 296 us with one column per lane and 232 us with 8 x 8
 // outputs (two CTAs per SM instead of three, 61 of 124 columns).
 // The zeros beside W are no zeros beside an infinite or NaN amplitude or template
 // value: a sum that is not finite at the end is taken again by the definition.
